@@ -123,6 +123,45 @@ int default_variant(int cls) {
 // FP64 kernels: multi-pass classes have the pipelined variants, the others one.
 int default_variant64(int cls) { return class_multi(cls) ? 1 : 0; }
 
+// The gap forms of a class's kernels: one for per-row classes, two for
+// uniform ones (PackedPlan::gap_form).
+constexpr GapForm kUniformForms[2] = {kGapsUniform, kGapsConst};
+
+// Calls fn for every forward kernel the engine can launch.
+template <class Fn>
+void for_each_kernel(const Fn& fn) {
+  for (int c = 0; c < kNumClasses; ++c)
+    for (int u = 0; u < (class_uniform(c) ? 2 : 1); ++u)
+      for (int p = 0; p < 3; ++p) {
+        const Precision pr = p == 2 ? Precision::kF64 : Precision::kF32x2;
+        const GapForm gaps = class_uniform(c) ? kUniformForms[u] : kGapsPerRow;
+        const int nv = forward_kernel_variants(pr, p == 0, class_rows(c), class_multi(c));
+        for (int v = 0; v < nv; ++v)
+          fn(forward_kernel_info(pr, class_rows(c), gaps, class_multi(c), p == 0, v));
+      }
+}
+
+// The constants of launches whose uniform-gap reads all have insertion and
+// deletion quality `ins` and gap continuation quality `gcp`: the values the
+// kGapsUniform kernels compute from a read's first row, by the same
+// operations in the same precision.
+GapConsts gap_consts(uint8_t ins, uint8_t gcp) {
+  const HostPriorTables& t = host_prior_tables();
+  const int mm = ((int)ins * (ins + 1)) / 2 + ins;
+  GapConsts g{};
+  const float iif = t.ph2pr_f[gcp];
+  g.mi = t.ph2pr_f[ins];
+  g.c = g.mi * (1.0f - iif);
+  const float mmf = t.mm_f[mm] / g.c;
+  g.mm2 = make_float2(mmf, mmf);
+  g.ii2 = make_float2(iif, iif);
+  g.mi_d = t.ph2pr_d[ins];
+  g.ii_d = t.ph2pr_d[gcp];
+  g.c_d = g.mi_d * (1.0 - g.ii_d);
+  g.mm_d = t.mm_d[mm] / g.c_d;
+  return g;
+}
+
 }  // namespace
 
 // Every device and pinned-host allocation of the engine and the service goes
@@ -306,17 +345,12 @@ rodv_status Engine::init() {
   RODV_CUDA(ce);
   // Kernels whose tables exceed the default 48 KB of dynamic shared memory
   // per block opt in to their size.
-  for (int c = 0; c < kNumClasses; ++c)
-    for (int p = 0; p < 3; ++p)
-      for (int v = 0; v < kTuneVariants; ++v) {
-        const Precision pr = p == 2 ? Precision::kF64 : Precision::kF32x2;
-        if (v >= forward_kernel_variants(pr, p == 0, class_rows(c), class_multi(c))) continue;
-        const KernelInfo k =
-            forward_kernel_info(pr, class_rows(c), class_uniform(c), class_multi(c), p == 0, v);
-        if (k.fn && k.smem_bytes > 48 * 1024)
-          RODV_CUDA(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         k.smem_bytes));
-      }
+  cudaError_t ke = cudaSuccess;
+  for_each_kernel([&](const KernelInfo& k) {
+    if (ke == cudaSuccess && k.smem_bytes > 48 * 1024)
+      ke = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem_bytes);
+  });
+  RODV_CUDA(ke);
   ready_ = true;
   if (opt_.tune_cache && opt_.tune_cache[0]) load_tuning(opt_.tune_cache);
   if (opt_.autotune) {
@@ -332,16 +366,7 @@ rodv_status Engine::init() {
 // persistent_blocks uses).
 rodv_status Engine::load_kernels() {
   RODV_CUDA(cudaSetDevice(device_));
-  for (int c = 0; c < kNumClasses; ++c)
-    for (int p = 0; p < 3; ++p) {
-      const Precision pr = p == 2 ? Precision::kF64 : Precision::kF32x2;
-      const int nv = forward_kernel_variants(pr, p == 0, class_rows(c), class_multi(c));
-      for (int v = 0; v < nv; ++v) {
-        const KernelInfo k =
-            forward_kernel_info(pr, class_rows(c), class_uniform(c), class_multi(c), p == 0, v);
-        if (k.fn) persistent_blocks(k);
-      }
-    }
+  for_each_kernel([&](const KernelInfo& k) { persistent_blocks(k); });
   RODV_CUDA(cudaGetLastError());
   return RODV_OK;
 }
@@ -351,13 +376,9 @@ rodv_status Engine::load_kernels() {
 // variant on its batches).
 size_t Engine::multi_scratch_rows() const {
   size_t rows = 0;
-  for (int u = 0; u < 2; ++u)
-    for (int p = 0; p < 3; ++p)
-      for (int v = 0; v < kPipeVariants; ++v) {
-        const Precision pr = p == 2 ? Precision::kF64 : Precision::kF32x2;
-        const KernelInfo k = forward_kernel_info(pr, kMaxRowsPerLane, u != 0, true, p == 0, v);
-        rows = std::max(rows, (size_t)persistent_blocks(k) * k.boundary_rows);
-      }
+  for_each_kernel([&](const KernelInfo& k) {
+    if (k.multi) rows = std::max(rows, (size_t)persistent_blocks(k) * k.boundary_rows);
+  });
   return rows;
 }
 
@@ -498,7 +519,11 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   std::vector<uint8_t>& read_class = plan.read_class;
   read_class.resize(b.num_reads);
   const HostPriorTables& pt = host_prior_tables();
+  // gap qualities (ins << 8 | gcp) of the uniform-gap reads, while they agree
+  constexpr uint32_t kNoGaps = 0xffffffffu, kMixedGaps = 0xfffffffeu;
+  std::atomic<uint32_t> gap_quals{kNoGaps};
   parallel_for(b.num_reads, 512, [&](size_t lo, size_t hi) {
+    uint32_t seen = kNoGaps;  // of this range's uniform reads
     for (size_t r = lo; r < hi; ++r) {
       const uint64_t off = b.read_offsets[r];
       const uint32_t n = b.read_lengths[r];
@@ -516,8 +541,19 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
       const bool uniform = u && c0 != 0 && i0 == d0 &&
                            (double)pt.ph2pr_f[i0] * (1.0 - (double)pt.ph2pr_f[c0]) >= 1e-6;
       read_class[r] = (uint8_t)class_of(n, uniform);
+      if (uniform) {
+        const uint32_t key = (uint32_t)i0 << 8 | c0;
+        seen = seen == kNoGaps || seen == key ? key : kMixedGaps;
+      }
     }
+    if (seen == kNoGaps) return;
+    uint32_t all = kNoGaps;
+    if (!gap_quals.compare_exchange_strong(all, seen) && all != seen)
+      gap_quals.store(kMixedGaps);
   });
+  const uint32_t gq = gap_quals.load();
+  plan.const_gaps = gq != kNoGaps && gq != kMixedGaps;
+  if (plan.const_gaps) plan.gaps = gap_consts((uint8_t)(gq >> 8), (uint8_t)(gq & 0xff));
 
   timer.mark("classes");
   // ---- per region and class: reads, chain items, same items, leftovers ----
@@ -544,7 +580,7 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   // the uniform classes' item geometry, from the kernel variants packed for
   int chain_ipw[kMaxRowsPerLane + 1] = {};
   for (int R = 1; R <= kMaxRowsPerLane; ++R)
-    chain_ipw[R] = forward_kernel_info(Precision::kF32x2, R, true, false, true,
+    chain_ipw[R] = forward_kernel_info(Precision::kF32x2, R, kGapsUniform, false, true,
                                        variant_[single_pass_class(R, true)])
                        .items_per_warp;
   ChainGeom geom[kMaxRowsPerLane + 1];
@@ -611,7 +647,7 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   }
   for (int c = 0; c < kSinglePassClasses; ++c) {
     // chain items a warp of this class's kernel sweeps at once
-    const int ipw = forward_kernel_info(Precision::kF32x2, class_rows(c), class_uniform(c),
+    const int ipw = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c),
                                         false, true, plan.variant[c]).items_per_warp;
     const uint64_t target_items = (uint64_t)num_sms_ * 16 * 2 * ipw;
     plan.chain_haps[c] = 1;
@@ -949,7 +985,7 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   if (!n) return RODV_OK;
   // the multi-pass two-haplotype kernel shares the class's variant (strip
   // height), which the packer paired its items by
-  const KernelInfo k = forward_kernel_info(Precision::kF32x2, class_rows(c), class_uniform(c),
+  const KernelInfo k = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c),
                                            class_multi(c), same,
                                            (same || class_multi(c)) ? variant : 0);
   ClassLaunch cl{};
@@ -963,6 +999,7 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   cl.scratch_cols = plan.scratch_cols;
   cl.error_flags = a.counts + kCtrError;
   cl.stack = reinterpret_cast<const uint32_t*>(dbase + plan.off_stack[c]);
+  cl.gaps = plan.gaps;
   if (class_multi(c)) {  // rescues at their items' positions: same items, then two-haplotype
     cl.flags |= kLaunchRescueByItem;
     cl.rescue_base = same ? 0u : 2u * plan.same_items[c];
@@ -982,7 +1019,7 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
 rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int c,
                                       int variant, cudaStream_t stream) {
   ArenaView a = arena_view(plan, dbase, tab_);
-  const KernelInfo k = forward_kernel_info(Precision::kF64, class_rows(c), class_uniform(c),
+  const KernelInfo k = forward_kernel_info(Precision::kF64, class_rows(c), plan.gap_form(c),
                                            class_multi(c), false, variant);
   ClassLaunch cl{};
   cl.work = dbase + plan.off_lists[c];
@@ -995,6 +1032,7 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
     cl.static_count = 2u * (plan.same_items[c] + plan.diff_items[c]);
   }
   cl.counter = a.counts + kCtrF64 + c;
+  cl.gaps = plan.gaps;
   cl.scratch = class_scratch(plan, a, c);
   cl.scratch_cols = plan.scratch_cols;
   cl.error_flags = a.counts + kCtrError;
@@ -1492,7 +1530,7 @@ rodv_status Engine::plain(rodv_device_batch* db, double* out, rodv_stats* st) {
           const bool f64 = pass == 1 || plan.fp64;
           const KernelInfo k =
               forward_kernel_info(f64 ? Precision::kF64 : Precision::kF32x2, class_rows(c),
-                                  class_uniform(c), class_multi(c), true,
+                                  plan.gap_form(c), class_multi(c), true,
                                   f64 ? variant64_[c] : variant_[c]);
           ClassLaunch cl{};
           cl.work = f64 ? static_cast<const void*>(w + 32) : static_cast<const void*>(w);
@@ -1505,6 +1543,7 @@ rodv_status Engine::plain(rodv_device_batch* db, double* out, rodv_stats* st) {
           cl.scratch_cols = plan.scratch_cols;
           cl.error_flags = wc + 3;
           cl.stack = reinterpret_cast<const uint32_t*>(w + 64);
+          cl.gaps = plan.gaps;
           void* args[] = {&a.view, &cl};
           RODV_CUDA(
               cudaLaunchKernel(k.fn, dim3(1), dim3(k.threads), args, k.smem_bytes, stream_));

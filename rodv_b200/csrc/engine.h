@@ -80,6 +80,13 @@ struct PackedPlan {
   uint32_t multi_max_hap = 0;
   bool fp64 = false;                       // every pair computed in FP64
   bool raw = false;                        // raw likelihoods and their precision
+  // Every uniform-gap read of the batch has the same gap qualities: the
+  // uniform classes run the kernels that take them as constants.
+  bool const_gaps = false;
+  GapConsts gaps = {};
+  GapForm gap_form(int cls) const {
+    return !class_uniform(cls) ? kGapsPerRow : const_gaps ? kGapsConst : kGapsUniform;
+  }
   // FP32 same-haplotype items: ChainItem for single-pass classes, SameItem
   // for the multi-pass ones
   uint32_t same_items[kNumClasses] = {};

@@ -12,11 +12,11 @@
 
 namespace rodv {
 
-template <class P, int R, bool U, bool MU, bool SAME, int MINB, int GROUP = 32>
+template <class P, int R, int GAPS, bool MU, bool SAME, int MINB, int GROUP = 32>
 KernelInfo make_info(int variant) {
-  using F = Forward<P, R, U, MU, SAME, MINB, GROUP>;
+  using F = Forward<P, R, GAPS, MU, SAME, MINB, GROUP>;
   KernelInfo k;
-  k.fn = reinterpret_cast<const void*>(&forward_kernel<P, R, U, MU, SAME, MINB, GROUP>);
+  k.fn = reinterpret_cast<const void*>(&forward_kernel<P, R, GAPS, MU, SAME, MINB, GROUP>);
   k.threads = F::kWarpsPerBlock * kWarp;
   k.warps_per_block = F::kWarpsPerBlock;
   k.smem_bytes = F::kWarpsPerBlock * F::kSmemPerWarp;
@@ -32,11 +32,11 @@ KernelInfo make_info(int variant) {
 }
 
 // Multi-pass kernels: the passes of one item on the W warps of a block.
-template <class P, int R, bool U, bool SAME, int W>
+template <class P, int R, int GAPS, bool SAME, int W>
 KernelInfo make_pipe_info(int variant) {
-  using F = PipeForward<P, R, U, SAME, 1, W>;
+  using F = PipeForward<P, R, GAPS, SAME, 1, W>;
   KernelInfo k;
-  k.fn = reinterpret_cast<const void*>(&forward_pipe_kernel<P, R, U, SAME, 1, W>);
+  k.fn = reinterpret_cast<const void*>(&forward_pipe_kernel<P, R, GAPS, SAME, 1, W>);
   k.threads = W * kWarp;
   k.warps_per_block = W;
   k.smem_bytes = W * F::kSmemPerWarp;
@@ -53,29 +53,27 @@ KernelInfo make_pipe_info(int variant) {
 }
 
 // The multi-pass variants of strip height R (pipe_variant_rows) for one
-// precision and item kind: W = 2 or 4 warps per item.
-template <int R>
-KernelInfo pipe_info_for(Precision prec, bool uniform, bool same, int variant) {
+// precision, gap form and item kind: W = 2 or 4 warps per item.
+template <int R, int GAPS>
+KernelInfo pipe_gap_info(Precision prec, bool same, int variant) {
   const bool w4 = pipe_variant_warps(variant) == 4;
-  if (prec == Precision::kF64) {
-    if (uniform)
-      return w4 ? make_pipe_info<F64, R, true, false, 4>(variant)
-                : make_pipe_info<F64, R, true, false, 2>(variant);
-    return w4 ? make_pipe_info<F64, R, false, false, 4>(variant)
-              : make_pipe_info<F64, R, false, false, 2>(variant);
+  if (prec == Precision::kF64)
+    return w4 ? make_pipe_info<F64, R, GAPS, false, 4>(variant)
+              : make_pipe_info<F64, R, GAPS, false, 2>(variant);
+  if (same)
+    return w4 ? make_pipe_info<F32x2, R, GAPS, true, 4>(variant)
+              : make_pipe_info<F32x2, R, GAPS, true, 2>(variant);
+  return w4 ? make_pipe_info<F32x2, R, GAPS, false, 4>(variant)
+            : make_pipe_info<F32x2, R, GAPS, false, 2>(variant);
+}
+
+template <int R>
+KernelInfo pipe_info_for(Precision prec, GapForm gaps, bool same, int variant) {
+  switch (gaps) {
+    case kGapsPerRow: return pipe_gap_info<R, kGapsPerRow>(prec, same, variant);
+    case kGapsUniform: return pipe_gap_info<R, kGapsUniform>(prec, same, variant);
+    default: return pipe_gap_info<R, kGapsConst>(prec, same, variant);
   }
-  if (same) {
-    if (uniform)
-      return w4 ? make_pipe_info<F32x2, R, true, true, 4>(variant)
-                : make_pipe_info<F32x2, R, true, true, 2>(variant);
-    return w4 ? make_pipe_info<F32x2, R, false, true, 4>(variant)
-              : make_pipe_info<F32x2, R, false, true, 2>(variant);
-  }
-  if (uniform)
-    return w4 ? make_pipe_info<F32x2, R, true, false, 4>(variant)
-              : make_pipe_info<F32x2, R, true, false, 2>(variant);
-  return w4 ? make_pipe_info<F32x2, R, false, false, 4>(variant)
-            : make_pipe_info<F32x2, R, false, false, 2>(variant);
 }
 
 // Same-haplotype FP32 kernels come in occupancy targets (kVariantMinBlocks);
@@ -85,42 +83,46 @@ KernelInfo pipe_info_for(Precision prec, bool uniform, bool same, int variant) {
 // table loads, row-0 selects) covers twice the rows (faster at R <= 2 on B200,
 // slower at R >= 3, where the longer per-step dependency chain shows; the
 // autotuner picks).  Every other kernel has one variant.
-template <class P, int R, bool U, bool MU, bool SAME>
+template <class P, int R, int GAPS, bool MU, bool SAME>
 KernelInfo variant_info(int variant) {
   if constexpr (!(std::is_same<P, F32x2>::value && SAME)) {
     (void)variant;
-    return make_info<P, R, U, MU, SAME, 1>(0);
+    return make_info<P, R, GAPS, MU, SAME, 1>(0);
   } else {
     if constexpr (!MU && R <= kMaxGroupedRows) {
       switch (variant) {
-        case 4: return make_info<P, 2 * R, U, MU, SAME, kVariantMinBlocks[4], 16>(4);
-        case 5: return make_info<P, 2 * R, U, MU, SAME, kVariantMinBlocks[5], 16>(5);
-        case 6: return make_info<P, 2 * R, U, MU, SAME, kVariantMinBlocks[6], 16>(6);
-        case 7: return make_info<P, 2 * R, U, MU, SAME, kVariantMinBlocks[7], 16>(7);
+        case 4: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[4], 16>(4);
+        case 5: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[5], 16>(5);
+        case 6: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[6], 16>(6);
+        case 7: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[7], 16>(7);
         default: break;
       }
     }
     switch (variant) {
-      case 0: return make_info<P, R, U, MU, SAME, kVariantMinBlocks[0]>(0);
-      case 1: return make_info<P, R, U, MU, SAME, kVariantMinBlocks[1]>(1);
-      case 2: return make_info<P, R, U, MU, SAME, kVariantMinBlocks[2]>(2);
-      default: return make_info<P, R, U, MU, SAME, kVariantMinBlocks[3]>(3);
+      case 0: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[0]>(0);
+      case 1: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[1]>(1);
+      case 2: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[2]>(2);
+      default: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[3]>(3);
     }
   }
 }
 
-template <int R, bool MU>
-KernelInfo info_for(Precision prec, bool uniform, bool same, int variant) {
-  if (prec == Precision::kF64)
-    return uniform ? variant_info<F64, R, true, MU, false>(0)
-                   : variant_info<F64, R, false, MU, false>(0);
-  if (same)
-    return uniform ? variant_info<F32x2, R, true, MU, true>(variant)
-                   : variant_info<F32x2, R, false, MU, true>(variant);
+template <int R, bool MU, int GAPS>
+KernelInfo gap_info(Precision prec, bool same, int variant) {
+  if (prec == Precision::kF64) return variant_info<F64, R, GAPS, MU, false>(0);
+  if (same) return variant_info<F32x2, R, GAPS, MU, true>(variant);
   // Two-haplotype items: multi-pass leftovers, and the odd single-pass read
   // of a region against each of its haplotypes.
-  return uniform ? variant_info<F32x2, R, true, MU, false>(0)
-                 : variant_info<F32x2, R, false, MU, false>(0);
+  return variant_info<F32x2, R, GAPS, MU, false>(0);
+}
+
+template <int R, bool MU>
+KernelInfo info_for(Precision prec, GapForm gaps, bool same, int variant) {
+  switch (gaps) {
+    case kGapsPerRow: return gap_info<R, MU, kGapsPerRow>(prec, same, variant);
+    case kGapsUniform: return gap_info<R, MU, kGapsUniform>(prec, same, variant);
+    default: return gap_info<R, MU, kGapsConst>(prec, same, variant);
+  }
 }
 
 }  // namespace rodv

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "layout.h"
+
 namespace rodv {
 
 enum class Precision { kF32x2 = 0, kF64 = 1 };
@@ -49,7 +51,7 @@ constexpr int kMaxGroupedRows = 4;  // classes with R <= 4 have the grouped vari
 // single-pass kernels, and of every multi-pass kernel (FP32 same and
 // two-haplotype items share the class's variant, so they agree on the pass
 // count; FP64 ones have their own).
-KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, bool uniform, bool multi,
+KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, GapForm gaps, bool multi,
                                bool same = true, int variant = 0);
 inline int forward_kernel_variants(Precision prec, bool same, int rows_per_lane = 8,
                                    bool multi = true) {

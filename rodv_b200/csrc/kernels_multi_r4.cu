@@ -3,5 +3,5 @@
 #include "kernel_table.cuh"
 
 namespace rodv {
-template KernelInfo pipe_info_for<4>(Precision, bool, bool, int);
+template KernelInfo pipe_info_for<4>(Precision, GapForm, bool, int);
 }  // namespace rodv

@@ -3,5 +3,5 @@
 #include "kernel_table.cuh"
 
 namespace rodv {
-template KernelInfo pipe_info_for<8>(Precision, bool, bool, int);
+template KernelInfo pipe_info_for<8>(Precision, GapForm, bool, int);
 }  // namespace rodv

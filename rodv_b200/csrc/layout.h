@@ -28,6 +28,8 @@
 //   out        f64[num_pairs]  final log10 likelihood, in the reference's
 //              result order (region, hap-major, read-minor)
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 #if defined(__CUDACC__)
@@ -142,6 +144,24 @@ struct PriorTables {
   const double* mm_d;
 };
 
+// How a class's kernels get the gap priors (ins, del and gcp) of their reads.
+// kGapsPerRow: per read row.  kGapsUniform: one set per read (the scaled
+// form), in registers.  kGapsConst: one set for every uniform-gap read of the
+// launch (GapConsts), the same scaled form.
+enum GapForm : int { kGapsPerRow = 0, kGapsUniform = 1, kGapsConst = 2 };
+
+// The gap priors of kGapsConst launches, kernel parameters so that the sweep's
+// FMAs take the M-to-M coefficient mm/c and the gap continuation ii from the
+// constant bank.  An f32x2 FMA with three distinct register operands issues
+// every 2.9 cycles on B200 (one 64-bit register operand a cycle), with two
+// every 2.0-2.2: a chain step of R = 8 rows alone, without loads and shuffles,
+// takes 101 cycles with both in registers and 89 with both constant.
+struct GapConsts {
+  float2 mm2, ii2;              // (mm/c, mm/c), (ii, ii): f32x2 operands
+  float mi, c;                  // c = mi * (1 - ii), the emission scale
+  double mm_d, ii_d, mi_d, c_d;  // the same for the FP64 kernels
+};
+
 // Everything a forward kernel needs about the resident batch.
 struct BatchView {
   const uint8_t* hap_codes;
@@ -171,6 +191,7 @@ struct ClassLaunch {
   uint32_t wait_polls;         // pipelined sweeps: polls before a wait gives up (0: default)
   uint32_t rescue_base;        // kLaunchRescueByItem: list position of item 0's first pair
   const uint32_t* stack;       // chain items: their read pairs (read indices)
+  GapConsts gaps;              // kGapsConst kernels
 };
 
 // ClassLaunch::flags.  Testing hook: the producers of a pipelined sweep

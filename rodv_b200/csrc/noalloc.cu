@@ -60,8 +60,8 @@ constexpr uint64_t kNaMaxHapBases = RODV_NOALLOC_MAX_HAP_BASES;
 constexpr uint64_t kNaMaxReadBases = RODV_NOALLOC_MAX_READ_BASES;
 // The two forward kernels of this call: the multi-pass FP32 kernel with
 // per-row gap priors and its FP64 rescue.
-using NaF32 = Forward<F32x2, kMaxRowsPerLane, false, true, false, 1>;
-using NaF64 = Forward<F64, kMaxRowsPerLane, false, true, false, 1>;
+using NaF32 = Forward<F32x2, kMaxRowsPerLane, kGapsPerRow, true, false, 1>;
+using NaF64 = Forward<F64, kMaxRowsPerLane, kGapsPerRow, true, false, 1>;
 constexpr int kNaBlocks = 32;                    // forward kernels' fixed grid
 // resident warps owning boundary rows
 constexpr int kNaWarps = kNaBlocks * (NaF32::kWarpsPerBlock > NaF64::kWarpsPerBlock
@@ -352,10 +352,10 @@ cudaError_t setup_device(int dev, unsigned char** out) {
       // the two kernels' shared memory (tables and boundary ring) may exceed
       // the default 48 KB per block
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(&forward_kernel<F32x2, kMaxRowsPerLane, false, true, false, 1>,
+        e = cudaFuncSetAttribute(&forward_kernel<F32x2, kMaxRowsPerLane, kGapsPerRow, true, false, 1>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF32);
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(&forward_kernel<F64, kMaxRowsPerLane, false, true, false, 1>,
+        e = cudaFuncSetAttribute(&forward_kernel<F64, kMaxRowsPerLane, kGapsPerRow, true, false, 1>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF64);
     }
     if (e == cudaSuccess) slot.ptr = static_cast<unsigned char*>(p);
@@ -453,7 +453,7 @@ extern "C" rodv_status rodv_pairhmm_batch_noalloc(const rodv_batch* batch, int32
   c32.scratch = reinterpret_cast<float*>(s + kOffBoundary);
   c32.scratch_cols = kNaCols;
   c32.error_flags = cnt + kCErr;
-  forward_kernel<F32x2, kMaxRowsPerLane, false, true, false, 1>
+  forward_kernel<F32x2, kMaxRowsPerLane, kGapsPerRow, true, false, 1>
       <<<kNaBlocks, F32::kWarpsPerBlock * kWarp,
          F32::kWarpsPerBlock * F32::kSmemPerWarp, st>>>(
           v, c32);
@@ -463,7 +463,7 @@ extern "C" rodv_status rodv_pairhmm_batch_noalloc(const rodv_batch* batch, int32
   c64.counter = cnt + kCCtr64;
   c64.rescue_list = nullptr;
   c64.rescue_count = nullptr;
-  forward_kernel<F64, kMaxRowsPerLane, false, true, false, 1>
+  forward_kernel<F64, kMaxRowsPerLane, kGapsPerRow, true, false, 1>
       <<<kNaBlocks, D64::kWarpsPerBlock * kWarp,
          D64::kWarpsPerBlock * D64::kSmemPerWarp, st>>>(
           v, c64);

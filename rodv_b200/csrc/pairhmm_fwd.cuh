@@ -172,6 +172,26 @@ struct Tables<double> {
   __device__ __forceinline__ static const double* mm(const PriorTables& t) { return t.mm_d; }
 };
 
+// The launch's gap priors in a kernel's precision (kGapsConst).
+template <class S>
+struct ConstGaps;
+template <>
+struct ConstGaps<float> {
+  __device__ __forceinline__ static float2 mm_operand(const GapConsts& g) { return g.mm2; }
+  __device__ __forceinline__ static float2 ii_operand(const GapConsts& g) { return g.ii2; }
+  __device__ __forceinline__ static float ii(const GapConsts& g) { return g.ii2.x; }
+  __device__ __forceinline__ static float mi(const GapConsts& g) { return g.mi; }
+  __device__ __forceinline__ static float c(const GapConsts& g) { return g.c; }
+};
+template <>
+struct ConstGaps<double> {
+  __device__ __forceinline__ static double mm_operand(const GapConsts& g) { return g.mm_d; }
+  __device__ __forceinline__ static double ii_operand(const GapConsts& g) { return g.ii_d; }
+  __device__ __forceinline__ static double ii(const GapConsts& g) { return g.ii_d; }
+  __device__ __forceinline__ static double mi(const GapConsts& g) { return g.mi_d; }
+  __device__ __forceinline__ static double c(const GapConsts& g) { return g.c_d; }
+};
+
 // Priors of one read row (pairhmm_impl.cpp:88-115, pairhmm_inter.cpp:83-98).
 template <class S>
 struct RowPriors {
@@ -244,7 +264,7 @@ struct ChainMeta {
 // GROUP: lanes per wavefront.  32 (the whole warp) for every kernel but the
 // chain kernels of short reads, which split the warp into two 16-lane groups
 // with twice the rows per lane, each sweeping its own chain item.
-template <class P, int R, bool UNIFORM, bool MULTI, bool SAME, int MINB, int GROUP = 32>
+template <class P, int R, int GAPS, bool MULTI, bool SAME, int MINB, int GROUP = 32>
 struct Forward {
   using V = typename P::V;
   using S = typename P::S;
@@ -264,7 +284,9 @@ struct Forward {
   // of the 2^1020 scaling's underflow limit (log10 about -615, below which
   // the reference returns -inf); there M keeps at least 32 of its 52
   // mantissa bits (37 at ins = del = 45, gcp = 10), 1e-10 relative or better.
-  static constexpr bool kScaled = UNIFORM;
+  static constexpr bool kScaled = GAPS != kGapsPerRow;
+  // gap priors from the launch's constants (layout.h, GapConsts)
+  static constexpr bool kConst = GAPS == kGapsConst;
   static constexpr int kWarpsPerBlock = 4;
   // Multi-pass kernels also keep a ring of 2 x 32 boundary cells per warp
   // (the next 32 columns of the previous pass's last row, see run_item).
@@ -289,11 +311,11 @@ struct Forward {
   };
 
   // Transition priors of this lane's R rows (per row, or the read's uniform
-  // values), both slots packed.
+  // values), both slots packed.  kConst: mmU and ddU are kernel parameters.
   struct Priors {
-    V mm[UNIFORM ? 1 : R], gapm[UNIFORM ? 1 : R], md[UNIFORM ? 1 : R];
-    V mi[R], ii[R];
-    V mmU, mdU, ddU;
+    V mm[kScaled ? 1 : R], gapm[kScaled ? 1 : R], mi[kScaled ? 1 : R], md[kScaled ? 1 : R];
+    V ii[R];
+    V mmU, ddU;  // kScaled: the uniform mm/c and ii
     V iiN;  // kScaled: ii of the next lane's first row (the row below this lane's last)
   };
 
@@ -318,7 +340,7 @@ struct Forward {
   // first_row[s] + [0, R) of the two slots s (reads of L[s] rows starting at
   // row word row_off[s]).
   // Rows past a read's end are pass-through rows: emission 0, mi = ii = 1,
-  // md = 0 (in the uniform form mi*gapm = gapm, since M~ = M/gapm).
+  // md = 0.
   //
   // Scaled form (kScaled; uniform gaps with mi == md).  With c = mi*gapm the
   // sweep keeps M~ = M/gapm, I^ = I/c, D^ = D/c of a DP whose row 0 holds
@@ -336,25 +358,35 @@ struct Forward {
   // overflow for likely pairs on short haplotypes.)
   // sum_lane (scaled form, chain sweeps): this lane's last row is a pair's
   // sum row, a pass-through row with emission 1 for every code (run_chain).
-  __device__ __forceinline__ static void load_rows(const BatchView& b, const uint32_t (&L)[2],
+  __device__ __forceinline__ static void load_rows(const BatchView& b, const GapConsts& gaps,
+                                                   const uint32_t (&L)[2],
                                                    const uint64_t (&row_off)[2],
                                                    const uint32_t (&first_row)[2], int lane,
                                                    uint4* table, Priors& p,
                                                    bool sum_lane = false) {
-    RowPriors<S> u[2];
-    S cs[2] = {S(1), S(1)};  // emission scale of rows before the last (kScaled)
-    if (UNIFORM) {  // uniform-gap priors come from the read's first row
-      u[0] = row_priors<S>(b.read_rows[row_off[0]], b.tab);
-      u[1] = row_priors<S>(b.read_rows[row_off[1]], b.tab);
-      if (kScaled) {
-        cs[0] = u[0].mi * u[0].gapm;
-        cs[1] = u[1].mi * u[1].gapm;
-        p.mmU = P::make(u[0].mm / cs[0], u[1].mm / cs[1]);
-      } else {
-        p.mmU = P::make(u[0].mm, u[1].mm);
-        p.mdU = P::make(u[0].md * u[0].gapm, u[1].md * u[1].gapm);
+    // kScaled: the reads' uniform mi and ii, and the emission scale c
+    S miU[2] = {S(0), S(0)}, iiU[2] = {S(0), S(0)}, cs[2] = {S(1), S(1)};
+    if constexpr (kConst) {
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        miU[s] = ConstGaps<S>::mi(gaps);
+        iiU[s] = ConstGaps<S>::ii(gaps);
+        cs[s] = ConstGaps<S>::c(gaps);
       }
-      p.ddU = P::make(u[0].ii, u[1].ii);
+      p.mmU = ConstGaps<S>::mm_operand(gaps);
+      p.ddU = ConstGaps<S>::ii_operand(gaps);
+    } else if constexpr (kScaled) {  // uniform-gap priors come from the read's first row
+      S mm[2];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const RowPriors<S> u = row_priors<S>(b.read_rows[row_off[s]], b.tab);
+        miU[s] = u.mi;
+        iiU[s] = u.ii;
+        cs[s] = u.mi * u.gapm;
+        mm[s] = u.mm / cs[s];
+      }
+      p.mmU = P::make(mm[0], mm[1]);
+      p.ddU = P::make(iiU[0], iiU[1]);
     }
     S* tab = reinterpret_cast<S*>(table);
 #pragma unroll
@@ -376,10 +408,7 @@ struct Forward {
         }
         put_emission(tab, s, kSep, k, lane, S(0));
         if (kScaled) {
-          iiv[s] = real ? u[s].ii : (row == L[s] ? u[s].mi : S(1));
-        } else if (UNIFORM) {
-          miv[s] = real ? u[s].mi * u[s].gapm : u[s].gapm;
-          iiv[s] = real ? u[s].ii : S(1);
+          iiv[s] = real ? iiU[s] : (row == L[s] ? miU[s] : S(1));
         } else {
           mmv[s] = real ? rp.mm : S(0);
           gv[s] = real ? rp.gapm : S(0);
@@ -389,15 +418,17 @@ struct Forward {
         }
       }
       if (P::kSlots == 1) {
-        miv[1] = miv[0]; iiv[1] = iiv[0];
-        mmv[1] = mmv[0]; gv[1] = gv[0]; mdv[1] = mdv[0];
+        iiv[1] = iiv[0];
+        if (!kScaled) {
+          miv[1] = miv[0]; mmv[1] = mmv[0]; gv[1] = gv[0]; mdv[1] = mdv[0];
+        }
       }
-      p.mi[k] = P::make(miv[0], miv[1]);
       p.ii[k] = P::make(iiv[0], iiv[1]);
-      if (!UNIFORM) {
-        p.mm[UNIFORM ? 0 : k] = P::make(mmv[0], mmv[1]);
-        p.gapm[UNIFORM ? 0 : k] = P::make(gv[0], gv[1]);
-        p.md[UNIFORM ? 0 : k] = P::make(mdv[0], mdv[1]);
+      if constexpr (!kScaled) {
+        p.mi[k] = P::make(miv[0], miv[1]);
+        p.mm[k] = P::make(mmv[0], mmv[1]);
+        p.gapm[k] = P::make(gv[0], gv[1]);
+        p.md[k] = P::make(mdv[0], mdv[1]);
       }
     }
     if (kScaled && sum_lane) {
@@ -411,7 +442,7 @@ struct Forward {
 #pragma unroll
       for (int s = 0; s < 2; ++s) {
         const uint32_t row = first_row[s] + R;
-        iin[s] = row < L[s] ? u[s].ii : (row == L[s] ? u[s].mi : S(1));
+        iin[s] = row < L[s] ? iiU[s] : (row == L[s] ? miU[s] : S(1));
       }
       p.iiN = P::make(iin[0], iin[1]);
     }
@@ -469,7 +500,7 @@ struct Forward {
     for (int k = 0; k < R; ++k) {
       const V oM = M[k], oI = I[k], oD = D[k];
       V t = P::add(di, dd);
-      if (UNIFORM) {
+      if constexpr (kScaled) {
         t = P::fma(p.mmU, dm, t);
       } else {
         t = P::mul(p.gapm[k], t);
@@ -481,16 +512,12 @@ struct Forward {
         M[k] = P::make(P::sx(t) * P::sx(e[k]), P::sy(t) * P::sy(e[k]));
       }
       if (k == R - 1) t_last = t;
-      if (kScaled) {
+      if constexpr (kScaled) {
         I[k] = P::fma(p.ii[k], ui, um);
         D[k] = P::fma(p.ddU, oD, oM);
       } else {
         I[k] = P::fma(p.ii[k], ui, P::mul(p.mi[k], um));
-        if (UNIFORM) {
-          D[k] = P::fma(p.ddU, oD, P::mul(p.mdU, oM));
-        } else {
-          D[k] = P::fma(p.ii[k], oD, P::mul(p.md[k], oM));
-        }
+        D[k] = P::fma(p.ii[k], oD, P::mul(p.md[k], oM));
       }
       dm = oM; di = oI; dd = oD;
       um = M[k]; ui = I[k];
@@ -507,7 +534,10 @@ struct Forward {
   // ii == dd, the value cells() uses), and 1 on pass-through rows below row
   // L, where M is 0 and D stays 0 -- except on a chain sweep's sum row, whose
   // emission 1 makes its M the pass-through value one column back and its D
-  // the exact running sum of the earlier ones (run_chain).
+  // the exact running sum of the earlier ones (run_chain).  kConst: every row
+  // but the last takes the launch's ii instead (a constant operand), which is
+  // the same value on the read's rows, and D stays 0 below them; only the last
+  // row can be a sum row.
   __device__ __forceinline__ static void cells_scaled(const V (&e)[R], V t0, V i0, V (&M)[R],
                                                       V (&I)[R], V (&D)[R], const Priors& p,
                                                       V& t_last) {
@@ -519,7 +549,7 @@ struct Forward {
       M[k] = P::mul(t, e[k]);
       if (k == R - 1) t_last = t;
       I[k] = k == 0 ? i0 : P::fma(p.ii[k], ui, um);
-      D[k] = P::fma(p.ii[k], oD, oM);
+      D[k] = P::fma(kConst && k < R - 1 ? p.ddU : p.ii[k], oD, oM);
       dm = oM; di = oI; dd = oD;
       um = M[k]; ui = I[k];
     }
@@ -544,10 +574,18 @@ struct Forward {
     }
   }
 
-  // gapm of a uniform-gap read (every row has the same gcp quality).
-  __device__ __forceinline__ static S uniform_gapm(const BatchView& b, uint32_t read) {
-    const uint32_t w = b.read_rows[b.reads[read].row_off];
-    return S(1) - __ldg(Tables<S>::ph2pr(b.tab) + rw_gcp(w));
+  // mi and 1 - ph2pr[gcp] of a uniform-gap read, in FP64 from the kernel's
+  // tables.
+  __device__ __forceinline__ static void read_gaps(const BatchView& b, const GapConsts& gaps,
+                                                   uint32_t read, double* mi, double* gapm) {
+    if constexpr (kConst) {
+      *mi = (double)ConstGaps<S>::mi(gaps);
+      *gapm = 1.0 - (double)ConstGaps<S>::ii(gaps);
+    } else {
+      const uint32_t w = b.read_rows[b.reads[read].row_off];
+      *mi = (double)__ldg(Tables<S>::ph2pr(b.tab) + rw_ins(w));
+      *gapm = 1.0 - (double)__ldg(Tables<S>::ph2pr(b.tab) + rw_gcp(w));
+    }
   }
 
   // The scaled form's likelihood from the last register's column sums of
@@ -556,12 +594,12 @@ struct Forward {
   // about c = mi*gapm times smaller than the reference's FP32 sweep, so its
   // bound is 1e-28/c: an accepted result keeps the reference's headroom above
   // the FP32 denormal range (below the bound, the pair goes to FP64).
-  __device__ __forceinline__ static double scaled_result(const BatchView& b, uint32_t read,
+  __device__ __forceinline__ static double scaled_result(const BatchView& b,
+                                                         const GapConsts& gaps, uint32_t read,
                                                          uint32_t len, uint32_t rows, S acc_m,
                                                          S acc_i, double* accept_min) {
-    const uint32_t w = b.read_rows[b.reads[read].row_off];
-    const double mi = (double)__ldg(Tables<S>::ph2pr(b.tab) + rw_ins(w));
-    const double gapm = 1.0 - (double)__ldg(Tables<S>::ph2pr(b.tab) + rw_gcp(w));
+    double mi, gapm;
+    read_gaps(b, gaps, read, &mi, &gapm);
     *accept_min = (double)kMinAcceptedF / (mi * gapm);
     return len < rows ? (double)acc_i / mi : (double)acc_m / mi + (double)acc_i;
   }
@@ -620,16 +658,13 @@ struct Forward {
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       if (s == 1 && refs[1].read == kNoPair) continue;
-      const uint32_t w = b.read_rows[b.reads[refs[s].read].row_off];
-      const double mi = (double)__ldg(Tables<S>::ph2pr(b.tab) + rw_ins(w));
-      const double gapm = 1.0 - (double)__ldg(Tables<S>::ph2pr(b.tab) + rw_gcp(w));
       double bound, amin = (double)kMinAcceptedF;
       if (kScaled) {
         // M~ = mi * M and I^ = I; a pass-through row holds mi * (M_L + I_L) in I^
+        double mi, gapm;
+        read_gaps(b, c.gaps, refs[s].read, &mi, &gapm);
         bound = row < L[s] ? sum_m[s] / mi + sum_i[s] : sum_i[s] / mi;
         amin /= mi * gapm;
-      } else if (UNIFORM) {
-        bound = gapm * sum_m[s] + sum_i[s];  // M is kept divided by gapm
       } else {
         bound = sum_m[s] + sum_i[s];
       }
@@ -701,7 +736,7 @@ struct Forward {
       const bool last = (pass + 1 == passes);
       Priors pr;
       const uint32_t fr = pass * (kWarp * R) + lane * R;
-      load_rows(b, L, row_off, {fr, fr}, lane, table, pr);
+      load_rows(b, c.gaps, L, row_off, {fr, fr}, lane, table, pr);
 
       V M[R], I[R], D[R];
 #pragma unroll
@@ -783,12 +818,9 @@ struct Forward {
     double amin[2] = {(double)kMinAcceptedF, (double)kMinAcceptedF};
     if (kScaled) {
       const uint32_t rows = passes * kWarp * R;
-      res[0] = scaled_result(b, fr[0].read, L[0], rows, P::sx(acc_m), P::sx(acc_i), &amin[0]);
+      res[0] = scaled_result(b, c.gaps, fr[0].read, L[0], rows, P::sx(acc_m), P::sx(acc_i), &amin[0]);
       if (valid_y)
-        res[1] = scaled_result(b, fr[1].read, L[1], rows, frozen_m, frozen_i, &amin[1]);
-    } else if (UNIFORM) {
-      res[0] = uniform_gapm(b, fr[0].read) * P::sx(acc_m) + P::sx(acc_i);
-      if (valid_y) res[1] = uniform_gapm(b, fr[1].read) * frozen_m + frozen_i;
+        res[1] = scaled_result(b, c.gaps, fr[1].read, L[1], rows, frozen_m, frozen_i, &amin[1]);
     } else {
       res[0] = P::sx(acc_m) + P::sx(acc_i);
       res[1] = frozen_m + frozen_i;
@@ -916,7 +948,7 @@ struct Forward {
     const V init = P::make(init_s, init_s);
     Priors pr;
     const uint32_t fr = (uint32_t)lag * R;  // this lane's first row in its pair's reads
-    load_rows(b, L, row_off, {fr, fr}, lane, table, pr, (uint32_t)lag == nl - 1);
+    load_rows(b, c.gaps, L, row_off, {fr, fr}, lane, table, pr, (uint32_t)lag == nl - 1);
     __syncwarp();
 
     const bool top = lag == 0;  // a pair's first lane
@@ -1034,7 +1066,7 @@ struct Forward {
           double res, amin = (double)kMinAcceptedF;
           if (kScaled) {  // the pass-through row holds (M_L + I_L)/gapm: the sum / mi
             const uint32_t len = b.reads[read[s]].len;
-            res = scaled_result(b, read[s], len, len + 1, S(0), sum, &amin);
+            res = scaled_result(b, c.gaps, read[s], len, len + 1, S(0), sum, &amin);
           } else {        // the pass-through row holds M_L + I_L (its M is 0)
             res = sum;
           }
@@ -1088,11 +1120,11 @@ struct Forward {
   }
 };
 
-template <class P, int R, bool UNIFORM, bool MULTI, bool SAME, int MINB, int GROUP = 32>
+template <class P, int R, int GAPS, bool MULTI, bool SAME, int MINB, int GROUP = 32>
 __global__ void __launch_bounds__(
-    Forward<P, R, UNIFORM, MULTI, SAME, MINB, GROUP>::kWarpsPerBlock * kWarp, MINB)
+    Forward<P, R, GAPS, MULTI, SAME, MINB, GROUP>::kWarpsPerBlock * kWarp, MINB)
     forward_kernel(BatchView b, ClassLaunch c) {
-  using F = Forward<P, R, UNIFORM, MULTI, SAME, MINB, GROUP>;
+  using F = Forward<P, R, GAPS, MULTI, SAME, MINB, GROUP>;
   extern __shared__ uint4 smem[];
   const int lane = threadIdx.x & (kWarp - 1);
   const int warp = threadIdx.x / kWarp;

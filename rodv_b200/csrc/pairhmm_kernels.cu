@@ -9,26 +9,26 @@
 namespace rodv {
 
 template <int R, bool MU>
-KernelInfo info_for(Precision prec, bool uniform, bool same, int variant);
+KernelInfo info_for(Precision prec, GapForm gaps, bool same, int variant);
 template <int R>
-KernelInfo pipe_info_for(Precision prec, bool uniform, bool same, int variant);
+KernelInfo pipe_info_for(Precision prec, GapForm gaps, bool same, int variant);
 
-KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, bool uniform, bool multi,
+KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, GapForm gaps, bool multi,
                                bool same, int variant) {
   if (multi) {
     const int v = variant >= 0 && variant < kPipeVariants ? variant : 0;
-    return pipe_variant_rows(v) == 4 ? pipe_info_for<4>(prec, uniform, same, v)
-                                     : pipe_info_for<8>(prec, uniform, same, v);
+    return pipe_variant_rows(v) == 4 ? pipe_info_for<4>(prec, gaps, same, v)
+                                     : pipe_info_for<8>(prec, gaps, same, v);
   }
   switch (rows_per_lane) {
-    case 1: return info_for<1, false>(prec, uniform, same, variant);
-    case 2: return info_for<2, false>(prec, uniform, same, variant);
-    case 3: return info_for<3, false>(prec, uniform, same, variant);
-    case 4: return info_for<4, false>(prec, uniform, same, variant);
-    case 5: return info_for<5, false>(prec, uniform, same, variant);
-    case 6: return info_for<6, false>(prec, uniform, same, variant);
-    case 7: return info_for<7, false>(prec, uniform, same, variant);
-    default: return info_for<8, false>(prec, uniform, same, variant);
+    case 1: return info_for<1, false>(prec, gaps, same, variant);
+    case 2: return info_for<2, false>(prec, gaps, same, variant);
+    case 3: return info_for<3, false>(prec, gaps, same, variant);
+    case 4: return info_for<4, false>(prec, gaps, same, variant);
+    case 5: return info_for<5, false>(prec, gaps, same, variant);
+    case 6: return info_for<6, false>(prec, gaps, same, variant);
+    case 7: return info_for<7, false>(prec, gaps, same, variant);
+    default: return info_for<8, false>(prec, gaps, same, variant);
   }
 }
 

@@ -87,9 +87,9 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gmem) : "memory");
 }
 
-template <class P, int R, bool UNIFORM, bool SAME, int MINB, int W>
+template <class P, int R, int GAPS, bool SAME, int MINB, int W>
 struct PipeForward {
-  using F = Forward<P, R, UNIFORM, true, SAME, MINB>;
+  using F = Forward<P, R, GAPS, true, SAME, MINB>;
   using V = typename P::V;
   using S = typename P::S;
   static constexpr bool kTwo = F::kScaled;  // two-value hand-over (t, i)
@@ -175,9 +175,8 @@ struct PipeForward {
       for (int s = 0; s < 2; ++s) {
         if (s == 1 && refs[1].read == kNoPair) continue;
         const uint32_t w = b.read_rows[b.reads[refs[s].read].row_off];
-        const S* ph2pr = Tables<S>::ph2pr(b.tab);
-        const double mi = (double)__ldg(ph2pr + rw_ins(w));
-        const double gapm = 1.0 - (double)__ldg(ph2pr + rw_gcp(w));
+        double mi, gapm;
+        F::read_gaps(b, c.gaps, refs[s].read, &mi, &gapm);
         const double mm = (double)row_priors<S>(w, b.tab).mm;
         const double bound = row < L[s] ? (gapm > mm ? gapm / mm : 1.0) * sum[s] : sum[s] / mi;
         const double amin = (double)kMinAcceptedF / (mi * gapm);  // as scaled_result's
@@ -276,7 +275,7 @@ struct PipeForward {
 
       typename F::Priors pr;
       const uint32_t fr = p * (kWarp * R) + lane * R;
-      F::load_rows(b, L, row_off, {fr, fr}, lane, table, pr);
+      F::load_rows(b, c.gaps, L, row_off, {fr, fr}, lane, table, pr);
       V M[R], I[R], D[R];
 #pragma unroll
       for (int k = 0; k < R; ++k) M[k] = I[k] = D[k] = P::zero();
@@ -422,8 +421,8 @@ struct PipeForward {
     double res[2] = {0.0, 0.0};
     double amin[2] = {(double)kMinAcceptedF, (double)kMinAcceptedF};
     if (F::kScaled) {
-      res[0] = F::scaled_result(b, fr[0].read, Lx, rows, S(0), P::sx(sm.acc), &amin[0]);
-      if (valid_y) res[1] = F::scaled_result(b, fr[1].read, Ly, rows, S(0), fy, &amin[1]);
+      res[0] = F::scaled_result(b, c.gaps, fr[0].read, Lx, rows, S(0), P::sx(sm.acc), &amin[0]);
+      if (valid_y) res[1] = F::scaled_result(b, c.gaps, fr[1].read, Ly, rows, S(0), fy, &amin[1]);
     } else {
       // the pass-through row holds M_L + I_L in its I (non-uniform form)
       res[0] = P::sx(sm.acc);
@@ -436,10 +435,10 @@ struct PipeForward {
 
 // One work item per block at a time; c.scratch holds kRows boundary rows of
 // c.scratch_cols cells for every block of the grid.
-template <class P, int R, bool UNIFORM, bool SAME, int MINB, int W>
+template <class P, int R, int GAPS, bool SAME, int MINB, int W>
 __global__ void __launch_bounds__(W * kWarp, MINB)
     forward_pipe_kernel(BatchView b, ClassLaunch c) {
-  using F = PipeForward<P, R, UNIFORM, SAME, MINB, W>;
+  using F = PipeForward<P, R, GAPS, SAME, MINB, W>;
   extern __shared__ uint4 smem[];
   __shared__ typename F::Ctl ctl;
   const int lane = threadIdx.x & (kWarp - 1);
