@@ -488,7 +488,7 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   // haplotype code buffer: [pad][hap 0][sep][hap 1][sep]...[hap n-1][sep]
   // [pad + max len + pad]; any run of consecutive haplotypes is one chain.
   std::vector<uint64_t> hap_code_off(b.num_haps);
-  uint64_t hb = kHapPad;
+  uint64_t hb = kHapFrontPad;
   uint32_t max_h = 0;
   for (uint32_t h = 0; h < b.num_haps; ++h) {
     const uint32_t len = b.hap_lengths[h];
@@ -804,7 +804,7 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
       hd[h].pad_ = 0;
     }
   });
-  std::memset(codes, 0, kHapPad);
+  std::memset(codes, 0, kHapFrontPad);
   std::memset(codes + tail_begin, 0, hb - tail_begin);
   timer.mark("haps");
   // ---- read rows ----

@@ -5,7 +5,7 @@
 //
 //   hap_codes  u8   the haplotypes in batch order as base codes A0 C1 G2 T3
 //                   N4, one separator code (kSep) between consecutive
-//                   haplotypes, kHapPad code-0 bytes before the first; the
+//                   haplotypes, kHapFrontPad code-0 bytes before the first; the
 //                   tail holds kHapPad + max_hap_len + kHapPad more, so a warp
 //                   whose shorter slot runs past its haplotype end still
 //                   reads in bounds.  Any run of consecutive haplotypes is
@@ -41,7 +41,10 @@
 namespace rodv {
 
 constexpr int kWarp = 32;
-constexpr int kHapPad = 32;          // code bytes before the first haplotype
+constexpr int kHapPad = 32;          // code bytes after the last haplotype (twice)
+// code bytes before the first haplotype: lane 31 of an FP64 sweep starts 62
+// columns behind lane 0
+constexpr int kHapFrontPad = 64;
 constexpr int kChainHaps = 32;       // haplotypes per chain item (one per lane)
 constexpr int kMaxRowsPerLane = 8;   // R: read rows held in registers per lane
 constexpr int kPassRows = kWarp * kMaxRowsPerLane;  // rows per multi-pass sweep

@@ -489,6 +489,13 @@ struct Forward {
     }
   }
 
+  // t * e: the M of a cell.  The DIFF layout's emissions come from two tables
+  // and are multiplied slot by slot.
+  __device__ __forceinline__ static V emit(V t, V e) {
+    if constexpr (kSameHap) return P::mul(t, e);
+    else return P::make(P::sx(t) * P::sx(e), P::sy(t) * P::sy(e));
+  }
+
   // One column of this lane's R rows.  (M, I, D)[k] hold the previous
   // column on entry (the left neighbours) and this column on exit; dg is the
   // row above the lane's first row at the previous column, up the same row
@@ -508,11 +515,7 @@ struct Forward {
         t = P::mul(p.gapm[k], t);
         t = P::fma(p.mm[k], dm, t);
       }
-      if (kSameHap) {
-        M[k] = P::mul(t, e[k]);
-      } else {
-        M[k] = P::make(P::sx(t) * P::sx(e[k]), P::sy(t) * P::sy(e[k]));
-      }
+      M[k] = emit(t, e[k]);
       if (k == R - 1) t_last = t;
       if constexpr (kScaled) {
         I[k] = P::fma(p.ii[k], ui, um);
@@ -548,7 +551,7 @@ struct Forward {
     for (int k = 0; k < R; ++k) {
       const V oM = M[k], oI = I[k], oD = D[k];
       const V t = k == 0 ? t0 : P::fma(p.mmU, dm, P::add(di, dd));
-      M[k] = P::mul(t, e[k]);
+      M[k] = emit(t, e[k]);
       if (k == R - 1) t_last = t;
       I[k] = k == 0 ? i0 : P::fma(p.ii[k], ui, um);
       D[k] = P::fma(kConst && k < R - 1 ? p.ddU : p.ii[k], oD, oM);
@@ -829,6 +832,100 @@ struct Forward {
     }
     finish(b, c, fr[0], res[0], amin[0]);
     if (valid_y) finish(b, c, fr[1], res[1], amin[1]);
+  }
+
+  // One pair per slot (DiffItem or, for F64, PairRef) in one sweep, scaled
+  // form.  The lanes hand over two values a step, as in a chain sweep
+  // (cells_scaled), and lane 31's last row is the sum row, so no running sum
+  // is kept: D + M of that row at the column after a slot's last one is its
+  // sum.  FP64 lanes lag their left neighbour by two columns (kLag): a value
+  // shuffled in one step is used in the next, so the shuffle's latency is off
+  // the step's dependency chain (R = 8, constant gaps: 106 cycles a step with
+  // four warps a sub-partition and 111 for a lone warp; 112 and 149 at a lag
+  // of one column, which FP32 keeps for its 31 fewer steps).  Measured on
+  // 40,000 pairs of 250 x 400 bases: FP32 pass 1.11 -> 0.91 ms, FP64 pass 2.00
+  // -> 1.72 ms; 124 registers in FP64 where three values and two running sums
+  // took 166.
+  __device__ static void run_single(const BatchView& b, const ClassLaunch& c, uint32_t item,
+                                    int lane, uint4* table) {
+    constexpr int kLag = P::kSlots == 1 ? 2 : 1;
+    PairRef refs[2];
+    load_refs(c, item, refs);
+    SlotInfo sl[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const PairRef r = s == 0 || refs[1].read != kNoPair ? refs[s] : refs[0];
+      const HapDesc hd = b.haps[r.hap];
+      const ReadDesc rd = b.reads[r.read];
+      sl[s] = SlotInfo{b.hap_codes + hd.code_off, hd.len, rd.len, rd.row_off};
+    }
+    const uint32_t L[2] = {sl[0].L, sl[1].L};
+    const uint64_t row_off[2] = {sl[0].row_off, sl[1].row_off};
+    // slot x has the longer haplotype; a pass-through and the sum row fit
+    if (sl[1].H == 0 || sl[1].H > sl[0].H || L[0] == 0 || L[1] == 0 ||
+        max(L[0], L[1]) + 2 > (uint32_t)(kWarp * R)) {
+      if (lane == 0) atomicOr(c.error_flags, kErrBadLength);
+      return;
+    }
+    const V init = P::make(P::init_const() / (S)sl[0].H, P::init_const() / (S)sl[1].H);
+    Priors pr;
+    const uint32_t fr = (uint32_t)lane * R;
+    load_rows(b, c.gaps, L, row_off, {fr, fr}, lane, table, pr, lane == kWarp - 1);
+    __syncwarp();
+    const bool top = lane == 0;
+    V M[R], I[R], D[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) M[k] = I[k] = D[k] = P::zero();
+    V dg_t = top ? init : P::zero();  // the first row's M term of the previous column
+    // kLag 2: this column's hand-over, shuffled in the previous step
+    V next_t = top ? init : P::zero(), next_i = P::zero();
+    const uint8_t* hx = sl[0].hap - kLag * lane;
+    const uint8_t* hy = sl[1].hap - kLag * lane;
+    // lane 31 is at column H + 1 in step H + 31 kLag
+    const int nsteps = (int)sl[0].H + kLag * (kWarp - 1) + 1;
+    S sum_y = S(0);
+    int s = 0;
+    // codes of the next step, loaded one step ahead
+    uint32_t cx_next = hx[0], cy_next = kSameHap ? 0u : (uint32_t)hy[0];
+#pragma unroll 1
+    for (int part = kSameHap ? 1 : 0; part < 2; ++part) {
+      const int end = part == 0 ? (int)sl[1].H + kLag * (kWarp - 1) + 1 : nsteps;
+#pragma unroll 4
+      for (; s < end; ++s) {
+        const uint32_t cx = cx_next, cy = cy_next;
+        cx_next = hx[s + 1];
+        if (!kSameHap) cy_next = hy[s + 1];
+        V in_t = P::shfl_up(P::fma(pr.mmU, M[R - 1], P::add(I[R - 1], D[R - 1])));
+        V in_i = P::shfl_up(P::fma(pr.iiN, I[R - 1], M[R - 1]));
+        if (top) {
+          in_t = init; in_i = P::zero();
+        }
+        if (kLag == 2) {
+          const V t = in_t, i = in_i;
+          in_t = next_t; in_i = next_i;
+          next_t = t; next_i = i;
+        }
+        V e[R], t_last;
+        load_emission(table, lane, cx, cy, e);
+        cells_scaled(e, dg_t, in_i, M, I, D, pr, t_last);
+        dg_t = in_t;
+      }
+      if (part == 0) sum_y = P::sy(P::add(D[R - 1], M[R - 1]));
+    }
+    if (lane != kWarp - 1) return;
+    const S sum_x = P::sx(P::add(D[R - 1], M[R - 1]));
+    // Values needed only now are re-read rather than kept live in registers
+    // through the sweep.
+    load_refs(c, item, refs);
+#pragma unroll
+    for (int q = 0; q < P::kSlots; ++q) {
+      if (refs[q].read == kNoPair) continue;
+      const uint32_t len = b.reads[refs[q].read].len;
+      double amin = (double)kMinAcceptedF;
+      const double res = scaled_result(b, c.gaps, refs[q].read, len, len + 1, S(0),
+                                       q == 0 ? sum_x : sum_y, &amin);
+      finish(b, c, refs[q], res, amin);
+    }
   }
 
   // A chain item: reads x and y against haplotypes hap_start .. +num_haps-1,
@@ -1148,6 +1245,8 @@ __global__ void __launch_bounds__(
     if (item >= n) break;
     if constexpr (F::kChain)
       F::run_chain(b, c, item, n, lane, table);
+    else if constexpr (F::kScaled && !MULTI)
+      F::run_single(b, c, item, lane, table);
     else
       F::run_item(b, c, item, lane, gwarp, table);
   }

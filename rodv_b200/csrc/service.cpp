@@ -122,7 +122,7 @@ uint64_t Service::estimate_bytes(const rodv_batch& b, uint64_t pairs) const {
     bytes += b.hap_lengths[h] + 1;
     max_h = std::max(max_h, b.hap_lengths[h]);
   }
-  bytes += 3 * kHapPad + max_h;
+  bytes += kHapFrontPad + 2 * kHapPad + max_h;
   for (uint32_t r = 0; r < b.num_reads; ++r) {
     bytes += (uint64_t)((b.read_lengths[r] + 3) & ~3u) * 4;
     multi = multi || b.read_lengths[r] + 2 > (uint32_t)kPassRows;  // class_of, either form
