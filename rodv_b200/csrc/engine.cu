@@ -347,7 +347,7 @@ rodv_status Engine::init() {
   // per block opt in to their size.
   cudaError_t ke = cudaSuccess;
   for_each_kernel([&](const KernelInfo& k) {
-    if (ke == cudaSuccess && k.smem_bytes > 48 * 1024)
+    if (ke == cudaSuccess && k.smem_bytes > 47 * 1024)  // + a kernel's static shared memory
       ke = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem_bytes);
   });
   RODV_CUDA(ke);
@@ -1014,18 +1014,45 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   return RODV_OK;
 }
 
-// FP64 launch of class c over its list (rescued pairs, or every pair when
-// FP64 is forced); the list's length is read by the kernel.
+// FP64 launch of every single-pass class of one gap form over their lists
+// (rescued pairs, or every pair when FP64 is forced); the lists' lengths are
+// read by the kernel.
+rodv_status Engine::launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform,
+                                  cudaStream_t stream) {
+  ArenaView a = arena_view(plan, dbase, tab_);
+  RescueLaunch r{};
+  uint64_t pairs = 0;
+  for (int R = 1; R <= kMaxRowsPerLane; ++R) {
+    const int c = single_pass_class(R, uniform);
+    if (!plan.pairs[c]) continue;
+    pairs += plan.pairs[c];
+    r.list[R - 1] = reinterpret_cast<const PairRef*>(dbase + plan.off_lists[c]);
+    r.count[R - 1] = a.counts + kCtrRescue + c;
+  }
+  const int first = single_pass_class(1, uniform);
+  r.c.counter = a.counts + kCtrF64 + first;
+  r.c.error_flags = a.counts + kCtrError;
+  r.c.gaps = plan.gaps;
+  const KernelInfo k = forward_kernel_info(Precision::kF64, kMaxRowsPerLane,
+                                           plan.gap_form(first), false, false, 0);
+  const uint64_t need = (pairs + k.items_per_block - 1) / k.items_per_block;
+  const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(persistent_blocks(k), need));
+  void* args[] = {&a.view, &r};
+  RODV_CUDA(cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream));
+  return RODV_OK;
+}
+
+// FP64 launch of multi-pass class c over its list.
 rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int c,
                                       int variant, cudaStream_t stream) {
   ArenaView a = arena_view(plan, dbase, tab_);
   const KernelInfo k = forward_kernel_info(Precision::kF64, class_rows(c), plan.gap_form(c),
-                                           class_multi(c), false, variant);
+                                           true, false, variant);
   ClassLaunch cl{};
   cl.work = dbase + plan.off_lists[c];
   cl.work_count = a.counts + kCtrRescue + c;
   cl.static_count = 0;
-  if (class_multi(c) && !plan.fp64) {
+  if (!plan.fp64) {
     // rescues sit at their FP32 items' positions (longest items first); the
     // kernel passes over the empty positions
     cl.work_count = nullptr;
@@ -1101,11 +1128,23 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
   }
   if (ev) RODV_CUDA(cudaEventRecord(ev[1], stream));
   if (parts & 2) RODV_CUDA(fork());
-  for (int c = 0; c < kNumClasses && (parts & 2); ++c) {
+  // the multi-pass classes, then the single-pass ones of each gap form (on
+  // the side stream of the form's first class)
+  for (int c = kNumClasses - 1; c >= kSinglePassClasses && (parts & 2); --c) {
     if (!plan.pairs[c]) continue;
     const cudaStream_t ls = lane(c);
     if (!ls) return cuda_fail(cudaErrorUnknown, "class stream fork");
     const rodv_status s = launch_fp64_class(plan, dbase, c, plan.variant64[c], ls);
+    if (s != RODV_OK) return s;
+    ++launches;
+  }
+  for (int u = 1; u >= 0 && (parts & 2); --u) {
+    bool any = false;
+    for (int R = 1; R <= kMaxRowsPerLane; ++R) any = any || plan.pairs[single_pass_class(R, u != 0)];
+    if (!any) continue;
+    const cudaStream_t ls = lane(single_pass_class(1, u != 0));
+    if (!ls) return cuda_fail(cudaErrorUnknown, "class stream fork");
+    const rodv_status s = launch_rescue(plan, dbase, u != 0, ls);
     if (s != RODV_OK) return s;
     ++launches;
   }
@@ -1493,13 +1532,14 @@ rodv_status Engine::plain(rodv_device_batch* db, double* out, rodv_stats* st) {
   // control block: [0,32) ChainItem (one haplotype, one read pair) or
   // SameItem (multi-pass), [32,44) rescue PairRef, words 12..15: fp32
   // counter, fp64 counter, rescue count, error flags, words 16..17: the
-  // chain item's pair (the read, kNoPair)
+  // chain item's pair (the read, kNoPair), word 18: 1, the FP64 list's length
+  constexpr size_t kCtlBytes = 76;
   DeviceMem ctl;
-  RODV_CUDA(ctl.ensure(72));
+  RODV_CUDA(ctl.ensure(kCtlBytes));
   uint8_t* w = static_cast<uint8_t*>(ctl.ptr);
   uint32_t* wc = reinterpret_cast<uint32_t*>(w + 48);
   PinnedMem host;
-  RODV_CUDA(host.ensure(72));
+  RODV_CUDA(host.ensure(kCtlBytes));
   uint8_t* hw = static_cast<uint8_t*>(host.ptr);
   uint32_t* hc = reinterpret_cast<uint32_t*>(hw + 48);
   uint32_t launches = 0;
@@ -1522,10 +1562,10 @@ rodv_status Engine::plain(rodv_device_batch* db, double* out, rodv_stats* st) {
         }
         const PairRef ref{rg.hap_start + h, read, (uint32_t)p};
         std::memcpy(hw + 32, &ref, sizeof(ref));
-        const uint32_t pair[2] = {read, kNoPair};
+        const uint32_t pair[3] = {read, kNoPair, 1};
         std::memcpy(hw + 64, pair, sizeof(pair));
         hc[0] = hc[1] = hc[2] = hc[3] = 0;
-        RODV_CUDA(cudaMemcpyAsync(w, hw, 72, cudaMemcpyHostToDevice, stream_));
+        RODV_CUDA(cudaMemcpyAsync(w, hw, kCtlBytes, cudaMemcpyHostToDevice, stream_));
         for (int pass = 0; pass < 2; ++pass) {
           const bool f64 = pass == 1 || plan.fp64;
           const KernelInfo k =
@@ -1544,7 +1584,12 @@ rodv_status Engine::plain(rodv_device_batch* db, double* out, rodv_stats* st) {
           cl.error_flags = wc + 3;
           cl.stack = reinterpret_cast<const uint32_t*>(w + 64);
           cl.gaps = plan.gaps;
-          void* args[] = {&a.view, &cl};
+          RescueLaunch rl{};
+          rl.c = cl;
+          rl.list[class_rows(c) - 1] = reinterpret_cast<const PairRef*>(w + 32);
+          rl.count[class_rows(c) - 1] = reinterpret_cast<const uint32_t*>(w + 72);
+          const bool rescue = f64 && !class_multi(c);
+          void* args[] = {&a.view, rescue ? (void*)&rl : (void*)&cl};
           RODV_CUDA(
               cudaLaunchKernel(k.fn, dim3(1), dim3(k.threads), args, k.smem_bytes, stream_));
           ++launches;

@@ -193,6 +193,8 @@ class Engine {
                                 int variant, int blocks_cap, cudaStream_t stream);
   rodv_status launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int cls, int variant,
                                 cudaStream_t stream);
+  rodv_status launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform,
+                            cudaStream_t stream);
   rodv_status check_errors(const PackedPlan& plan, uint8_t* dbase);
   rodv_status run_host_single(const rodv_batch& b, double* out, rodv_stats* st, bool fp64,
                               uint8_t* prec);

@@ -52,6 +52,21 @@ KernelInfo make_pipe_info(int variant) {
   return k;
 }
 
+// The FP64 kernel of every single-pass class of one gap form.
+template <int GAPS>
+KernelInfo rescue_info_for() {
+  using F = Forward<F64, kMaxRowsPerLane, GAPS, false, false, 1>;
+  KernelInfo k;
+  k.fn = reinterpret_cast<const void*>(&rescue_kernel<GAPS>);
+  k.threads = F::kWarpsPerBlock * kWarp;
+  k.warps_per_block = F::kWarpsPerBlock;
+  k.smem_bytes = F::kWarpsPerBlock * F::kSmemPerWarp;
+  k.rows_per_lane = kMaxRowsPerLane;
+  k.same_hap = true;
+  k.items_per_block = F::kWarpsPerBlock;
+  return k;
+}
+
 // The multi-pass variants of strip height R (pipe_variant_rows) for one
 // precision, gap form and item kind: W = 2 or 4 warps per item.
 template <int R, int GAPS>
@@ -108,8 +123,7 @@ KernelInfo variant_info(int variant) {
 }
 
 template <int R, bool MU, int GAPS>
-KernelInfo gap_info(Precision prec, bool same, int variant) {
-  if (prec == Precision::kF64) return variant_info<F64, R, GAPS, MU, false>(0);
+KernelInfo gap_info(bool same, int variant) {
   if (same) return variant_info<F32x2, R, GAPS, MU, true>(variant);
   // Two-haplotype items: multi-pass leftovers, and the odd single-pass read
   // of a region against each of its haplotypes.
@@ -117,11 +131,11 @@ KernelInfo gap_info(Precision prec, bool same, int variant) {
 }
 
 template <int R, bool MU>
-KernelInfo info_for(Precision prec, GapForm gaps, bool same, int variant) {
+KernelInfo info_for(GapForm gaps, bool same, int variant) {
   switch (gaps) {
-    case kGapsPerRow: return gap_info<R, MU, kGapsPerRow>(prec, same, variant);
-    case kGapsUniform: return gap_info<R, MU, kGapsUniform>(prec, same, variant);
-    default: return gap_info<R, MU, kGapsConst>(prec, same, variant);
+    case kGapsPerRow: return gap_info<R, MU, kGapsPerRow>(same, variant);
+    case kGapsUniform: return gap_info<R, MU, kGapsUniform>(same, variant);
+    default: return gap_info<R, MU, kGapsConst>(same, variant);
   }
 }
 

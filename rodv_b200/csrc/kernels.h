@@ -9,7 +9,9 @@ namespace rodv {
 enum class Precision { kF32x2 = 0, kF64 = 1 };
 
 struct KernelInfo {
-  const void* fn = nullptr;   // __global__ forward_kernel<...>(BatchView, ClassLaunch)
+  // __global__ forward_kernel<...>(BatchView, ClassLaunch), or for FP64
+  // single-pass classes rescue_kernel<...>(BatchView, RescueLaunch)
+  const void* fn = nullptr;
   int threads = 0;            // threads per block
   int warps_per_block = 0;
   int smem_bytes = 0;         // dynamic shared memory per block
@@ -46,7 +48,8 @@ constexpr int kMaxGroupedRows = 4;  // classes with R <= 4 have the grouped vari
 // same: FP32 items whose reads share the haplotypes -- ChainItem for
 // single-pass classes, SameItem for multi-pass ones; !same: DiffItem
 // (multi-pass leftovers; in a single-pass class, the pairs of each region's
-// odd read).  FP64 kernels take PairRef lists.  variant <
+// odd read).  FP64 kernels take PairRef lists; the single-pass classes of one
+// gap form share one, whatever rows_per_lane.  variant <
 // forward_kernel_variants(...) selects the variant: of same-haplotype FP32
 // single-pass kernels, and of every multi-pass kernel (FP32 same and
 // two-haplotype items share the class's variant, so they agree on the pass

@@ -2,5 +2,5 @@
 #include "kernel_table.cuh"
 
 namespace rodv {
-template KernelInfo info_for<2, false>(Precision, GapForm, bool, int);
+template KernelInfo info_for<2, false>(GapForm, bool, int);
 }  // namespace rodv

@@ -197,6 +197,15 @@ struct ClassLaunch {
   GapConsts gaps;              // kGapsConst kernels
 };
 
+// FP64 launch over the lists of every single-pass class of one gap form:
+// list[R - 1] and count[R - 1] (device; null: none) are those of the class of
+// R rows per lane.
+struct RescueLaunch {
+  ClassLaunch c;               // counter, error_flags, gaps
+  const PairRef* list[kMaxRowsPerLane];
+  const uint32_t* count[kMaxRowsPerLane];
+};
+
 // ClassLaunch::flags.  Testing hook: the producers of a pipelined sweep
 // publish no progress, so every consumer's wait runs out (its expiry path is
 // tested without a fault).

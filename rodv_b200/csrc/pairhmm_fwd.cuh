@@ -564,16 +564,20 @@ struct Forward {
   // the item holds one pair).
   __device__ __forceinline__ static void load_refs(const ClassLaunch& c, uint32_t item,
                                                    PairRef refs[2]) {
+    load_refs(c.work, item, refs);
+  }
+  __device__ __forceinline__ static void load_refs(const void* work, uint32_t item,
+                                                   PairRef refs[2]) {
     if (P::kSlots == 1) {
-      refs[0] = static_cast<const PairRef*>(c.work)[item];
+      refs[0] = static_cast<const PairRef*>(work)[item];
       refs[1] = refs[0];
       refs[1].read = kNoPair;
     } else if (SAME) {
-      const SameItem it = static_cast<const SameItem*>(c.work)[item];
+      const SameItem it = static_cast<const SameItem*>(work)[item];
       refs[0] = PairRef{it.hap, it.read_x, it.out_x};
       refs[1] = PairRef{it.hap, it.read_y, it.out_x + (it.read_y - it.read_x)};
     } else {
-      const DiffItem it = static_cast<const DiffItem*>(c.work)[item];
+      const DiffItem it = static_cast<const DiffItem*>(work)[item];
       refs[0] = it.x;
       refs[1] = it.y;
     }
@@ -680,10 +684,10 @@ struct Forward {
 
   // One pair per slot (SameItem, DiffItem or, for F64, PairRef), swept in one
   // or (MULTI) several passes of 32R rows.
-  __device__ static void run_item(const BatchView& b, const ClassLaunch& c, uint32_t item,
-                                  int lane, int gwarp, uint4* table) {
+  __device__ static void run_item(const BatchView& b, const ClassLaunch& c, const void* work,
+                                  uint32_t item, int lane, int gwarp, uint4* table) {
     PairRef refs[2];
-    load_refs(c, item, refs);
+    load_refs(work, item, refs);
     SlotInfo sl[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
@@ -817,7 +821,7 @@ struct Forward {
     // Values needed only now are re-read rather than kept live in registers
     // through the sweep.
     PairRef fr[2];
-    load_refs(c, item, fr);
+    load_refs(work, item, fr);
     const bool valid_y = P::kSlots == 2 && fr[1].read != kNoPair;
     double res[2] = {0.0, 0.0};
     double amin[2] = {(double)kMinAcceptedF, (double)kMinAcceptedF};
@@ -846,11 +850,11 @@ struct Forward {
   // 40,000 pairs of 250 x 400 bases: FP32 pass 1.11 -> 0.91 ms, FP64 pass 2.00
   // -> 1.72 ms; 124 registers in FP64 where three values and two running sums
   // took 166.
-  __device__ static void run_single(const BatchView& b, const ClassLaunch& c, uint32_t item,
-                                    int lane, uint4* table) {
+  __device__ static void run_single(const BatchView& b, const ClassLaunch& c, const void* work,
+                                    uint32_t item, int lane, uint4* table) {
     constexpr int kLag = P::kSlots == 1 ? 2 : 1;
     PairRef refs[2];
-    load_refs(c, item, refs);
+    load_refs(work, item, refs);
     SlotInfo sl[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
@@ -916,7 +920,7 @@ struct Forward {
     const S sum_x = P::sx(P::add(D[R - 1], M[R - 1]));
     // Values needed only now are re-read rather than kept live in registers
     // through the sweep.
-    load_refs(c, item, refs);
+    load_refs(work, item, refs);
 #pragma unroll
     for (int q = 0; q < P::kSlots; ++q) {
       if (refs[q].read == kNoPair) continue;
@@ -1246,9 +1250,69 @@ __global__ void __launch_bounds__(
     if constexpr (F::kChain)
       F::run_chain(b, c, item, n, lane, table);
     else if constexpr (F::kScaled && !MULTI)
-      F::run_single(b, c, item, lane, table);
+      F::run_single(b, c, c.work, item, lane, table);
     else
-      F::run_item(b, c, item, lane, gwarp, table);
+      F::run_item(b, c, c.work, item, lane, gwarp, table);
+  }
+}
+
+// FP64 pass of every single-pass class of one gap form in one launch: the
+// classes' lists (rescued pairs, or every pair when FP64 is forced) drain in
+// one queue, longest reads first, each pair with the rows per lane of its
+// class.  One launch per class left the GPU with eight mostly empty launches
+// after an FP32 pass that rescues a handful of pairs, and with the classes'
+// tails one after the other when every pair is FP64 (use_double on 50 uneven
+// regions: 1.65 -> 1.44 ms; 16 launches of a 100-region batch become 9).  The
+// rows-per-lane code of all classes shares one register budget: 118 with four
+// blocks per SM; uncapped it takes 166 and three blocks.
+template <int R, int GAPS>
+__device__ __forceinline__ void rescue_one(const BatchView& b, const RescueLaunch& r,
+                                           uint32_t item, int lane, uint4* table) {
+  using F = Forward<F64, R, GAPS, false, false, 1>;
+  if constexpr (F::kScaled)
+    F::run_single(b, r.c, r.list[R - 1], item, lane, table);
+  else
+    F::run_item(b, r.c, r.list[R - 1], item, lane, 0, table);
+}
+
+template <int GAPS>
+__global__ void __launch_bounds__(4 * kWarp, GAPS == kGapsPerRow ? 2 : 4)
+    rescue_kernel(BatchView b, RescueLaunch r) {
+  using F = Forward<F64, kMaxRowsPerLane, GAPS, false, false, 1>;
+  static_assert(F::kWarpsPerBlock == 4, "launch bounds");
+  extern __shared__ uint4 smem[];
+  __shared__ uint32_t ends[kMaxRowsPerLane];  // items of the classes of 8, 7, ... rows per lane
+  const int lane = threadIdx.x & (kWarp - 1);
+  const int warp = threadIdx.x / kWarp;
+  uint4* table = smem + warp * (F::kSmemPerWarp / 16);
+  if (threadIdx.x == 0) {
+    uint32_t n = 0;
+    for (int k = 0; k < kMaxRowsPerLane; ++k) {
+      const uint32_t* count = r.count[kMaxRowsPerLane - 1 - k];
+      if (count) n += *count;
+      ends[k] = n;
+    }
+  }
+  __syncthreads();
+  for (;;) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(r.c.counter, 1u);
+    item = __shfl_sync(kFullMask, item, 0);
+    if (item >= ends[kMaxRowsPerLane - 1]) break;
+    int k = 0;
+    while (item >= ends[k]) ++k;
+    if (k) item -= ends[k - 1];
+    switch (kMaxRowsPerLane - k) {
+      case 8: rescue_one<8, GAPS>(b, r, item, lane, table); break;
+      case 7: rescue_one<7, GAPS>(b, r, item, lane, table); break;
+      case 6: rescue_one<6, GAPS>(b, r, item, lane, table); break;
+      case 5: rescue_one<5, GAPS>(b, r, item, lane, table); break;
+      case 4: rescue_one<4, GAPS>(b, r, item, lane, table); break;
+      case 3: rescue_one<3, GAPS>(b, r, item, lane, table); break;
+      case 2: rescue_one<2, GAPS>(b, r, item, lane, table); break;
+      default: rescue_one<1, GAPS>(b, r, item, lane, table); break;
+    }
+    __syncwarp();
   }
 }
 

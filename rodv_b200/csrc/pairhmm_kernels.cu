@@ -9,7 +9,9 @@
 namespace rodv {
 
 template <int R, bool MU>
-KernelInfo info_for(Precision prec, GapForm gaps, bool same, int variant);
+KernelInfo info_for(GapForm gaps, bool same, int variant);
+template <int GAPS>
+KernelInfo rescue_info_for();
 template <int R>
 KernelInfo pipe_info_for(Precision prec, GapForm gaps, bool same, int variant);
 
@@ -20,15 +22,22 @@ KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, GapForm gaps, 
     return pipe_variant_rows(v) == 4 ? pipe_info_for<4>(prec, gaps, same, v)
                                      : pipe_info_for<8>(prec, gaps, same, v);
   }
+  if (prec == Precision::kF64) {  // one kernel for every single-pass class
+    switch (gaps) {
+      case kGapsPerRow: return rescue_info_for<kGapsPerRow>();
+      case kGapsUniform: return rescue_info_for<kGapsUniform>();
+      default: return rescue_info_for<kGapsConst>();
+    }
+  }
   switch (rows_per_lane) {
-    case 1: return info_for<1, false>(prec, gaps, same, variant);
-    case 2: return info_for<2, false>(prec, gaps, same, variant);
-    case 3: return info_for<3, false>(prec, gaps, same, variant);
-    case 4: return info_for<4, false>(prec, gaps, same, variant);
-    case 5: return info_for<5, false>(prec, gaps, same, variant);
-    case 6: return info_for<6, false>(prec, gaps, same, variant);
-    case 7: return info_for<7, false>(prec, gaps, same, variant);
-    default: return info_for<8, false>(prec, gaps, same, variant);
+    case 1: return info_for<1, false>(gaps, same, variant);
+    case 2: return info_for<2, false>(gaps, same, variant);
+    case 3: return info_for<3, false>(gaps, same, variant);
+    case 4: return info_for<4, false>(gaps, same, variant);
+    case 5: return info_for<5, false>(gaps, same, variant);
+    case 6: return info_for<6, false>(gaps, same, variant);
+    case 7: return info_for<7, false>(gaps, same, variant);
+    default: return info_for<8, false>(gaps, same, variant);
   }
 }
 
