@@ -1699,7 +1699,9 @@ std::string variant_name(int cls, int v, bool fp64) {
   else if (fp64)
     snprintf(buf, sizeof(buf), "one variant");
   else
-    snprintf(buf, sizeof(buf), "%d blocks/SM%s", kVariantMinBlocks[v],
+    snprintf(buf, sizeof(buf), "%d blocks/SM%s",
+             variant_min_blocks(v, class_rows(cls) * (v >= kOccupancyTargets ? 2 : 1),
+                                !class_uniform(cls)),
              v >= kOccupancyTargets ? ", two 16-lane chains per warp" : "");
   return buf;
 }

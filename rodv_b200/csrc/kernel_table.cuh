@@ -91,7 +91,7 @@ KernelInfo pipe_info_for(Precision prec, GapForm gaps, bool same, int variant) {
   }
 }
 
-// Same-haplotype FP32 kernels come in occupancy targets (kVariantMinBlocks);
+// Same-haplotype FP32 kernels come in occupancy targets (variant_min_blocks);
 // the chain kernels of reads up to 128 bases (R <= 4) also in a lane-grouped
 // form: two 16-lane groups per warp, each sweeping its own chain item with
 // 2R rows per lane, so that each lane's per-step overhead (shuffles, code and
@@ -104,20 +104,21 @@ KernelInfo variant_info(int variant) {
     (void)variant;
     return make_info<P, R, GAPS, MU, SAME, 1>(0);
   } else {
+    constexpr bool kRow = GAPS == kGapsPerRow;
     if constexpr (!MU && R <= kMaxGroupedRows) {
       switch (variant) {
-        case 4: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[4], 16>(4);
-        case 5: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[5], 16>(5);
-        case 6: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[6], 16>(6);
-        case 7: return make_info<P, 2 * R, GAPS, MU, SAME, kVariantMinBlocks[7], 16>(7);
+        case 4: return make_info<P, 2 * R, GAPS, MU, SAME, variant_min_blocks(4, 2 * R, kRow), 16>(4);
+        case 5: return make_info<P, 2 * R, GAPS, MU, SAME, variant_min_blocks(5, 2 * R, kRow), 16>(5);
+        case 6: return make_info<P, 2 * R, GAPS, MU, SAME, variant_min_blocks(6, 2 * R, kRow), 16>(6);
+        case 7: return make_info<P, 2 * R, GAPS, MU, SAME, variant_min_blocks(7, 2 * R, kRow), 16>(7);
         default: break;
       }
     }
     switch (variant) {
-      case 0: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[0]>(0);
-      case 1: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[1]>(1);
-      case 2: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[2]>(2);
-      default: return make_info<P, R, GAPS, MU, SAME, kVariantMinBlocks[3]>(3);
+      case 0: return make_info<P, R, GAPS, MU, SAME, variant_min_blocks(0, R, kRow)>(0);
+      case 1: return make_info<P, R, GAPS, MU, SAME, variant_min_blocks(1, R, kRow)>(1);
+      case 2: return make_info<P, R, GAPS, MU, SAME, variant_min_blocks(2, R, kRow)>(2);
+      default: return make_info<P, R, GAPS, MU, SAME, variant_min_blocks(3, R, kRow)>(3);
     }
   }
 }

@@ -41,6 +41,13 @@ inline int pipe_variant_warps(int variant) { return (variant & 1) ? 4 : 2; }
 constexpr int kTuneVariants = 8;
 constexpr int kOccupancyTargets = 4;
 constexpr int kVariantMinBlocks[kTuneVariants] = {4, 5, 6, 8, 4, 5, 6, 8};
+// Per-row kernels of seven and eight rows per lane keep five coefficients a
+// row: at 128 registers (four blocks per SM) R = 7 spills 240 and R = 8 860
+// bytes a thread, so their targets start at three blocks (168 registers).
+constexpr int kPerRowMinBlocks[kTuneVariants] = {3, 4, 5, 6, 3, 4, 5, 6};
+constexpr int variant_min_blocks(int variant, int rows, bool per_row) {
+  return per_row && rows >= 7 ? kPerRowMinBlocks[variant] : kVariantMinBlocks[variant];
+}
 constexpr int kMaxGroupedRows = 4;  // classes with R <= 4 have the grouped variants
 
 // Forward kernel for one work class.  rows_per_lane in 1..8 for single-pass
