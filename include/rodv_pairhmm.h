@@ -379,8 +379,9 @@ void rodv_debug_live_allocations(uint64_t* device, uint64_t* pinned_host);
  * have read_lengths[r] bases and uniform[r] != 0 when their gap priors are
  * uniform (constant ins/del/gcp, ins == del, as the packer decides from the
  * qualities); items_per_warp[R - 1] (R = 1..8) is 1, or 2 for the
- * lane-grouped variant of the uniform class of R rows per lane; stack != 0
- * lets uniform reads stack (every batch call does).  out receives
+ * lane-grouped variant of the classes of R rows per lane; stack == 2 lets
+ * read pairs share an item (as large batches do), any other value but 0
+ * only uniform reads' pairs.  out receives
  * [items, leftover read or 0xFFFFFFFF], then per item [class, pairs, then
  * x read and y read (or 0xFFFFFFFF) of each pair]; *words_written is set
  * even when out_words is too small (RODV_ERR_INVALID_ARG then).  Multi-pass

@@ -248,17 +248,20 @@ rodv_status rodv_debug_chain_plan(const uint32_t* read_lengths, const uint8_t* u
     if (read_lengths[r] == 0 || read_lengths[r] > RODV_MAX_READ_LEN) return RODV_ERR_INVALID_ARG;
     cls[r] = (uint8_t)rodv::class_of(read_lengths[r], uniform[r] != 0);
   }
-  int ipw[rodv::kMaxRowsPerLane + 1] = {};
+  int ipw[2][rodv::kMaxRowsPerLane + 1] = {};
   for (int R = 1; R <= rodv::kMaxRowsPerLane; ++R) {
     if (items_per_warp[R - 1] != 1 && items_per_warp[R - 1] != 2) return RODV_ERR_INVALID_ARG;
-    ipw[R] = items_per_warp[R - 1];
+    ipw[0][R] = ipw[1][R] = items_per_warp[R - 1];
   }
-  rodv::ChainGeom geom[rodv::kMaxRowsPerLane + 1];
-  rodv::chain_geometry(ipw, geom);
+  rodv::ChainGeoms geoms;
+  rodv::chain_geometry(ipw, geoms);
   std::vector<uint32_t> sr;
   rodv::sort_single_pass(read_lengths, cls.data(), 0, num_reads, sr);
   rodv::RegionChains rc;
-  rodv::plan_region_chains(read_lengths, cls.data(), geom, stack != 0, sr, rc);
+  const rodv::ChainStacking stacking = stack == 0   ? rodv::ChainStacking::kNone
+                                       : stack == 2 ? rodv::ChainStacking::kAll
+                                                    : rodv::ChainStacking::kUniform;
+  rodv::plan_region_chains(read_lengths, cls.data(), geoms, stacking, sr, rc);
   std::vector<uint32_t> words{(uint32_t)rc.items.size(), rc.leftover};
   for (const rodv::ChainPairs& it : rc.items) {
     words.push_back((uint32_t)it.cls);

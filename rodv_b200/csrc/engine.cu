@@ -116,9 +116,11 @@ float* class_scratch(const PackedPlan& p, const ArenaView& a, int c) {
 int default_variant(int cls) {
   const int R = class_rows(cls);
   if (class_multi(cls)) return 1;            // strip height 8, 4 warps per item
-  if (R >= 3) return 0;                      // one chain per warp, 4 blocks/SM (128 registers)
-  if (R == 2) return 4;                      // two 16-lane groups, 4 blocks/SM
-  return 6;                                  // two 16-lane groups, 6 blocks/SM (80 registers)
+  // two 16-lane groups, 4 (per-row R = 4: 3) blocks/SM: uniform R = 3 2.61 ms
+  // on its tuning batch against 2.99 with one chain per warp, R = 4 3.44 and
+  // 3.31; per-row R = 4 4.91 and 5.33
+  if (R <= 3 || (R == 4 && !class_uniform(cls))) return 4;
+  return 0;  // one chain per warp, 4 blocks/SM (128 registers; per-row R >= 7: 3)
 }
 // FP64 kernels: multi-pass classes have the pipelined variants, the others one.
 int default_variant64(int cls) { return class_multi(cls) ? 1 : 0; }
@@ -466,7 +468,7 @@ bool low7_all_equal(const uint8_t* p, uint32_t n, uint8_t v) {
 }  // namespace
 
 rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& staging, bool fp64,
-                         bool raw, bool stack_uniform) {
+                         bool raw, bool stack) {
   TraceRange trace("rodv: pack");
   PackTimer timer(opt_.verbose >= 2);
   plan = PackedPlan{};
@@ -557,12 +559,8 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
 
   timer.mark("classes");
   // ---- per region and class: reads, chain items, same items, leftovers ----
-  // Single-pass reads of a region are sorted by (uniform gaps, length).
-  // Reads with per-row gap priors pair neighbour by neighbour, one read per
-  // bin of a chain item, the pair in the class of its longer read (an odd
-  // last one pairs with the shortest uniform read, in a per-row class).
-  // Uniform reads either do the same or, where the cost model below finds it
-  // cheaper, stack into bins of the R = 8 uniform class (stack_uniform).
+  // Single-pass reads of a region are sorted by (uniform gaps, length), pair
+  // up, and the pairs go into chain items (plan_region_chains).
   // Each item takes ceil(haps / chain_haps[class]) chain items.  An odd last
   // read is a leftover: its pairs (one per haplotype) go into two-haplotype
   // items with other regions' leftover pairs of its class, so that both
@@ -577,16 +575,28 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   auto sorted_single = [&](const rodv_region& rg, std::vector<uint32_t>& out_reads) {
     sort_single_pass(b.read_lengths, read_class.data(), rg.read_start, rg.num_reads, out_reads);
   };
-  // the uniform classes' item geometry, from the kernel variants packed for
-  int chain_ipw[kMaxRowsPerLane + 1] = {};
-  for (int R = 1; R <= kMaxRowsPerLane; ++R)
-    chain_ipw[R] = forward_kernel_info(Precision::kF32x2, R, kGapsUniform, false, true,
-                                       variant_[single_pass_class(R, true)])
-                       .items_per_warp;
-  ChainGeom geom[kMaxRowsPerLane + 1];
-  chain_geometry(chain_ipw, geom);
+  // the classes' item geometry, from the kernel variants packed for
+  int chain_ipw[2][kMaxRowsPerLane + 1] = {};
+  for (int u = 0; u < 2; ++u)
+    for (int R = 1; R <= kMaxRowsPerLane; ++R)
+      chain_ipw[u][R] =
+          forward_kernel_info(Precision::kF32x2, R, u ? kGapsUniform : kGapsPerRow, false, true,
+                              variant_[single_pass_class(R, u != 0)])
+              .items_per_warp;
+  ChainGeoms geoms;
+  chain_geometry(chain_ipw, geoms);
+  // Per-row pairs share items only in a batch of eight pairs and more for
+  // every resident warp: below, the one-pair items spread over more warps and
+  // fewer rows per lane (regions of 3-60 reads x 1-9 haplotypes with per-row
+  // gaps: 4,300 pairs 0.16 ms apart, 0.18 sharing; 17,700 pairs 0.36 and 0.37;
+  // 300,000 pairs of longer regions 6.5 and 5.7).  Uniform pairs always may:
+  // they gain from 100 pairs on (19,600 pairs of short reads 0.146 ms apart,
+  // 0.114 sharing).
+  const ChainStacking stacking = !stack ? ChainStacking::kNone
+                                 : pairs >= (uint64_t)num_sms_ * 16 * 8 ? ChainStacking::kAll
+                                                                        : ChainStacking::kUniform;
   auto region_chains = [&](const std::vector<uint32_t>& sr, RegionChains& rc) {
-    plan_region_chains(b.read_lengths, read_class.data(), geom, stack_uniform, sr, rc);
+    plan_region_chains(b.read_lengths, read_class.data(), geoms, stacking, sr, rc);
   };
   std::vector<uint32_t> rc((size_t)G * K, 0);      // reads of class c in region g
   std::vector<uint32_t> rpairs((size_t)G * K, 0);  // bin pairs of chain class c in region g

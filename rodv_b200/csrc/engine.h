@@ -174,11 +174,10 @@ class Engine {
   rodv_status cuda_fail(cudaError_t e, const char* where);
 
  private:
-  // stack_uniform: uniform-gap reads may stack into bins of the R = 8 class
-  // (off: one read per bin, every class keeps its own reads; the autotuner's
-  // per-class batches)
+  // stack: read pairs may share an item's lanes (off: one pair per item,
+  // every class keeps its own reads; the autotuner's per-class batches)
   rodv_status pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& staging, bool fp64,
-                   bool raw = false, bool stack_uniform = true);
+                   bool raw = false, bool stack = true);
   // parts: 1 = counter reset and FP32 launches, 2 = FP64 launches.  ev: null,
   // or three events recorded before the FP32 launches, between the two parts
   // and after the FP64 launches.  fan_out: each class's launches go to its own
