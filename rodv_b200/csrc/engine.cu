@@ -99,7 +99,7 @@ ArenaView arena_view(const PackedPlan& p, uint8_t* base, const PriorTables& tab)
   a.view.raw_prec = p.raw ? base + p.off_prec : nullptr;
   a.view.tab = tab;
   a.counts = reinterpret_cast<uint32_t*>(base + p.off_counts);
-  a.scratch = p.scratch_bytes ? reinterpret_cast<float*>(base + p.off_scratch) : nullptr;
+  a.scratch = p.scratch_cols ? reinterpret_cast<float*>(base + p.off_scratch) : nullptr;
   return a;
 }
 
@@ -108,7 +108,7 @@ ArenaView arena_view(const PackedPlan& p, uint8_t* base, const PriorTables& tab)
 float* class_scratch(const PackedPlan& p, const ArenaView& a, int c) {
   if (!a.scratch || !class_multi(c)) return a.scratch;
   return reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(a.scratch) +
-                                  (size_t)(c - kSinglePassClasses) * p.scratch_bytes);
+                                  (class_uniform(c) ? p.scratch_bytes[0] : 0));
 }
 
 // Occupancy variant used before (or without) tuning: the register budget
@@ -373,15 +373,17 @@ rodv_status Engine::load_kernels() {
   return RODV_OK;
 }
 
-// Boundary rows a multi-pass class's kernels need: per block of the largest
-// grid any multi-pass kernel variant launches (the autotuner runs every
-// variant on its batches).
-size_t Engine::multi_scratch_rows() const {
+// Bytes of boundary rows of `cols` cells that the kernels of a multi-pass class
+// need (cells of 16 bytes in the uniform form, 24 in the per-row one): the
+// rows of the largest grid any of its variants launches (the autotuner runs
+// every variant on its batches).
+size_t Engine::multi_scratch_bytes(bool uniform, size_t cols) const {
   size_t rows = 0;
   for_each_kernel([&](const KernelInfo& k) {
-    if (k.multi) rows = std::max(rows, (size_t)persistent_blocks(k) * k.boundary_rows);
+    if (k.multi && k.uniform == uniform)
+      rows = std::max(rows, (size_t)persistent_blocks(k) * k.boundary_rows);
   });
-  return rows;
+  return align_up(rows * cols * (uniform ? 16 : 24));
 }
 
 // Resident blocks of a kernel on the whole device, queried once per kernel
@@ -779,13 +781,15 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   plan.off_counts = o; o = align_up(o + kCountWords * 4);
   plan.off_prec = o;
   if (raw) o = align_up(o + pairs);
-  plan.scratch_cols = plan.multi_max_hap ? plan.multi_max_hap + 40 : 0;
+  plan.scratch_cols = plan.multi_max_hap ? plan.multi_max_hap + kBoundaryPad : 0;
   plan.off_scratch = o;
   if (plan.scratch_cols) {
     // one region per multi-pass class: the two classes' kernels run as
     // parallel graph branches and must not share boundary rows
-    plan.scratch_bytes = align_up(multi_scratch_rows() * plan.scratch_cols * 24);
-    o = align_up(o + 2 * plan.scratch_bytes);
+    for (int u = 0; u < 2; ++u) {
+      plan.scratch_bytes[u] = multi_scratch_bytes(u != 0, plan.scratch_cols);
+      o = align_up(o + plan.scratch_bytes[u]);
+    }
   }
   plan.total_bytes = o;
 

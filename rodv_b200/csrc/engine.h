@@ -108,7 +108,7 @@ struct PackedPlan {
   size_t off_out = 0, off_counts = 0, off_scratch = 0;
   size_t off_prec = 0;                     // raw mode: precision byte per pair
   size_t total_bytes = 0;
-  size_t scratch_bytes = 0;
+  size_t scratch_bytes[2] = {0, 0};        // of the per-row and the uniform multi-pass class
   uint32_t scratch_cols = 0;
   // host copies kept for the plain per-pair form
   std::vector<rodv_region> regions;
@@ -201,7 +201,7 @@ class Engine {
                                const std::vector<uint32_t>& bounds, uint8_t* prec);
   rodv_status finish_lane(HostLane& lane, double* out, rodv_stats* st, uint8_t* prec);
   int persistent_blocks(const KernelInfo& k) const;
-  size_t multi_scratch_rows() const;
+  size_t multi_scratch_bytes(bool uniform, size_t cols) const;
   std::string device_key() const;
   bool load_tuning(const std::string& path);
   bool save_tuning(const std::string& path) const;

@@ -21,6 +21,7 @@ KernelInfo make_info(int variant) {
   k.warps_per_block = F::kWarpsPerBlock;
   k.smem_bytes = F::kWarpsPerBlock * F::kSmemPerWarp;
   k.rows_per_lane = R;
+  k.uniform = GAPS != kGapsPerRow;
   k.multi = MU;
   k.same_hap = SAME || P::kSlots == 1;
   k.chain = F::kChain;
@@ -34,19 +35,23 @@ KernelInfo make_info(int variant) {
 // Multi-pass kernels: the passes of one item on the W warps of a block.
 template <class P, int R, int GAPS, bool SAME, int W>
 KernelInfo make_pipe_info(int variant) {
-  using F = PipeForward<P, R, GAPS, SAME, 1, W>;
+  // 168 registers (12 warps per SM) in the scaled form; per-row kernels keep
+  // five coefficients a row
+  constexpr int kMinBlocks = GAPS == kGapsPerRow ? 1 : 12 / W;
+  using F = PipeForward<P, R, GAPS, SAME, kMinBlocks, W>;
   KernelInfo k;
-  k.fn = reinterpret_cast<const void*>(&forward_pipe_kernel<P, R, GAPS, SAME, 1, W>);
+  k.fn = reinterpret_cast<const void*>(&forward_pipe_kernel<P, R, GAPS, SAME, kMinBlocks, W>);
   k.threads = W * kWarp;
   k.warps_per_block = W;
   k.smem_bytes = W * F::kSmemPerWarp;
   k.rows_per_lane = R;
+  k.uniform = GAPS != kGapsPerRow;
   k.multi = true;
   k.same_hap = SAME || P::kSlots == 1;
   k.chain = false;
   k.items_per_warp = 1;
   k.items_per_block = 1;
-  k.min_blocks = 1;
+  k.min_blocks = kMinBlocks;
   k.boundary_rows = F::kRows;
   k.variant = variant;
   return k;
@@ -62,6 +67,7 @@ KernelInfo rescue_info_for() {
   k.warps_per_block = F::kWarpsPerBlock;
   k.smem_bytes = F::kWarpsPerBlock * F::kSmemPerWarp;
   k.rows_per_lane = kMaxRowsPerLane;
+  k.uniform = GAPS != kGapsPerRow;
   k.same_hap = true;
   k.items_per_block = F::kWarpsPerBlock;
   return k;

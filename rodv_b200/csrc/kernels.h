@@ -16,6 +16,7 @@ struct KernelInfo {
   int warps_per_block = 0;
   int smem_bytes = 0;         // dynamic shared memory per block
   int rows_per_lane = 0;      // R
+  bool uniform = false;       // of a uniform-gap class
   bool multi = false;         // sweeps reads longer than 32*R rows in passes
   bool same_hap = false;      // both pairs of an item share the haplotype
   bool chain = false;         // takes ChainItem work (single-pass same-haplotype FP32)

@@ -45,6 +45,7 @@ constexpr int kHapPad = 32;          // code bytes after the last haplotype (twi
 // code bytes before the first haplotype: lane 31 of an FP64 sweep starts 62
 // columns behind lane 0
 constexpr int kHapFrontPad = 64;
+constexpr int kBoundaryPad = 72;     // cells of a boundary row beyond its columns
 constexpr int kChainHaps = 32;       // haplotypes per chain item (one per lane)
 constexpr int kMaxRowsPerLane = 8;   // R: read rows held in registers per lane
 constexpr int kPassRows = kWarp * kMaxRowsPerLane;  // rows per multi-pass sweep
@@ -188,7 +189,7 @@ struct ClassLaunch {
   PairRef* rescue_list;        // FP32 only: pairs whose result fell below 1e-28
   uint32_t* rescue_count;
   float* scratch;              // MULTI: per resident warp boundary-row buffer
-  uint32_t scratch_cols;       // columns per warp buffer (max hap len + 40)
+  uint32_t scratch_cols;       // cells per boundary row (max hap len + kBoundaryPad)
   uint32_t* error_flags;       // bit set by a kernel that hit a bad descriptor
   uint32_t flags;              // kLaunch* bits
   uint32_t wait_polls;         // pipelined sweeps: polls before a wait gives up (0: default)

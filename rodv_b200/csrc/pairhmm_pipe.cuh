@@ -87,6 +87,37 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gmem) : "memory");
 }
 
+// Stores of boundary cells where `on` is set, as predicated instructions: a
+// branch in every step would split the unrolled steps (as the separator test
+// does in the chain sweeps).  No "memory" clobber: the loads of the following
+// steps (codes, emissions, the ring) never read what they write and may move
+// ahead of them.  The release that publishes the cells (st_release_cta) is a
+// volatile asm too and stays behind them.
+__device__ __forceinline__ void st_cell(bool on, void* p, float2 a, float2 b) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+      "@q st.global.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"l"(p),
+      "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "r"((uint32_t)on));
+}
+__device__ __forceinline__ void st_cell(bool on, void* p, double a, double b) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t"
+      "@q st.global.v2.f64 [%0], {%1, %2};\n\t}" ::"l"(p),
+      "d"(a), "d"(b), "r"((uint32_t)on));
+}
+__device__ __forceinline__ void st_cell(bool on, void* p, float2 a) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t"
+      "@q st.global.v2.f32 [%0], {%1, %2};\n\t}" ::"l"(p),
+      "f"(a.x), "f"(a.y), "r"((uint32_t)on));
+}
+__device__ __forceinline__ void st_cell(bool on, void* p, double a) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+      "@q st.global.f64 [%0], %1;\n\t}" ::"l"(p),
+      "d"(a), "r"((uint32_t)on));
+}
+
 template <class P, int R, int GAPS, bool SAME, int MINB, int W>
 struct PipeForward {
   using F = Forward<P, R, GAPS, true, SAME, MINB>;
@@ -99,13 +130,16 @@ struct PipeForward {
   using Cell = typename std::conditional<kTwo, HandCell, typename F::BoundaryCell>::type;
   static_assert(sizeof(Cell) <= 24, "the engine sizes boundary rows at 24 bytes a cell");
   static constexpr int kRows = W + 1;                   // boundary rows per block
-  static constexpr int kPad = kWarp;                    // cells before column 0 of a row
-  // Steps per loop iteration, measured on the 2,000 long pairs above.  FP32:
-  // four (FP32 pass 2.78 ms, 3.09 at two).  FP64: two, 166 registers at R = 8,
-  // so three warps a sub-partition (FP64 pass 7.19 ms; 7.33 at four, 173
-  // registers and two warps; 8.25 at one; 9.76 at one capped to 128
-  // registers and four warps).
-  static constexpr int kUnroll = P::kSlots == 1 ? 2 : 4;
+  // Columns a lane runs behind its left neighbour.  FP64 (two-value form): two,
+  // so a value shuffled in one step is used in the next (Forward::run_single).
+  static constexpr int kLag = kTwo && P::kSlots == 1 ? 2 : 1;
+  static constexpr int kPad = kLag * kWarp;             // cells before column 0 of a row
+  static_assert(kPad + 8 <= kBoundaryPad, "the engine sizes boundary rows");
+  // Steps per loop iteration of a whole chunk: eight at 168 registers (12 warps
+  // per SM).  2,000-pair batches of 1,500 x 3,500 bases: FP32 2.46 ms, FP64
+  // 4.77 (four steps 2.46 and 4.90); at 128 registers and 16 warps both spill
+  // (2.77 and 4.47 at eight steps, 3.4 and 5.0 at four).
+  static constexpr int kUnroll = 8;
   static constexpr int kSmemPerWarp = F::kSmemPerWarp;  // emission table + cell ring
   // polls of a progress word (about 100 ns each) before a wait gives up
   static constexpr uint32_t kWaitPolls = 1u << 24;
@@ -221,7 +255,7 @@ struct PipeForward {
     const uint32_t Lmax = sl[0].L > sl[1].L ? sl[0].L : sl[1].L;
     if (sl[0].H == 0 || sl[1].H == 0 || sl[0].L == 0 || sl[1].L == 0 ||
         (F::kSameHap && sl[0].hap != sl[1].hap) || sl[1].H > sl[0].H ||
-        (uint64_t)sl[0].H + 40 > c.scratch_cols) {
+        (uint64_t)sl[0].H + kPad + 8 > c.scratch_cols) {
       if (warp == 0 && lane == 0) atomicOr(c.error_flags, kErrBadLength);
       return out;
     }
@@ -229,8 +263,9 @@ struct PipeForward {
     const uint32_t passes = pipe_passes(Lmax, R);
     out.passes = passes;
     const uint32_t H = sl[0].H;
-    const int nsteps = (int)H + kWarp - 1;         // slot x has the longer haplotype
-    const int nfreeze = (int)sl[1].H + kWarp - 1;  // slot y's last accumulated step + 1
+    const int nsteps = (int)H + kLag * (kWarp - 1);  // slot x has the longer haplotype
+    // slot y's last accumulated step + 1
+    const int nfreeze = (int)sl[1].H + kLag * (kWarp - 1);
     const V init = P::make(P::init_const() / (S)sl[0].H, P::init_const() / (S)sl[1].H);
     const uint32_t L[2] = {sl[0].L, sl[1].L};
     const uint64_t row_off[2] = {sl[0].row_off, sl[1].row_off};
@@ -245,8 +280,9 @@ struct PipeForward {
       const int out_row = (int)(p % kRows);
       const int in_row = (int)((p + kRows - 1) % kRows);
       Cell* const out_cells = rows + (size_t)out_row * c.scratch_cols + kPad;  // column 0
-      // lane 31's step s holds column s - 30 after the step
-      Cell* const dst = out_cells - (kWarp - 2);
+      // lane 31's step s holds column s - 31 kLag + 1 after the step
+      constexpr int kLastCol = kLag * (kWarp - 1) - 1;
+      Cell* const dst = out_cells - kLastCol;
       const Cell* const src = rows + (size_t)in_row * c.scratch_cols + kPad;
       // cells of steps [32 k, 32 k + 32) from the previous pass's row
       // (columns 32 k + 1 .. 32 k + 32), copied once they are published
@@ -295,18 +331,63 @@ struct PipeForward {
         ring[kWarp + lane] = top;
       }
       __syncwarp();
-      uint32_t cx_next = sl[0].hap[-lane];
-      uint32_t cy_next = F::kSameHap ? 0u : (uint32_t)sl[1].hap[-lane];
-      const uint8_t* hx = sl[0].hap - lane + 1;  // code of the step after s: hx[s]
-      const uint8_t* hy = sl[1].hap - lane + 1;
+      uint32_t cx_next = sl[0].hap[-kLag * lane];
+      uint32_t cy_next = F::kSameHap ? 0u : (uint32_t)sl[1].hap[-kLag * lane];
+      const uint8_t* hx = sl[0].hap - kLag * lane + 1;  // code of the step after s: hx[s]
+      const uint8_t* hy = sl[1].hap - kLag * lane + 1;
       V acc = P::zero();
       S frozen = 0;
       // two-value form: this lane's hand-over for the lane below, and the M
       // term of its first row carried to the next column
       V h_t = P::zero(), h_i = P::zero();
+      V next_t = P::zero(), next_i = P::zero();  // kLag 2: shuffled in the previous step
       V dg_t = (lane == 0 && p == 0) ? init : P::zero();
       // three-value form: the row above at the previous column
       V dg_m = P::zero(), dg_i = P::zero(), dg_d = (lane == 0 && p == 0) ? init : P::zero();
+
+      // One step; i: the step of its chunk.  The sum of the last row is kept
+      // in every pass (only the last pass's is used): a test in each step
+      // cost more than the add.
+      Cell cell_next;  // lane 0's row above in the next step, loaded a step ahead
+      auto step = [&](int s, const Cell* next) {
+        const uint32_t cx = cx_next, cy = cy_next;
+        cx_next = hx[s];
+        if (!F::kSameHap) cy_next = hy[s];
+        V e[R], t_last;
+        const Cell cl = cell_next;
+        cell_next = *next;
+        if constexpr (kTwo) {
+          V in_t = P::shfl_up(h_t), in_i = P::shfl_up(h_i);
+          if (kLag == 2) {
+            const V t = in_t, i = in_i;
+            in_t = next_t; in_i = next_i;
+            next_t = t; next_i = i;
+          }
+          if (lane == 0) {
+            in_t = cl.t; in_i = cl.i;
+          }
+          F::load_emission(table, lane, cx, cy, e);
+          F::cells_scaled(e, dg_t, in_i, M, I, D, pr, t_last);
+          dg_t = in_t;
+          h_t = P::fma(pr.mmU, M[R - 1], P::add(I[R - 1], D[R - 1]));
+          h_i = P::fma(pr.iiN, I[R - 1], M[R - 1]);
+          st_cell(store, dst + s, h_t, h_i);
+        } else {
+          V up_m = P::shfl_up(M[R - 1]);
+          V up_i = P::shfl_up(I[R - 1]);
+          V up_d = P::shfl_up(D[R - 1]);
+          if (lane == 0) {
+            up_m = cl.m; up_i = cl.i; up_d = cl.d;
+          }
+          F::load_emission(table, lane, cx, cy, e);
+          F::cells(e, up_m, up_i, up_d, dg_m, dg_i, dg_d, M, I, D, pr, t_last);
+          st_cell(store, &dst[s].m, M[R - 1]);
+          st_cell(store, &dst[s].i, I[R - 1]);
+          st_cell(store, &dst[s].d, D[R - 1]);
+        }
+        (void)t_last;
+        acc = P::add(acc, I[R - 1]);
+      };
 
       const int nchunks = (nsteps + kWarp - 1) / kWarp;
       for (int k = 0; k < nchunks; ++k) {
@@ -322,52 +403,26 @@ struct PipeForward {
           break;
         }
         const Cell* rc = ring + (k & 1) * kWarp;
+        cell_next = rc[0];
         const int s0 = k * kWarp;
         const int cnt = nsteps - s0 < kWarp ? nsteps - s0 : kWarp;
-#pragma unroll kUnroll
-        for (int i = 0; i < cnt; ++i) {
-          const int s = s0 + i;
-          const uint32_t cx = cx_next, cy = cy_next;
-          cx_next = hx[s];
-          if (!F::kSameHap) cy_next = hy[s];
-          V e[R], t_last;
-          if constexpr (kTwo) {
-            V in_t = P::shfl_up(h_t), in_i = P::shfl_up(h_i);
-            if (lane == 0) {
-              const Cell cl = rc[i];
-              in_t = cl.t; in_i = cl.i;
-            }
-            F::load_emission(table, lane, cx, cy, e);
-            F::cells_scaled(e, dg_t, in_i, M, I, D, pr, t_last);
-            dg_t = in_t;
-            h_t = P::fma(pr.mmU, M[R - 1], P::add(I[R - 1], D[R - 1]));
-            h_i = P::fma(pr.iiN, I[R - 1], M[R - 1]);
-            if (store) dst[s] = Cell{h_t, h_i};
-          } else {
-            V up_m = P::shfl_up(M[R - 1]);
-            V up_i = P::shfl_up(I[R - 1]);
-            V up_d = P::shfl_up(D[R - 1]);
-            if (lane == 0) {
-              const Cell cl = rc[i];
-              up_m = cl.m; up_i = cl.i; up_d = cl.d;
-            }
-            F::load_emission(table, lane, cx, cy, e);
-            F::cells(e, up_m, up_i, up_d, dg_m, dg_i, dg_d, M, I, D, pr, t_last);
-            if (store) {
-              Cell cl;
-              cl.m = M[R - 1]; cl.i = I[R - 1]; cl.d = D[R - 1];
-              dst[s] = cl;
-            }
+        // slot y of a two-haplotype item ends within this chunk
+        const bool freeze = P::kSlots == 2 && !F::kSameHap && nfreeze > s0 && nfreeze <= s0 + cnt;
+        if (cnt == kWarp && !freeze) {
+#pragma unroll 1
+          for (int i = 0; i < kWarp; i += kUnroll) {
+#pragma unroll
+            for (int u = 0; u < kUnroll; ++u) step(s0 + i + u, rc + ((i + u + 1) & (kWarp - 1)));
           }
-          (void)t_last;
-          if (last) {
-            acc = P::add(acc, I[R - 1]);
-            if (P::kSlots == 2 && !F::kSameHap && s == nfreeze - 1) frozen = P::sy(acc);
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < cnt; ++i) {
+            step(s0 + i, rc + ((i + 1) & (kWarp - 1)));
+            if (freeze && s0 + i == nfreeze - 1) frozen = P::sy(acc);
           }
         }
         if (store && publish) {
-          // columns up to (the chunk's last step) - 30 are stored
-          const int col = s0 + cnt - 1 - (kWarp - 2);
+          const int col = s0 + cnt - 1 - kLastCol;  // the last column stored
           if (col >= 1) {
             __threadfence_block();
             st_release_cta(&ctl.prog[out_row], enc(p, (uint32_t)col));

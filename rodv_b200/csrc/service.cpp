@@ -129,9 +129,10 @@ uint64_t Service::estimate_bytes(const rodv_batch& b, uint64_t pairs) const {
   }
   bytes += (uint64_t)(b.num_haps + b.num_reads) * 16;
   bytes += pairs * (16 + 12 + 8);
-  // boundary scratch: 24 bytes per column per boundary row of the multi-pass
-  // kernels, one region per multi-pass class
-  if (multi) bytes += 2 * (uint64_t)engine_.multi_scratch_rows() * (max_h + 40) * 24 + 512;
+  // boundary rows of the multi-pass kernels, one region per multi-pass class
+  if (multi)
+    for (int u = 0; u < 2; ++u)
+      bytes += engine_.multi_scratch_bytes(u != 0, max_h + kBoundaryPad) + 256;
   return bytes;
 }
 
