@@ -37,6 +37,7 @@
 
 #include "engine.h"
 #include "chain_plan.h"
+#include "pack_rows.h"
 #include "tables.h"
 #include "trace.h"
 #include "worker_pool.h"
@@ -48,16 +49,6 @@ namespace {
 constexpr size_t kAlign = 256;
 inline size_t align_up(size_t v, size_t a = kAlign) { return (v + a - 1) / a * a; }
 
-// A0 C1 G2 T3 N4; 0xff marks a base outside the engine's domain.
-struct CodeTable {
-  uint8_t v[256];
-  CodeTable() {
-    std::memset(v, 0xff, sizeof(v));
-    v['A'] = kA; v['C'] = kC; v['G'] = kG; v['T'] = kT; v['N'] = kN;
-  }
-};
-const CodeTable kCodes;
-
 // Section timer of the packer, printed at verbose level 2.
 struct PackTimer {
   bool on;
@@ -68,7 +59,7 @@ struct PackTimer {
     if (!on) return;
     const auto now = std::chrono::steady_clock::now();
     char buf[64];
-    snprintf(buf, sizeof(buf), " %s %.2f", what,
+    snprintf(buf, sizeof(buf), " %s %.3f", what,
              std::chrono::duration<double, std::milli>(now - t).count());
     line += buf;
     t = now;
@@ -432,19 +423,15 @@ rodv_status validate_batch(const rodv_batch& b, bool check_bases, uint64_t* num_
     const uint32_t len = b.hap_lengths[h];
     if (len == 0) return bad(RODV_ERR_INVALID_ARG, "haplotype " + std::to_string(h) + " is empty");
     if (len > RODV_MAX_HAP_LEN) return bad(RODV_ERR_TOO_LONG, "haplotype longer than limit");
-    if (check_bases)
-      for (uint32_t k = 0; k < len; ++k)
-        if (kCodes.v[b.hap_bases[b.hap_offsets[h] + k]] == 0xff)
-          return bad(RODV_ERR_INVALID_BASE, "haplotype base is not one of A, C, G, T, N");
+    if (check_bases && !bases_valid(b.hap_bases + b.hap_offsets[h], len))
+      return bad(RODV_ERR_INVALID_BASE, "haplotype base is not one of A, C, G, T, N");
   }
   for (uint32_t r = 0; r < b.num_reads; ++r) {
     const uint32_t len = b.read_lengths[r];
     if (len == 0) return bad(RODV_ERR_INVALID_ARG, "read " + std::to_string(r) + " is empty");
     if (len > RODV_MAX_READ_LEN) return bad(RODV_ERR_TOO_LONG, "read longer than limit");
-    if (check_bases)
-      for (uint32_t k = 0; k < len; ++k)
-        if (kCodes.v[b.read_bases[b.read_offsets[r] + k]] == 0xff)
-          return bad(RODV_ERR_INVALID_BASE, "read base is not one of A, C, G, T, N");
+    if (check_bases && !bases_valid(b.read_bases + b.read_offsets[r], len))
+      return bad(RODV_ERR_INVALID_BASE, "read base is not one of A, C, G, T, N");
   }
   if (num_pairs) *num_pairs = pairs;
   return RODV_OK;
@@ -465,6 +452,41 @@ bool low7_all_equal(const uint8_t* p, uint32_t n, uint8_t v) {
   for (; k < n; ++k)
     if ((p[k] & 127) != v) return false;
   return true;
+}
+
+}  // namespace
+
+namespace {
+
+// The indices of v in decreasing order of value, equal ones in increasing order
+// of index: a radix sort of 11 bits a pass where a comparison sort of 40,000
+// regions took 2 ms.
+void decreasing_order(const std::vector<uint64_t>& v, std::vector<uint32_t>& order) {
+  const size_t n = v.size();
+  order.resize(n);
+  uint64_t top = 0;
+  bool sorted = true;
+  for (size_t k = 0; k < n; ++k) {
+    order[k] = (uint32_t)k;
+    top = std::max(top, v[k]);
+    sorted = sorted && (k == 0 || v[k - 1] >= v[k]);
+  }
+  if (sorted) return;
+  if (n < 512) {
+    std::stable_sort(order.begin(), order.end(),
+                     [&](uint32_t x, uint32_t y) { return v[x] > v[y]; });
+    return;
+  }
+  constexpr int kBits = 11;
+  std::vector<uint32_t> next(n);
+  for (int shift = 0; shift < 64 && (top >> shift) != 0; shift += kBits) {
+    uint32_t start[(1 << kBits) + 1] = {};
+    auto digit = [&](uint32_t k) { return (uint32_t)((top - v[k]) >> shift) & ((1u << kBits) - 1); };
+    for (uint32_t k : order) ++start[digit(k) + 1];
+    for (int d = 0; d < (1 << kBits); ++d) start[d + 1] += start[d];
+    for (uint32_t k : order) next[start[digit(k)]++] = k;
+    order.swap(next);
+  }
 }
 
 }  // namespace
@@ -573,10 +595,6 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   // the rest of the batch.
   // Multi-pass reads keep their own class: same-haplotype items per
   // haplotype, leftovers in two-haplotype items.
-  const uint32_t K = kNumClasses;
-  auto sorted_single = [&](const rodv_region& rg, std::vector<uint32_t>& out_reads) {
-    sort_single_pass(b.read_lengths, read_class.data(), rg.read_start, rg.num_reads, out_reads);
-  };
   // the classes' item geometry, from the kernel variants packed for
   int chain_ipw[2][kMaxRowsPerLane + 1] = {};
   for (int u = 0; u < 2; ++u)
@@ -600,151 +618,197 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   auto region_chains = [&](const std::vector<uint32_t>& sr, RegionChains& rc) {
     plan_region_chains(b.read_lengths, read_class.data(), geoms, stacking, sr, rc);
   };
-  std::vector<uint32_t> rc((size_t)G * K, 0);      // reads of class c in region g
-  std::vector<uint32_t> rpairs((size_t)G * K, 0);  // bin pairs of chain class c in region g
-  std::vector<uint32_t> chains((size_t)G * K, 0);  // chain items of class c in region g
-  std::vector<uint64_t> cpairs((size_t)G * K, 0);  // pairs those chains compute
-  std::vector<uint32_t> nstack((size_t)G * K, 0);  // reads in those bins (stack list entries)
-  std::vector<uint64_t> hsum(G, 0);
-  std::vector<uint32_t> hmax(G, 0);
-  // multi-pass leftovers: the last read of each multi-pass class in the region
-  std::vector<uint32_t> left_read((size_t)G * 2, kNoPair);
-  // single-pass leftover: the odd last read of the region's sorted single-pass reads
-  std::vector<uint32_t> single_read(G, kNoPair);
-  std::atomic<bool> chain_class_bad{false};  // a chain item outside the single-pass classes
-  parallel_for(G, 16, [&](size_t lo, size_t hi) {
-    std::vector<uint32_t> sr;
-    RegionChains chs;
-    for (size_t g = lo; g < hi; ++g) {
-      const rodv_region& rg = b.regions[g];
-      for (uint32_t r = 0; r < rg.num_reads; ++r) {
-        const uint32_t read = rg.read_start + r;
-        const int c = read_class[read];
-        rc[g * K + c]++;
-        if (class_multi(c)) left_read[g * 2 + (c - kSinglePassClasses)] = read;
-      }
-      for (int u = 0; u < 2; ++u)
-        if (!(rc[g * K + kSinglePassClasses + u] & 1)) left_read[g * 2 + u] = kNoPair;
-      for (uint32_t h = 0; h < rg.num_haps; ++h) {
-        hsum[g] += b.hap_lengths[rg.hap_start + h];
-        hmax[g] = std::max(hmax[g], b.hap_lengths[rg.hap_start + h]);
-      }
-      if (fp64) continue;
-      sorted_single(rg, sr);
-      region_chains(sr, chs);
-      for (const ChainPairs& ci : chs.items) {
-        if (ci.cls < 0 || ci.cls >= kSinglePassClasses) {
-          chain_class_bad.store(true);
-          break;
-        }
-        rpairs[g * K + ci.cls] += 1;
-        nstack[g * K + ci.cls] += 2 * ci.pairs;
-        cpairs[g * K + ci.cls] += (uint64_t)rg.num_haps * 2 * ci.pairs;
-      }
-      if (chs.leftover != kNoPair) {
-        single_read[g] = chs.leftover;
-        cpairs[g * K + read_class[chs.leftover]] += rg.num_haps;
-      }
-    }
-  });
-  if (chain_class_bad.load())
-    return fail(RODV_ERR_INTERNAL, "packer placed a chain item outside the single-pass classes");
-  // Haplotypes per chain item, per class: the longest chains (up to
-  // kChainHaps) that still leave every resident warp of the class's launch
-  // (16 per SM at most) two items; a small batch gets short chains (down to
-  // one haplotype).
   for (int c = 0; c < kNumClasses; ++c) {
     plan.variant[c] = variant_[c];
     plan.variant64[c] = variant64_[c];
   }
+  auto passes_of = [&](uint32_t read) -> uint32_t {
+    const int c = read_class[read];
+    if (!class_multi(c)) return 1u;  // single-pass leftovers: one group
+    return pipe_passes(b.read_lengths[read], pipe_variant_rows(plan.variant[c]));
+  };
+  // Items are laid out region by region in decreasing order of the region's
+  // haplotype-length sum (a chain's cost), so the persistent kernels take the
+  // longest chains first.
+  std::vector<uint64_t> hsum(G), region_out(G);
+  std::vector<uint32_t> hmax(G);
+  parallel_for(G, 1024, [&](size_t lo, size_t hi) {
+    for (size_t g = lo; g < hi; ++g) {
+      const rodv_region& rg = b.regions[g];
+      uint64_t sum = 0;
+      uint32_t mx = 0;
+      for (uint32_t h = 0; h < rg.num_haps; ++h) {
+        const uint32_t len = b.hap_lengths[rg.hap_start + h];
+        sum += len;
+        mx = std::max(mx, len);
+      }
+      hsum[g] = sum;
+      hmax[g] = mx;
+    }
+  });
+  for (uint32_t g = 0, acc = 0; g < G; ++g) {
+    region_out[g] = acc;
+    acc += b.regions[g].num_haps * b.regions[g].num_reads;
+  }
+  std::vector<uint32_t> order;
+  decreasing_order(hsum, order);
+  // Blocks of regions (in that order) are planned and counted in parallel; a
+  // scan over the blocks' totals then gives each block's first position in
+  // every class's lists, and the blocks write their items in parallel.  (A
+  // table of positions per region and class took 17-30 ms of a 40,000-region
+  // batch, most of it page faults; the blocks take 1.)  Up to 16 regions are
+  // one block: waking a pool thread costs more than planning them.
+  const uint32_t kBlockRegions = G <= 16 ? 16 : std::min(32u, std::max(8u, G / 64));
+  constexpr int kCaps = 6;  // haplotypes per chain item: 32, 16, ..., 1
+  struct RegionPlan {
+    uint32_t first_item, end_item;  // of the block's items
+    uint32_t first_read;            // of the block's reads
+    uint32_t single;                // the odd single-pass read, or kNoPair
+    uint32_t left[2];               // the odd last read of each multi-pass class, or kNoPair
+  };
+  struct Counts {
+    uint64_t same[kNumClasses], left[kNumClasses], list[kNumClasses], cap[kNumClasses],
+        stack[kNumClasses];
+  };
+  struct Block {
+    std::vector<ChainPairs> items;
+    std::vector<uint32_t> reads;
+    std::vector<RegionPlan> regions;
+    Counts n = {};                               // same: of multi-pass classes only
+    uint64_t chains[kSinglePassClasses][kCaps] = {};  // chain items by cap
+    uint64_t cells = 0;
+    uint32_t multi_hap = 0;
+    bool bad_class = false;
+  };
+  const uint32_t nblocks = (G + kBlockRegions - 1) / kBlockRegions;
+  std::vector<Block> blocks(nblocks);
+  parallel_for(nblocks, 1, [&](size_t lo, size_t hi) {
+    std::vector<uint32_t> sr;
+    RegionChains chs;
+    for (size_t k = lo; k < hi; ++k) {
+      Block& bl = blocks[k];
+      const uint32_t i1 = std::min<uint32_t>(G, (uint32_t)(k + 1) * kBlockRegions);
+      bl.regions.reserve(i1 - k * kBlockRegions);
+      for (uint32_t i = (uint32_t)k * kBlockRegions; i < i1; ++i) {
+        const uint32_t g = order[i];
+        const rodv_region& rg = b.regions[g];
+        const uint64_t H = rg.num_haps;
+        RegionPlan rp{(uint32_t)bl.items.size(), 0, (uint32_t)bl.reads.size(), kNoPair,
+                      {kNoPair, kNoPair}};
+        uint32_t n[kNumClasses] = {};
+        uint64_t rs = 0;
+        for (uint32_t r = rg.read_start; r < rg.read_start + rg.num_reads; ++r) {
+          const int c = read_class[r];
+          ++n[c];
+          rs += b.read_lengths[r];
+          if (class_multi(c)) rp.left[c - kSinglePassClasses] = r;
+        }
+        bl.cells += hsum[g] * rs;
+        for (int c = 0; c < kNumClasses; ++c) {
+          if (!n[c]) continue;
+          bl.n.list[c] += H * n[c];
+          if (!class_multi(c)) continue;
+          bl.multi_hap = std::max(bl.multi_hap, hmax[g]);
+          bl.n.same[c] += H * (n[c] / 2);
+          bl.n.left[c] += H * (n[c] & 1);
+          bl.n.cap[c] += H * n[c];
+        }
+        for (int u = 0; u < 2; ++u)
+          if (!(n[kSinglePassClasses + u] & 1)) rp.left[u] = kNoPair;
+        if (!fp64) {
+          sort_single_pass(b.read_lengths, read_class.data(), rg.read_start, rg.num_reads, sr);
+          plan_region_chains(b.read_lengths, read_class.data(), geoms, stacking, sr, chs);
+          for (ChainPairs it : chs.items) {
+            if (it.cls < 0 || it.cls >= kSinglePassClasses) {
+              bl.bad_class = true;
+              break;
+            }
+            for (int q = 0; q < kCaps; ++q) {
+              const uint32_t cap = (uint32_t)kChainHaps >> q;
+              bl.chains[it.cls][q] += (H + cap - 1) / cap;
+            }
+            bl.n.stack[it.cls] += 2 * it.pairs;
+            bl.n.cap[it.cls] += H * 2 * it.pairs;
+            bl.items.push_back(it);
+          }
+          bl.reads.insert(bl.reads.end(), chs.reads.begin(), chs.reads.end());
+          rp.single = chs.leftover;
+          if (rp.single != kNoPair) {
+            const int c = read_class[rp.single];
+            bl.n.cap[c] += H;
+            bl.n.left[c] += H;
+          }
+        }
+        rp.end_item = (uint32_t)bl.items.size();
+        bl.regions.push_back(rp);
+      }
+    }
+  });
+  for (const Block& bl : blocks) {
+    if (bl.bad_class)
+      return fail(RODV_ERR_INTERNAL,
+                  "packer placed a chain item outside the single-pass classes");
+    plan.cells += bl.cells;
+    plan.multi_max_hap = std::max(plan.multi_max_hap, bl.multi_hap);
+  }
+  // Haplotypes per chain item, per class: the longest chains (up to
+  // kChainHaps) that still leave every resident warp of the class's launch
+  // (16 per SM at most) two items; a small batch gets short chains (down to
+  // one haplotype).
+  int cap_index[kSinglePassClasses];
   for (int c = 0; c < kSinglePassClasses; ++c) {
     // chain items a warp of this class's kernel sweeps at once
     const int ipw = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c),
                                         false, true, plan.variant[c]).items_per_warp;
     const uint64_t target_items = (uint64_t)num_sms_ * 16 * 2 * ipw;
-    plan.chain_haps[c] = 1;
-    for (uint32_t cap = kChainHaps / ipw; cap >= 1; cap /= 2) {
+    for (int q = ipw == 2 ? 1 : 0; q < kCaps; ++q) {
       uint64_t items = 0;
-      for (uint32_t g = 0; g < G; ++g)
-        items += (uint64_t)rpairs[(size_t)g * K + c] * ((b.regions[g].num_haps + cap - 1) / cap);
-      if (items >= target_items || cap == 1) {
-        plan.chain_haps[c] = cap;
-        break;
-      }
+      for (const Block& bl : blocks) items += bl.chains[c][q];
+      cap_index[c] = q;
+      plan.chain_haps[c] = (uint32_t)kChainHaps >> q;
+      if (items >= target_items) break;
     }
   }
-  for (uint32_t g = 0; g < G; ++g)
-    for (int c = 0; c < kSinglePassClasses; ++c)
-      chains[(size_t)g * K + c] = rpairs[(size_t)g * K + c] *
-          ((b.regions[g].num_haps + plan.chain_haps[c] - 1) / plan.chain_haps[c]);
-  // Chain items are laid out region by region in decreasing order of the
-  // region's haplotype-length sum (a chain's cost), so the persistent
-  // kernels take the longest chains first.
-  std::vector<uint32_t> order(G);
-  for (uint32_t g = 0; g < G; ++g) order[g] = g;
-  std::stable_sort(order.begin(), order.end(),
-                   [&](uint32_t x, uint32_t y) { return hsum[x] > hsum[y]; });
-  // prefix offsets (within each class) of same/chain items, leftovers, FP64 list entries
-  std::vector<uint64_t> same_off((size_t)G * K), left_off((size_t)G * K), list_off((size_t)G * K),
-      stack_off((size_t)G * K);
-  uint64_t same_tot[kNumClasses] = {}, left_tot[kNumClasses] = {}, list_tot[kNumClasses] = {},
-           cap_tot[kNumClasses] = {}, stack_tot[kNumClasses] = {};
-  for (uint32_t i = 0; i < G; ++i) {
-    const uint32_t g = order[i];
-    const uint64_t H = b.regions[g].num_haps;
+  // each block's first positions (within each class) of same/chain items,
+  // leftovers, FP64 list entries and stack list entries, and the totals
+  std::vector<Counts> at(nblocks);
+  Counts tot = {};
+  for (uint32_t k = 0; k < nblocks; ++k) {
+    const Block& bl = blocks[k];
+    at[k] = tot;
     for (int c = 0; c < kNumClasses; ++c) {
-      const uint64_t n = rc[(size_t)g * K + c];
-      same_off[(size_t)g * K + c] = same_tot[c];
-      left_off[(size_t)g * K + c] = left_tot[c];
-      list_off[(size_t)g * K + c] = list_tot[c];
-      stack_off[(size_t)g * K + c] = stack_tot[c];
-      stack_tot[c] += nstack[(size_t)g * K + c];
-      list_tot[c] += H * n;
-      if (class_multi(c)) {
-        same_tot[c] += H * (n / 2);
-        left_tot[c] += H * (n & 1);
-        cap_tot[c] += H * n;
-      } else {
-        same_tot[c] += chains[(size_t)g * K + c];
-        cap_tot[c] += cpairs[(size_t)g * K + c];
-        if (single_read[g] != kNoPair && read_class[single_read[g]] == c) left_tot[c] += H;
-      }
+      tot.same[c] += class_multi(c) ? bl.n.same[c] : bl.chains[c][cap_index[c]];
+      tot.left[c] += bl.n.left[c];
+      tot.list[c] += bl.n.list[c];
+      tot.cap[c] += bl.n.cap[c];
+      tot.stack[c] += bl.n.stack[c];
     }
   }
   // Multi-pass leftovers are paired with leftovers of the same pass count at
   // the class's strip height, so neither slot of an item sweeps passes of
   // pass-through rows only.  (A result does not depend on the partner: the
   // last pass always ends in pass-through rows, pipe_passes.)
-  auto passes_of = [&](uint32_t read) -> uint32_t {
-    const int c = read_class[read];
-    if (!class_multi(c)) return 1u;  // single-pass leftovers: one group
-    return pipe_passes(b.read_lengths[read], pipe_variant_rows(plan.variant[c]));
-  };
   std::vector<uint64_t> left_by_passes[2];
-  for (int u = 0; u < 2; ++u) left_by_passes[u].assign(RODV_MAX_READ_LEN / (kWarp * 4) + 2, 0);
-  for (uint32_t g = 0; g < G; ++g)
-    for (int u = 0; u < 2; ++u)
-      if (left_read[g * 2 + u] != kNoPair)
-        left_by_passes[u][passes_of(left_read[g * 2 + u])] += b.regions[g].num_haps;
+  for (int u = 0; u < 2; ++u) {
+    if (!tot.left[kSinglePassClasses + u]) continue;
+    left_by_passes[u].assign(RODV_MAX_READ_LEN / (kWarp * 4) + 2, 0);
+    for (uint32_t i = 0; i < G; ++i) {
+      const uint32_t r = blocks[i / kBlockRegions].regions[i % kBlockRegions].left[u];
+      if (r != kNoPair) left_by_passes[u][passes_of(r)] += b.regions[order[i]].num_haps;
+    }
+  }
   for (int c = 0; c < kNumClasses; ++c) {
     // FP64 list capacity: every pair whose FP32 work is in class c (or, FP64
     // forced, every pair whose read is of class c)
-    plan.pairs[c] = (uint32_t)(fp64 ? list_tot[c] : cap_tot[c]);
-    plan.same_items[c] = fp64 ? 0u : (uint32_t)same_tot[c];
-    uint64_t diff = (left_tot[c] + 1) / 2;  // single-pass leftovers pair freely
+    plan.pairs[c] = (uint32_t)(fp64 ? tot.list[c] : tot.cap[c]);
+    plan.same_items[c] = fp64 ? 0u : (uint32_t)tot.same[c];
+    uint64_t diff = (tot.left[c] + 1) / 2;  // single-pass leftovers pair freely
     if (class_multi(c)) {
       diff = 0;
       for (uint64_t n : left_by_passes[c - kSinglePassClasses]) diff += (n + 1) / 2;
     }
     plan.diff_items[c] = fp64 ? 0u : (uint32_t)diff;
   }
-  for (uint32_t g = 0; g < G; ++g) {
-    const rodv_region& rg = b.regions[g];
-    if (rc[(size_t)g * K + kSinglePassClasses] || rc[(size_t)g * K + kSinglePassClasses + 1])
-      for (uint32_t h = 0; h < rg.num_haps; ++h)
-        plan.multi_max_hap = std::max(plan.multi_max_hap, b.hap_lengths[rg.hap_start + h]);
-  }
-
   timer.mark("pairing");
   // ---- arena layout ----
   size_t o = 0;
@@ -757,7 +821,7 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
     const size_t item = class_multi(c) ? sizeof(SameItem) : sizeof(ChainItem);
     o = align_up(o + (size_t)plan.same_items[c] * item);
     plan.off_stack[c] = o;  // chain items' bins
-    if (!fp64 && !class_multi(c)) o = align_up(o + (size_t)stack_tot[c] * 4);
+    if (!fp64 && !class_multi(c)) o = align_up(o + (size_t)tot.stack[c] * 4);
   }
   for (int c = 0; c < kNumClasses; ++c) {
     plan.off_diff[c] = o;
@@ -804,14 +868,11 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   HapDesc* hd = reinterpret_cast<HapDesc*>(s + plan.off_haps);
   parallel_for(b.num_haps, 64, [&](size_t lo, size_t hi) {
     for (size_t h = lo; h < hi; ++h) {
-      const uint8_t* src = b.hap_bases + b.hap_offsets[h];
       uint8_t* dst = codes + hap_code_off[h];
       const uint32_t n = b.hap_lengths[h];
-      for (uint32_t k = 0; k < n; ++k) {
-        const uint8_t c = kCodes.v[src[k]];
-        if (c == 0xff) bad_base.store((int)src[k]);
-        dst[k] = c;
-      }
+      int bad = -1;
+      pack_codes(b.hap_bases + b.hap_offsets[h], n, dst, &bad);
+      if (bad >= 0) bad_base.store(bad);
       dst[n] = kSep;
       hd[h].code_off = hap_code_off[h];
       hd[h].len = n;
@@ -824,35 +885,22 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   // ---- read rows ----
   uint32_t* rw = reinterpret_cast<uint32_t*>(s + plan.off_read_rows);
   ReadDesc* rdesc = reinterpret_cast<ReadDesc*>(s + plan.off_reads);
+  const bool stream_rows = rows * 4 >= kStreamBytes;
   parallel_for(b.num_reads, 256, [&](size_t lo, size_t hi) {
     for (size_t r = lo; r < hi; ++r) {
       const uint64_t off = b.read_offsets[r];
       const uint32_t n = b.read_lengths[r];
-      uint32_t* dst = rw + row_off[r];
-      const uint8_t* base = b.read_bases + off;
-      const uint8_t* q = b.base_quals + off;
-      if (read_class[r] & 1) {
-        // uniform gaps: insertion, deletion and gcp qualities are the same
-        // on every row, so their fields are one constant
-        const uint32_t gaps = row_word(0, 0, b.ins_quals[off], b.del_quals[off], b.gcp_quals[off]);
-        for (uint32_t k = 0; k < n; ++k) {
-          const uint8_t c = kCodes.v[base[k]];
-          if (c == 0xff) bad_base.store((int)base[k]);
-          dst[k] = gaps | (c & 7u) | ((uint32_t)(q[k] & 127) << 3);
-        }
-      } else {
-        for (uint32_t k = 0; k < n; ++k) {
-          const uint8_t c = kCodes.v[base[k]];
-          if (c == 0xff) bad_base.store((int)base[k]);
-          dst[k] = row_word(c, q[k], b.ins_quals[off + k], b.del_quals[off + k],
-                            b.gcp_quals[off + k]);
-        }
-      }
-      for (uint32_t k = n; k < ((n + 3) & ~3u); ++k) dst[k] = 0;
+      int bad = -1;
+      pack_rows(b.read_bases + off,
+                ReadQuals{b.base_quals + off, b.ins_quals + off, b.del_quals + off,
+                          b.gcp_quals + off},
+                n, (read_class[r] & 1) != 0, stream_rows, rw + row_off[r], &bad);
+      if (bad >= 0) bad_base.store(bad);
       rdesc[r].row_off = row_off[r];
       rdesc[r].len = n;
       rdesc[r].flags = (read_class[r] & 1) ? kReadUniformGaps : 0u;
     }
+    pack_fence();
   });
   if (bad_base.load() >= 0) {
     char msg[96];
@@ -866,70 +914,64 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   }
   timer.mark("rows");
   // ---- work: chain items, same-haplotype items, leftovers, forced-FP64 lists ----
-  std::vector<uint64_t> region_out(G);
-  for (uint32_t g = 0, acc = 0; g < G; ++g) {
-    region_out[g] = acc;
-    acc += b.regions[g].num_haps * b.regions[g].num_reads;
-  }
   std::vector<PairRef> leftovers[kNumClasses];
-  for (int c = 0; c < kNumClasses; ++c) leftovers[c].resize(left_tot[c]);
-  parallel_for(G, 16, [&](size_t lo, size_t hi) {
+  for (int c = 0; c < kNumClasses && !fp64; ++c) leftovers[c].resize(tot.left[c]);
+  parallel_for(nblocks, 1, [&](size_t lo, size_t hi) {
     std::vector<uint32_t> byclass[kNumClasses];
-    std::vector<uint32_t> sr;
-    RegionChains chs;
-    for (size_t g = lo; g < hi; ++g) {
-      const rodv_region& rg = b.regions[g];
-      const uint32_t N = rg.num_reads;
-      // out index of (haplotype h of the region, read rr)
-      auto out_of = [&](uint32_t h, uint32_t rr) {
-        return (uint32_t)(region_out[g] + (uint64_t)h * N + (rr - rg.read_start));
-      };
-      if (!fp64) {
-        sorted_single(rg, sr);
-        region_chains(sr, chs);
-        uint64_t next[kNumClasses], snext[kNumClasses];
-        for (int c = 0; c < kNumClasses; ++c) {
-          next[c] = same_off[g * K + c];
-          snext[c] = stack_off[g * K + c];
-        }
-        for (const ChainPairs& cb : chs.items) {
+    for (size_t k = lo; k < hi; ++k) {
+      const Block& bl = blocks[k];
+      Counts n = at[k];  // next positions
+      for (size_t j = 0; j < bl.regions.size(); ++j) {
+        const RegionPlan& rp = bl.regions[j];
+        const uint32_t g = order[k * kBlockRegions + j];
+        const rodv_region& rg = b.regions[g];
+        const uint32_t N = rg.num_reads;
+        // out index of (haplotype h of the region, read rr)
+        auto out_of = [&](uint32_t h, uint32_t rr) {
+          return (uint32_t)(region_out[g] + (uint64_t)h * N + (rr - rg.read_start));
+        };
+        for (uint32_t q = rp.first_item; q < rp.end_item; ++q) {
+          const ChainPairs& cb = bl.items[q];
           const int c = cb.cls;
           ChainItem* ci = reinterpret_cast<ChainItem*>(s + plan.off_same[c]);
           uint32_t* stk = reinterpret_cast<uint32_t*>(s + plan.off_stack[c]);
-          const uint32_t e0 = (uint32_t)snext[c];
-          for (uint32_t j = 0; j < 2 * cb.pairs; ++j) stk[snext[c]++] = chs.reads[cb.first + j];
+          const uint32_t e0 = (uint32_t)n.stack[c];
+          const uint32_t* reads = bl.reads.data() + rp.first_read + cb.first;
+          for (uint32_t r = 0; r < 2 * cb.pairs; ++r) stk[n.stack[c]++] = reads[r];
           const uint32_t cap = plan.chain_haps[c];
           for (uint32_t h0 = 0; h0 < rg.num_haps; h0 += cap)
-            ci[next[c]++] = ChainItem{rg.hap_start + h0, std::min(cap, rg.num_haps - h0), e0,
-                                      cb.pairs, out_of(h0, rg.read_start), N, hmax[g],
-                                      rg.read_start};
+            ci[n.same[c]++] = ChainItem{rg.hap_start + h0, std::min(cap, rg.num_haps - h0), e0,
+                                        cb.pairs, out_of(h0, rg.read_start), N, hmax[g],
+                                        rg.read_start};
         }
-        if (single_read[g] != kNoPair) {
-          const uint32_t rr = single_read[g];
-          const int c = read_class[rr];
-          PairRef* lf = leftovers[c].data() + left_off[g * K + c];
+        if (rp.single != kNoPair) {
+          const int c = read_class[rp.single];
           for (uint32_t h = 0; h < rg.num_haps; ++h)
-            lf[h] = PairRef{rg.hap_start + h, rr, out_of(h, rr)};
+            leftovers[c][n.left[c]++] = PairRef{rg.hap_start + h, rp.single, out_of(h, rp.single)};
         }
-      }
-      for (auto& v : byclass) v.clear();
-      for (uint32_t r = 0; r < N; ++r) byclass[read_class[rg.read_start + r]].push_back(rg.read_start + r);
-      for (int c = 0; c < kNumClasses; ++c) {
-        const std::vector<uint32_t>& rd = byclass[c];
-        if (rd.empty() || (!fp64 && !class_multi(c))) continue;
-        SameItem* si = reinterpret_cast<SameItem*>(s + plan.off_same[c]) + same_off[g * K + c];
-        PairRef* lf = leftovers[c].data() + left_off[g * K + c];
-        PairRef* li = reinterpret_cast<PairRef*>(s + plan.off_lists[c]) + list_off[g * K + c];
-        for (uint32_t h = 0; h < rg.num_haps; ++h) {
-          const uint32_t hap = rg.hap_start + h;
-          if (fp64) {
-            for (uint32_t rr : rd) *li++ = PairRef{hap, rr, out_of(h, rr)};
-            continue;
+        bool any = fp64;
+        for (int u = 0; u < 2; ++u) any = any || plan.pairs[kSinglePassClasses + u] > 0;
+        if (!any) continue;  // only chain items and single-pass leftovers
+        for (auto& v : byclass) v.clear();
+        for (uint32_t r = rg.read_start; r < rg.read_start + N; ++r)
+          if (fp64 || class_multi(read_class[r])) byclass[read_class[r]].push_back(r);
+        for (int c = 0; c < kNumClasses; ++c) {
+          const std::vector<uint32_t>& rd = byclass[c];
+          if (rd.empty()) continue;
+          SameItem* si = reinterpret_cast<SameItem*>(s + plan.off_same[c]);
+          PairRef* li = reinterpret_cast<PairRef*>(s + plan.off_lists[c]);
+          for (uint32_t h = 0; h < rg.num_haps; ++h) {
+            const uint32_t hap = rg.hap_start + h;
+            if (fp64) {
+              for (uint32_t rr : rd) li[n.list[c]++] = PairRef{hap, rr, out_of(h, rr)};
+              continue;
+            }
+            size_t r = 0;
+            for (; r + 1 < rd.size(); r += 2)
+              si[n.same[c]++] = SameItem{hap, rd[r], rd[r + 1], out_of(h, rd[r])};
+            if (r < rd.size())
+              leftovers[c][n.left[c]++] = PairRef{hap, rd[r], out_of(h, rd[r])};
           }
-          size_t k = 0;
-          for (; k + 1 < rd.size(); k += 2)
-            *si++ = SameItem{hap, rd[k], rd[k + 1], out_of(h, rd[k])};
-          if (k < rd.size()) *lf++ = PairRef{hap, rd[k], out_of(h, rd[k])};
         }
       }
     }
@@ -940,11 +982,13 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
     // haplotype), paired longest-first within the group
     for (int c = 0; c < kNumClasses; ++c) {
       std::vector<PairRef>& lv = leftovers[c];
-      std::stable_sort(lv.begin(), lv.end(), [&](const PairRef& x, const PairRef& y) {
+      auto before = [&](const PairRef& x, const PairRef& y) {
         const uint32_t px = passes_of(x.read), py = passes_of(y.read);
         if (px != py) return px > py;
         return b.hap_lengths[x.hap] > b.hap_lengths[y.hap];
-      });
+      };
+      if (!std::is_sorted(lv.begin(), lv.end(), before))
+        std::stable_sort(lv.begin(), lv.end(), before);
       DiffItem* di = reinterpret_cast<DiffItem*>(s + plan.off_diff[c]);
       size_t n = 0;
       for (size_t k = 0; k < lv.size();) {
@@ -977,15 +1021,6 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
     }
   }
   timer.mark("work");
-  // cells
-  uint64_t cells = 0;
-  for (uint32_t g = 0; g < G; ++g) {
-    const rodv_region& rg = b.regions[g];
-    uint64_t rs = 0;
-    for (uint32_t r = 0; r < rg.num_reads; ++r) rs += b.read_lengths[rg.read_start + r];
-    cells += hsum[g] * rs;
-  }
-  plan.cells = cells;
   return RODV_OK;
 }
 

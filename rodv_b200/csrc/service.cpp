@@ -276,9 +276,11 @@ void Service::worker() {
         }
       } else {
         // Batches in flight, and no launch due or nothing queued: look again
-        // in 50 us, or as soon as something arrives while a launch is due.
-        cv_work_.wait_for(lk, std::chrono::microseconds(50),
-                          [&] { return can_launch && !pending_.empty(); });
+        // in a few microseconds.  (Asleep here, the worker cost every submit
+        // meanwhile a wake-up call.)
+        lk.unlock();
+        const Clock::time_point until = Clock::now() + std::chrono::microseconds(4);
+        while (Clock::now() < until) std::this_thread::yield();
         continue;
       }
     }
