@@ -1248,11 +1248,15 @@ static void fill_stats(rodv_stats* st, const PackedPlan& plan, const uint32_t* c
 // ms against 133).  Running every range's kernels on one stream was slower
 // (159 ms): concurrent ranges fill each other's per-class tails.
 constexpr double kChunkCells = 1.2e11;
-constexpr double kFirstChunkCells = 4e9;
-// first range: 1/32 of the batch's cells, at least 4e9 (1/64 measured the
-// same on the uneven batch: 121.2-121.7 ms per call either way)
+// First range: 1/32 of the batch's cells (1/64 measured the same on the uneven
+// batch: 121.2-121.7 ms per call either way), at least 2e9: a batch of more
+// than that is cut in two or more, and one of a few milliseconds packs and
+// uploads behind its own kernels (6e9 cells of uneven regions 2.57 ms in one
+// piece, 2.27 cut, 2.49-2.57 from 5e8 cells; 4e9 cells of 40,000 one-pair
+// regions 7.9 and 6.2; 1.7e10 per-row-gap cells 7.8 and 6.6).
+constexpr double kFirstChunkCells = 2e9;
 constexpr double kFirstChunkDiv = 32;
-constexpr double kMinChunkedCells = 2e10;
+constexpr double kMinChunkedCells = 2e9;
 
 // Range sizes, overridable for tuning (RODV_CHUNK_CELLS, RODV_FIRST_CHUNK_CELLS,
 // RODV_FIRST_CHUNK_DIV).
