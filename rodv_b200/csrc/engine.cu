@@ -257,7 +257,7 @@ Engine::~Engine() {
     cudaStreamSynchronize(stream_);
     for (auto& e : ev_) cudaEventDestroy(e);
     cudaStreamDestroy(stream_);
-    for (int c = 0; c < kNumClasses; ++c) {
+    for (int c = 0; c < kBranches; ++c) {
       if (side_[c]) cudaStreamSynchronize(side_[c]);
       if (side_[c]) cudaStreamDestroy(side_[c]);
       if (join_ev_[c]) cudaEventDestroy(join_ev_[c]);
@@ -310,7 +310,7 @@ rodv_status Engine::init() {
   for (auto& e : ev_) RODV_CUDA(cudaEventCreate(&e));
   ready_ = true;  // the destructor releases what was created
   RODV_CUDA(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
-  for (int c = 0; c < kNumClasses; ++c) {
+  for (int c = 0; c < kBranches; ++c) {
     RODV_CUDA(cudaStreamCreateWithFlags(&side_[c], cudaStreamNonBlocking));
     RODV_CUDA(cudaEventCreateWithFlags(&join_ev_[c], cudaEventDisableTiming));
   }
@@ -1129,11 +1129,11 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
   // used side stream back into `stream`.  A part of one branch (a region of
   // equal reads) forks nothing: each event call costs about a microsecond of a
   // call that takes a hundred.
-  bool forked[kNumClasses] = {};
-  int main_cls = -1;
+  bool forked[kBranches] = {};
+  int main_branch = -1;
   auto lane = [&](int c) -> cudaStream_t {
-    if (main_cls < 0) main_cls = c;
-    if (!fan_out || c == main_cls) return stream;
+    if (main_branch < 0) main_branch = c;
+    if (!fan_out || c == main_branch) return stream;
     if (!forked[c]) {
       if (cudaStreamWaitEvent(side_[c], fork_ev_, 0) != cudaSuccess) return nullptr;
       forked[c] = true;
@@ -1142,11 +1142,11 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
   };
   auto fork = [&](int branches) -> cudaError_t {
     for (bool& f : forked) f = false;
-    main_cls = -1;
+    main_branch = -1;
     return fan_out && branches > 1 ? cudaEventRecord(fork_ev_, stream) : cudaSuccess;
   };
   auto join = [&]() -> cudaError_t {
-    for (int c = 0; c < kNumClasses && fan_out; ++c) {
+    for (int c = 0; c < kBranches && fan_out; ++c) {
       if (!forked[c]) continue;
       cudaError_t e = cudaEventRecord(join_ev_[c], side_[c]);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, join_ev_[c], 0);
@@ -1168,8 +1168,19 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
   }
   if (ev) RODV_CUDA(cudaEventRecord(ev[0], stream));
   if (!plan.fp64 && (parts & 1)) {
+    // A single-pass class's two-haplotype items (its regions' odd reads) are a
+    // branch of their own: a handful of items behind the class's chains added
+    // their whole sweep to a small batch (7 regions of per-row-gap reads: 131 us
+    // on the device, 103 so).
+    // The multi-pass classes' two kinds share boundary rows and stay in
+    // sequence.
+    auto branch = [](int c, bool same) {
+      return same || class_multi(c) ? c : c + kNumClasses;
+    };
     int branches = 0;
-    for (int c = 0; c < kNumClasses; ++c) branches += plan.same_items[c] + plan.diff_items[c] > 0;
+    for (int c = 0; c < kNumClasses; ++c)
+      branches += class_multi(c) ? plan.same_items[c] + plan.diff_items[c] > 0
+                                 : (plan.same_items[c] > 0) + (plan.diff_items[c] > 0);
     RODV_CUDA(fork(branches));
     // the longest reads first: the short items of the small classes fill the
     // tail (300 regions of 1-300 reads x 1-32 haplotypes: 7.5 ms shortest
@@ -1177,7 +1188,7 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
     for (int c = kNumClasses - 1; c >= 0; --c) {
       for (int same = 1; same >= 0; --same) {
         if (!(same ? plan.same_items[c] : plan.diff_items[c])) continue;
-        const cudaStream_t ls = lane(c);
+        const cudaStream_t ls = lane(branch(c, same != 0));
         if (!ls) return cuda_fail(cudaErrorUnknown, "class stream fork");
         rodv_status s = launch_fp32_class(plan, dbase, c, same != 0, plan.variant[c], 0, ls);
         if (s != RODV_OK) return s;

@@ -214,8 +214,11 @@ class Engine {
   std::string device_name_;
   cudaStream_t stream_ = nullptr;
   cudaEvent_t ev_[4] = {};
-  cudaStream_t side_[kNumClasses] = {};  // launch_all fan-out, one per class
-  cudaEvent_t fork_ev_ = nullptr, join_ev_[kNumClasses] = {};
+  // launch_all fan-out: one per class, then one per single-pass class's
+  // two-haplotype items
+  static constexpr int kBranches = 2 * kNumClasses;
+  cudaStream_t side_[kBranches] = {};
+  cudaEvent_t fork_ev_ = nullptr, join_ev_[kBranches] = {};
   DeviceMem tables_;
   PriorTables tab_{};
   int variant_[kNumClasses] = {};          // tuned FP32 kernel variant per class
