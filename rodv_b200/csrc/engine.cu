@@ -827,24 +827,28 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
     plan.off_diff[c] = o;
     o = align_up(o + (size_t)plan.diff_items[c] * sizeof(DiffItem));
   }
-  const size_t lists_begin = o;
-  for (int c = 0; c < kNumClasses; ++c) {
-    plan.list_cap[c] = plan.pairs[c];
-    if (!fp64 && class_multi(c))
-      plan.list_cap[c] = std::max(plan.pairs[c], 2u * (plan.same_items[c] + plan.diff_items[c]));
-    plan.off_lists[c] = o;
-    o = align_up(o + (size_t)plan.list_cap[c] * sizeof(PairRef));
-  }
-  // forced FP64: the lists are full from the start; their lengths are uploaded
-  // too and copied into the counters at every run
+  auto layout_lists = [&]() {
+    for (int c = 0; c < kNumClasses; ++c) {
+      plan.list_cap[c] = plan.pairs[c];
+      if (!fp64 && class_multi(c))
+        plan.list_cap[c] =
+            std::max(plan.pairs[c], 2u * (plan.same_items[c] + plan.diff_items[c]));
+      plan.off_lists[c] = o;
+      o = align_up(o + (size_t)plan.list_cap[c] * sizeof(PairRef));
+    }
+  };
+  // FP32 runs fill the lists on the device; only forced-FP64 lists are uploaded
+  // (full from the start, with their lengths, which a rerun copies into the
+  // counters).  The counters end the upload: the ones a run starts from.
+  if (fp64) layout_lists();
   plan.off_preset = o;
   if (fp64) o = align_up(o + kNumClasses * 4);
-  // FP32 runs fill the lists on the device; only forced-FP64 lists are uploaded.
-  plan.upload_bytes = fp64 ? o : lists_begin;
-  plan.off_out = o; o = align_up(o + pairs * 8);
   plan.off_counts = o; o = align_up(o + kCountWords * 4);
+  plan.upload_bytes = o;
+  plan.off_out = o; o = align_up(o + pairs * 8);
   plan.off_prec = o;
   if (raw) o = align_up(o + pairs);
+  if (!fp64) layout_lists();
   plan.scratch_cols = plan.multi_max_hap ? plan.multi_max_hap + kBoundaryPad : 0;
   plan.off_scratch = o;
   if (plan.scratch_cols) {
@@ -908,9 +912,11 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
     return fail(RODV_ERR_INVALID_BASE, msg);
   }
 
+  uint32_t* counts = reinterpret_cast<uint32_t*>(s + plan.off_counts);
+  std::memset(counts, 0, kCountWords * 4);
   if (fp64) {
     uint32_t* preset = reinterpret_cast<uint32_t*>(s + plan.off_preset);
-    for (int c = 0; c < kNumClasses; ++c) preset[c] = plan.pairs[c];
+    for (int c = 0; c < kNumClasses; ++c) preset[c] = counts[kCtrRescue + c] = plan.pairs[c];
   }
   timer.mark("rows");
   // ---- work: chain items, same-haplotype items, leftovers, forced-FP64 lists ----
@@ -1121,7 +1127,8 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
 }
 
 rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stats* st,
-                               cudaStream_t stream, cudaEvent_t* ev, int parts, bool fan_out) {
+                               cudaStream_t stream, cudaEvent_t* ev, int parts, bool fan_out,
+                               bool reset) {
   ArenaView a = arena_view(plan, dbase, tab_);
   uint32_t launches = 0;
   // fan-out: the first branch of a part stays on `stream`; the first launch of
@@ -1154,11 +1161,13 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
     }
     return cudaSuccess;
   };
-  if (parts & 1) {
+  if (reset) {
     RODV_CUDA(cudaMemsetAsync(a.counts, 0, kCountWords * 4, stream));
     if (plan.fp64)  // every pair goes to the FP64 kernels: the uploaded lists are full
       RODV_CUDA(cudaMemcpyAsync(a.counts + kCtrRescue, dbase + plan.off_preset,
                                 kNumClasses * 4, cudaMemcpyDeviceToDevice, stream));
+  }
+  if (parts & 1) {
     // multi-pass classes' lists: every position empty (kNoPair) until a
     // rescue fills it (kLaunchRescueByItem)
     for (int c = kSinglePassClasses; c < kNumClasses && !plan.fp64; ++c)
@@ -1327,15 +1336,16 @@ rodv_status Engine::finish_lane(HostLane& l, double* out, rodv_stats* st, uint8_
   }
   const PackedPlan& p = l.plan;
   const uint8_t* h = static_cast<const uint8_t*>(l.out.ptr);
-  const uint32_t* counts = reinterpret_cast<const uint32_t*>(h + p.num_pairs * 8);
+  const uint32_t* counts = reinterpret_cast<const uint32_t*>(h);
   if (counts[kCtrError] != 0)
     return fail(RODV_ERR_DEVICE_CHECK,
                 "kernel reported error flags " + std::to_string(counts[kCtrError]));
   // results into the caller's (pageable) buffer, 128K pairs per task: the
   // last range's copy is on the call's critical path
-  const uint8_t* hp = h + p.num_pairs * 8 + kCountWords * 4;  // raw mode: precisions
+  const uint8_t* ho = h + p.result_out();
+  const uint8_t* hp = h + p.result_prec();  // raw mode: precisions
   parallel_for(p.num_pairs, 1u << 17, [&](size_t lo, size_t hi) {
-    std::memcpy(out + l.out_off + lo, h + lo * 8, (hi - lo) * 8);
+    std::memcpy(out + l.out_off + lo, ho + lo * 8, (hi - lo) * 8);
     if (prec) std::memcpy(prec + l.out_off + lo, hp + lo, hi - lo);
   });
   if (st) {
@@ -1417,7 +1427,7 @@ rodv_status Engine::run_host_chunked(const rodv_batch& b, double* out, rodv_stat
     const PackedPlan& p = l.plan;
     cudaError_t e = cudaSuccess;
     if (l.arena.bytes < p.total_bytes) e = l.arena.ensure(p.total_bytes + p.total_bytes / 4);
-    const size_t ob = p.num_pairs * 8 + kCountWords * 4 + (p.raw ? p.num_pairs : 0);
+    const size_t ob = p.result_bytes();
     if (e == cudaSuccess && l.out.bytes < ob) e = l.out.ensure(ob + ob / 4);
     uint8_t* d = static_cast<uint8_t*>(l.arena.ptr);
     uint8_t* h = static_cast<uint8_t*>(l.out.ptr);
@@ -1432,13 +1442,7 @@ rodv_status Engine::run_host_chunked(const rodv_batch& b, double* out, rodv_stat
     // per call of the uneven batch against 132-134 without)
     result = launch_all(p, d, &acc, l.stream, l.ev, 3, /*fan_out=*/true);
     if (result != RODV_OK) break;
-    e = cudaMemcpyAsync(h, d + p.off_out, p.num_pairs * 8, cudaMemcpyDeviceToHost, l.stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(h + p.num_pairs * 8, d + p.off_counts, kCountWords * 4,
-                          cudaMemcpyDeviceToHost, l.stream);
-    if (e == cudaSuccess && p.raw)
-      e = cudaMemcpyAsync(h + p.num_pairs * 8 + kCountWords * 4, d + p.off_prec, p.num_pairs,
-                          cudaMemcpyDeviceToHost, l.stream);
+    e = cudaMemcpyAsync(h, d + p.off_counts, ob, cudaMemcpyDeviceToHost, l.stream);
     if (e == cudaSuccess) e = cudaEventRecord(l.done, l.stream);
     if (e != cudaSuccess) {
       result = cuda_fail(e, "chunk download");
@@ -1477,8 +1481,7 @@ rodv_status Engine::run_host_single(const rodv_batch& b, double* out, rodv_stats
   rodv_status s = pack(b, plan, staging_, fp64, prec != nullptr);
   if (s != RODV_OK) return s;
   RODV_CUDA(arena_.ensure(plan.total_bytes));
-  RODV_CUDA(out_staging_.ensure(plan.num_pairs * 8 + kCountWords * 4 +
-                                (prec ? plan.num_pairs : 0)));
+  RODV_CUDA(out_staging_.ensure(plan.result_bytes()));
   uint8_t* d = static_cast<uint8_t*>(arena_.ptr);
   RODV_CUDA(cudaEventRecord(ev_[3], stream_));
   RODV_CUDA(cudaMemcpyAsync(d, staging_.ptr, plan.upload_bytes, cudaMemcpyHostToDevice, stream_));
@@ -1488,21 +1491,19 @@ rodv_status Engine::run_host_single(const rodv_batch& b, double* out, rodv_stats
   s = launch_all(plan, d, st, stream_, ev_, 3, /*fan_out=*/true);
   if (s != RODV_OK) return s;
   uint8_t* hs = static_cast<uint8_t*>(out_staging_.ptr);
-  RODV_CUDA(cudaMemcpyAsync(hs, d + plan.off_out, plan.num_pairs * 8, cudaMemcpyDeviceToHost,
-                            stream_));
-  RODV_CUDA(cudaMemcpyAsync(hs + plan.num_pairs * 8, d + plan.off_counts, kCountWords * 4,
+  // counters and results in one copy; the counters came with the upload (a
+  // reset and a copy of their own cost a call of one pair 5 us of 80)
+  RODV_CUDA(cudaMemcpyAsync(hs, d + plan.off_counts, plan.result_bytes(),
                             cudaMemcpyDeviceToHost, stream_));
-  if (prec)
-    RODV_CUDA(cudaMemcpyAsync(hs + plan.num_pairs * 8 + kCountWords * 4, d + plan.off_prec,
-                              plan.num_pairs, cudaMemcpyDeviceToHost, stream_));
   RODV_CUDA(cudaStreamSynchronize(stream_));
-  const uint32_t* counts = reinterpret_cast<const uint32_t*>(hs + plan.num_pairs * 8);
+  const uint32_t* counts = reinterpret_cast<const uint32_t*>(hs);
   if (counts[kCtrError] != 0)
     return fail(RODV_ERR_DEVICE_CHECK,
                 "kernel reported error flags " + std::to_string(counts[kCtrError]));
-  const uint8_t* hp = hs + plan.num_pairs * 8 + kCountWords * 4;
+  const uint8_t* ho = hs + plan.result_out();
+  const uint8_t* hp = hs + plan.result_prec();
   parallel_for(plan.num_pairs, 1u << 17, [&](size_t lo, size_t hi) {
-    std::memcpy(out + lo, hs + lo * 8, (hi - lo) * 8);
+    std::memcpy(out + lo, ho + lo * 8, (hi - lo) * 8);
     if (prec) std::memcpy(prec + lo, hp + lo, hi - lo);
   });
   if (st) {
@@ -1557,7 +1558,8 @@ rodv_status Engine::run_device(rodv_device_batch* db, rodv_stats* st) {
       rodv_stats cap{};
       RODV_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
       rodv_status s =
-          launch_all(db->plan, d, &cap, stream_, nullptr, part == 0 ? 1 : 2, /*fan_out=*/true);
+          launch_all(db->plan, d, &cap, stream_, nullptr, part == 0 ? 1 : 2, /*fan_out=*/true,
+                     /*reset=*/part == 0);
       cudaGraph_t g = nullptr;
       const cudaError_t ce = cudaStreamEndCapture(stream_, &g);
       if (s != RODV_OK) {

@@ -84,6 +84,13 @@ struct PackedPlan {
   // uniform classes run the kernels that take them as constants.
   bool const_gaps = false;
   GapConsts gaps = {};
+  // The part of the arena a call downloads, and where it holds the results and
+  // (raw mode) the precisions.
+  size_t result_bytes() const {
+    return (raw ? off_prec + num_pairs : off_out + num_pairs * 8) - off_counts;
+  }
+  size_t result_out() const { return off_out - off_counts; }
+  size_t result_prec() const { return off_prec - off_counts; }
   GapForm gap_form(int cls) const {
     return !class_uniform(cls) ? kGapsPerRow : const_gaps ? kGapsConst : kGapsUniform;
   }
@@ -105,7 +112,9 @@ struct PackedPlan {
   size_t off_lists[kNumClasses] = {};      // FP64 work lists (rescued or forced)
   size_t off_preset = 0;                   // forced FP64: list lengths (uploaded)
   size_t upload_bytes = 0;                 // the H2D part starts at 0
-  size_t off_out = 0, off_counts = 0, off_scratch = 0;
+  // the counters (uploaded as a run starts from), then the results, so that
+  // one copy brings both back
+  size_t off_counts = 0, off_out = 0, off_scratch = 0;
   size_t off_prec = 0;                     // raw mode: precision byte per pair
   size_t total_bytes = 0;
   size_t scratch_bytes[2] = {0, 0};        // of the per-row and the uniform multi-pass class
@@ -178,7 +187,8 @@ class Engine {
   // every class keeps its own reads; the autotuner's per-class batches)
   rodv_status pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& staging, bool fp64,
                    bool raw = false, bool stack = true);
-  // parts: 1 = counter reset and FP32 launches, 2 = FP64 launches.  ev: null,
+  // parts: 1 = FP32 launches, 2 = FP64 launches; reset: the counters first (a
+  // rerun; a fresh upload brings them).  ev: null,
   // or three events recorded before the FP32 launches, between the two parts
   // and after the FP64 launches.  fan_out: each class's launches go to its own
   // side stream (forked from and joined back into `stream`), so that class
@@ -187,7 +197,7 @@ class Engine {
   // use them from the one thread that launches for the engine at a time.
   rodv_status launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stats* st,
                          cudaStream_t stream, cudaEvent_t* ev, int parts,
-                         bool fan_out = false);
+                         bool fan_out = false, bool reset = false);
   rodv_status launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int cls, bool same,
                                 int variant, int blocks_cap, cudaStream_t stream);
   rodv_status launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int cls, int variant,

@@ -99,7 +99,7 @@ rodv_status Service::init() {
     // staging holds at most the estimate; results are 8 of its ~36 bytes per pair
     if (e == cudaSuccess) e = s.staging.ensure(batch_bytes_);
     if (e == cudaSuccess) e = s.arena.ensure(batch_bytes_);
-    if (e == cudaSuccess) e = s.out_host.ensure(batch_bytes_ / 4 + kCountWords * 4);
+    if (e == cudaSuccess) e = s.out_host.ensure(batch_bytes_ / 4 + 1024);
   }
   if (e != cudaSuccess) {
     st = engine_.cuda_fail(e, "service buffers");
@@ -408,7 +408,7 @@ rodv_status Service::launch(Slot& s) {
   const Clock::time_point t_pack = Clock::now();
   const PackedPlan& p = s.plan;
   cudaError_t e = grow(s.arena, p.total_bytes);
-  if (e == cudaSuccess) e = grow(s.out_host, p.num_pairs * 8 + kCountWords * 4);
+  if (e == cudaSuccess) e = grow(s.out_host, p.result_bytes());
   if (e != cudaSuccess) return engine_.cuda_fail(e, "service buffers");
   uint8_t* d = static_cast<uint8_t*>(s.arena.ptr);
   uint8_t* h = static_cast<uint8_t*>(s.out_host.ptr);
@@ -426,10 +426,7 @@ rodv_status Service::launch(Slot& s) {
   st = engine_.launch_all(p, d, nullptr, s.stream, s.ev, 3, /*fan_out=*/true);
   if (st != RODV_OK) return st;
   prev_kernels_ = s.ev[2];
-  e = cudaMemcpyAsync(h, d + p.off_out, p.num_pairs * 8, cudaMemcpyDeviceToHost, s.stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(h + p.num_pairs * 8, d + p.off_counts, kCountWords * 4,
-                        cudaMemcpyDeviceToHost, s.stream);
+  e = cudaMemcpyAsync(h, d + p.off_counts, p.result_bytes(), cudaMemcpyDeviceToHost, s.stream);
   if (e == cudaSuccess) e = cudaEventRecord(s.done, s.stream);
   if (e != cudaSuccess) return engine_.cuda_fail(e, "service download");
   if (opt_.verbose >= 2)
@@ -455,7 +452,7 @@ void Service::complete(Slot& s) {
   const Clock::time_point t0 = Clock::now();
   const PackedPlan& p = s.plan;
   const uint8_t* h = static_cast<const uint8_t*>(s.out_host.ptr);
-  const uint32_t* counts = reinterpret_cast<const uint32_t*>(h + p.num_pairs * 8);
+  const uint32_t* counts = reinterpret_cast<const uint32_t*>(h);
   if (counts[kCtrError] != 0) {
     fail_slot(s, engine_.fail(RODV_ERR_DEVICE_CHECK, "kernel reported error flags " +
                                                          std::to_string(counts[kCtrError])));
@@ -465,7 +462,7 @@ void Service::complete(Slot& s) {
   cudaEventElapsedTime(&ms, s.ev[0], s.ev[2]);
   uint64_t fp64 = 0;
   for (int c = 0; c < kNumClasses; ++c) fp64 += p.fp64 ? p.pairs[c] : counts[kCtrRescue + c];
-  const double* res = reinterpret_cast<const double*>(h);
+  const double* res = reinterpret_cast<const double*>(h + p.result_out());
   uint64_t off = 0;
   for (const auto& r : s.reqs) {
     r->out.assign(res + off, res + off + r->pairs);
