@@ -1,19 +1,32 @@
-// pairhmm_pipe.cuh -- multi-pass sweeps of long reads with the passes of one
-// work item running concurrently on the warps of a block.
+// pairhmm_pipe.cuh -- multi-pass sweeps of long reads: the passes of a block's
+// work items run concurrently on the warps of the block.
 //
 // A read longer than one pass (32 lanes x R rows) is swept in passes of 32R
 // rows; pass p needs the last row of pass p-1 (its boundary row) column by
 // column.  Swept one pass after the other by one warp, a pair of a 2,000-base
 // read and a 5,000-base haplotype takes 8 x 5,031 steps in sequence, and the
-// longest pairs of a batch set the length of the whole launch.  Here the W
-// warps of a block take one work item together: warp w sweeps passes w, w+W,
-// w+2W, ...  Lane 31 of the warp on pass p writes the pass's last row into a
-// boundary row in global memory and publishes, after every 32 steps, how far
-// it has come; lane 0 of the warp on pass p+1 reads that row through a
-// shared-memory ring (cp.async, 32 columns ahead), waiting for the
-// publication before each chunk.  Pass p+1 thus trails pass p by about 100
-// steps instead of a whole pass, and the item's sweep takes about ceil(P/W)
-// passes plus (W-1) x 100 steps.
+// longest pairs of a batch set the length of the whole launch.  Here lane 31 of
+// the warp on pass p writes the pass's last row into a boundary row in global
+// memory and publishes, after every 32 steps, how far it has come; lane 0 of the
+// warp on pass p+1 reads that row through a shared-memory ring (cp.async, 32
+// columns ahead), waiting for the publication before each chunk.  Pass p+1 can
+// thus trail pass p by about 100 steps instead of a whole pass.
+//
+// Tasks.  A block's W warps take passes one by one (acquire): a warp that ends
+// one takes the next, of the same item or of another, with no barrier between
+// items.  (With a team of W warps per item, warp w on passes w, w+W, ..., and a
+// block barrier at its end, six passes kept four warps busy three quarters of
+// the time, and a rejected item's W passes in flight were all swept.)  An open
+// item -- one with a pass started and not all ended -- occupies one of W slots.
+// The choice, in this order: the oldest open item's next pass, if fewer than
+// kWindow of its started passes have yet to end; a new item from the queue, up
+// to the block's even share of the queue; any open item's next pass; a new
+// item.  FP32 items are held to two passes in flight, so that an item rejected
+// after a pass (below) has swept at most one pass more; a queue too short to
+// fill the block lifts that.  FP64 items take every pass as soon as a warp is
+// free: the longest item comes first and ends soonest.  Measured with the team
+// of four warps before: 1,500 pairs of 1,500 x 3,500 bases 2.87 -> 2.55 ms in
+// FP32, 1.70 -> 1.31 where every pair is rejected, 4.83 -> 4.28 in FP64.
 //
 // What crosses a pass boundary is what the lanes of a warp hand each other.
 // In the scaled form (uniform gaps) that is two values per column: the M term
@@ -23,38 +36,33 @@
 // are bitwise those of a three-value hand-over of (M~, I^, D^).  Other forms
 // hand over (M, I, D).  A boundary cell is 16 or 24 bytes.
 //
-// Boundary rows.  A block owns W+1 rows; pass p writes row p mod (W+1) and
-// reads row (p-1) mod (W+1).  The next pass to write a row, p+W+1, runs on
-// the same warp as p+1, the row's only reader, after p+1 has finished, so a
-// producer never waits for a consumer.  Every wait is a consumer (pass p)
-// waiting for its producer (pass p-1): waits point to strictly earlier
-// passes, so they cannot form a cycle.  Each wait also gives up after a
-// bounded number of polls, sets kErrWaitTimeout and stops the item, so a
-// kernel always ends.  A row starts with kPad cells before its column 0:
-// lane 31 stores its hand-over every step, the first 31 of which are columns
-// <= 0 (zeros, never read), so no store needs a column test.
+// Boundary rows.  A block owns 2W rows; a started pass but the last owns one
+// until both it and the pass that reads it have ended (an item that is closed
+// early keeps its rows until its last pass in flight has ended).  W-1 other
+// warps are in passes, each with two rows at most, and an item between passes
+// keeps one, so a row is free for every pass; only while a closed item's last
+// pass leaves may a warp have to look again.  Every
+// wait is a pass waiting for the item's previous pass, which was started before
+// it: waits cannot form a cycle.  Each wait also gives up after a bounded number
+// of polls, sets kErrWaitTimeout and stops the block's warps, so a kernel always
+// ends.  A row starts with kPad cells before its column 0: lane 31 stores its
+// hand-over every step, the first of which are columns <= 0 (zeros, never read),
+// so no store needs a column test.
 //
 // Progress words live in shared memory: (pass << 17) | column, written with a
 // CTA-scope release by the producing lane after its row stores (and a block
 // fence), read with a CTA-scope acquire by every lane of the consumer before
 // it copies the chunk.  The warps are in one block, so they share the SM's
-// L1 and the CTA scope suffices.
+// L1 and the CTA scope suffices.  The rest of the block's state (Ctl) is
+// changed by one lane at a time under a lock.
 //
 // FP32 items stop early as in the single-warp sweep: after each pass but the
 // last, the warp that swept it bounds the likelihood by the sum over the row
 // it wrote (rejects(), the bound of Forward::row_bound_rejects restated for
 // the hand-over cells); once both slots are below the acceptance bound the
-// item stops on every warp and both pairs go to FP64.  The bound is exact, so
-// the rescued pairs and every result are those of the full sweep.  (Holding
-// pass 1 back until pass 0's verdict, so that a rejected item costs one pass
-// instead of the passes in flight, made no difference on 2,000 pairs of
-// 1,000-2,000-base reads and 2,000-5,000-base haplotypes that all go to FP64
-// (2.92 ms FP32 pass either way, since the warps of these latency-bound
-// sweeps leave issue slots free); at a quarter of the pairs it was slower,
-// 1.34 against 1.19 ms.)
+// item is closed and both pairs go to FP64.  The bound is exact, so the
+// rescued pairs and every result are those of the full sweep.
 //
-// Results are committed after a block barrier at the end of the item: by the
-// warp that swept the last pass, or, for a rejected item, as FP64 rescues.
 // The per-cell arithmetic is the single-warp sweep's (Forward::cells), and the
 // pass count (pipe_passes, layout.h) leaves at least one pass-through row at
 // the end, so a result is always the column sum of the I of a pass-through
@@ -129,25 +137,50 @@ struct PipeForward {
   };
   using Cell = typename std::conditional<kTwo, HandCell, typename F::BoundaryCell>::type;
   static_assert(sizeof(Cell) <= 24, "the engine sizes boundary rows at 24 bytes a cell");
-  static constexpr int kRows = W + 1;                   // boundary rows per block
+  static constexpr int kRows = 2 * W;                   // boundary rows per block
+  // started passes of an item that may be in flight before it has to wait
+  static constexpr uint32_t kWindow = P::kSlots == 2 ? 2u : ~0u;
   // Columns a lane runs behind its left neighbour.  FP64 (two-value form): two,
   // so a value shuffled in one step is used in the next (Forward::run_single).
   static constexpr int kLag = kTwo && P::kSlots == 1 ? 2 : 1;
   static constexpr int kPad = kLag * kWarp;             // cells before column 0 of a row
   static_assert(kPad + 8 <= kBoundaryPad, "the engine sizes boundary rows");
   // Steps per loop iteration of a whole chunk: eight at 168 registers (12 warps
-  // per SM).  2,000-pair batches of 1,500 x 3,500 bases: FP32 2.46 ms, FP64
-  // 4.77 (four steps 2.46 and 4.90); at 128 registers and 16 warps both spill
-  // (2.77 and 4.47 at eight steps, 3.4 and 5.0 at four).
+  // per SM).  4,440 pairs of 1,500 x 3,500 bases: FP32 6.48 ms, FP64 11.2 (four
+  // steps 6.46 and 11.3, sixteen 6.34 and 11.5); at 128 registers and 16 warps,
+  // with spills, 6.80 and 11.2 (four steps 6.78 and 12.1), and a lone item takes
+  // 0.92 and 0.78 ms instead of 0.81 and 0.72.
   static constexpr int kUnroll = 8;
   static constexpr int kSmemPerWarp = F::kSmemPerWarp;  // emission table + cell ring
   // polls of a progress word (about 100 ns each) before a wait gives up
   static constexpr uint32_t kWaitPolls = 1u << 24;
-  static constexpr uint32_t kStopRejected = 1u, kStopFailed = 2u;
+  static constexpr uint32_t kLockPolls = 1u << 22;
 
+  enum : uint32_t { kFree = 0, kOpen = 1, kClosed = 2 };  // Open::state
+  struct Open {
+    uint32_t state;
+    uint32_t item, passes;
+    uint32_t next;       // first pass not started
+    uint32_t done;       // passes ended
+    uint32_t running;    // passes in flight
+    uint32_t rows;       // boundary rows held (bits)
+    uint32_t wrote, read;  // of these: the pass that writes it, that reads it, has ended
+    uint32_t last_row;   // of the last pass started
+  };
+  // A warp's pass.
+  struct Task {
+    uint32_t slot, item, pass, passes, in_row, out_row;
+    bool last;
+  };
   struct Ctl {
-    uint32_t item;
-    uint32_t stop;         // 0, kStopRejected or kStopFailed
+    uint32_t lock;
+    uint32_t fail;       // a wait expired: every warp stops
+    uint32_t exhausted;  // the queue is empty
+    uint32_t num_open;
+    uint32_t free_rows;  // bits
+    uint32_t stop[W];    // per warp: its item is closed
+    Task task[W];        // per warp
+    Open open[W];
     uint32_t prog[kRows];  // per boundary row: (pass << 17) | last column published
   };
 
@@ -155,21 +188,202 @@ struct PipeForward {
     return (pass << 17) | col;
   }
 
-  __device__ __forceinline__ static bool stopped(Ctl& ctl) {
-    return __any_sync(kFullMask, *reinterpret_cast<volatile uint32_t*>(&ctl.stop) != 0u);
+  // Whether this warp has to leave its pass (its item is closed, or a wait
+  // expired), the same in every lane.
+  __device__ __forceinline__ static bool stopped(Ctl& ctl, int warp) {
+    return __any_sync(kFullMask, (*reinterpret_cast<volatile uint32_t*>(&ctl.stop[warp]) |
+                                  *reinterpret_cast<volatile uint32_t*>(&ctl.fail)) != 0u);
   }
 
-  // The whole warp waits until *word >= want; false (in every lane) when the
-  // item stopped meanwhile or the wait expired (which stops the item).
-  __device__ static bool wait_word(Ctl& ctl, const uint32_t* word, uint32_t want, uint32_t* err,
-                                   uint32_t polls) {
+  // The block's lock, taken by one lane; false if it was not to be had (which
+  // stops the block).
+  __device__ static bool lock(Ctl& ctl, uint32_t* err) {
+    for (uint32_t k = 0; atomicCAS(&ctl.lock, 0u, 1u) != 0u; ++k) {
+      if (k >= kLockPolls) {
+        atomicOr(err, kErrWaitTimeout);
+        atomicExch(&ctl.fail, 1u);
+        return false;
+      }
+      __nanosleep(32);
+    }
+    __threadfence_block();
+    return true;
+  }
+  __device__ static void unlock(Ctl& ctl) {
+    __threadfence_block();
+    atomicExch(&ctl.lock, 0u);
+  }
+
+  // Opens the queue's next valid item in a free slot; its slot, or -1 if the
+  // queue is empty.  Under the lock.
+  __device__ static int open_item(const BatchView& b, const ClassLaunch& c, uint32_t n, Ctl& ctl) {
+    int slot = -1;
+    for (int k = 0; k < W; ++k)
+      if (ctl.open[k].state == kFree) slot = k;
+    while (slot >= 0 && !ctl.exhausted) {
+      const uint32_t item = atomicAdd(c.counter, 1u);
+      if (item >= n) {
+        ctl.exhausted = 1u;
+        break;
+      }
+      PairRef refs[2];
+      F::load_refs(c, item, refs);
+      // an FP64 list position that no rescue filled (kLaunchRescueByItem lists)
+      if (P::kSlots == 1 && refs[0].read == kNoPair) continue;
+      if (refs[1].read == kNoPair) refs[1] = refs[0];
+      const HapDesc hx = b.haps[refs[0].hap], hy = b.haps[refs[1].hap];
+      const uint32_t lx = b.reads[refs[0].read].len, ly = b.reads[refs[1].read].len;
+      // slot x has the longer haplotype
+      if (hx.len == 0 || hy.len == 0 || lx == 0 || ly == 0 ||
+          (F::kSameHap && hx.code_off != hy.code_off) || hy.len > hx.len ||
+          (uint64_t)hx.len + kPad + 8 > c.scratch_cols) {
+        atomicOr(c.error_flags, kErrBadLength);
+        continue;
+      }
+      ctl.open[slot] = Open{kOpen, item, pipe_passes(lx > ly ? lx : ly, R), 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      ++ctl.num_open;
+      return slot;
+    }
+    return -1;
+  }
+
+  // The next pass for this warp, in ctl.task[warp]; false (in every lane) when
+  // there is none.  max_open: the block's even share of the queue.
+  __device__ static bool acquire(const BatchView& b, const ClassLaunch& c, uint32_t n,
+                                 uint32_t max_open, int warp, int lane, Ctl& ctl) {
+    int got = 0;  // 1: a pass, 0: none left, -1: none now
+    for (uint32_t tries = 0;; ++tries) {
+      if (lane == 0) got = try_acquire(b, c, n, max_open, warp, ctl);
+      got = __shfl_sync(kFullMask, got, 0);
+      __syncwarp();  // ctl.task[warp] is visible to the whole warp
+      if (got >= 0) return got != 0;
+      if (tries >= kLockPolls) {
+        if (lane == 0) {
+          atomicOr(c.error_flags, kErrWaitTimeout);
+          atomicExch(&ctl.fail, 1u);
+        }
+        return false;
+      }
+      __nanosleep(200);
+    }
+  }
+
+  // One try, by one lane: 1, 0 (no pass is left to start) or -1 (every row or
+  // slot is held by items that are being closed: their last passes end within a
+  // chunk).
+  __device__ static int try_acquire(const BatchView& b, const ClassLaunch& c, uint32_t n,
+                                    uint32_t max_open, int warp, Ctl& ctl) {
+    if (!lock(ctl, c.error_flags)) return 0;
+    auto oldest = [&](uint32_t window) {
+      int best = -1;
+      for (int k = 0; k < W; ++k) {
+        const Open& o = ctl.open[k];
+        if (o.state == kOpen && o.next < o.passes && o.next - o.done < window &&
+            (best < 0 || o.item < ctl.open[best].item))
+          best = k;
+      }
+      return best;
+    };
+    int k = -1, got = 0;
+    if (!ctl.fail) {
+      k = oldest(kWindow);
+      if (k < 0 && ctl.num_open < max_open) k = open_item(b, c, n, ctl);
+      if (k < 0) k = oldest(~0u);
+      if (k < 0) k = open_item(b, c, n, ctl);
+      if (k < 0 && !ctl.exhausted) got = -1;
+    }
+    if (k >= 0) {
+      Open& o = ctl.open[k];
+      Task t;
+      t.slot = (uint32_t)k;
+      t.item = o.item;
+      t.pass = o.next;
+      t.passes = o.passes;
+      t.last = t.pass + 1 == o.passes;
+      t.in_row = o.last_row;
+      t.out_row = 0;
+      if (!t.last && ctl.free_rows == 0u) {
+        got = -1;
+      } else {
+        if (!t.last) {
+          t.out_row = (uint32_t)__ffs((int)ctl.free_rows) - 1u;
+          ctl.free_rows &= ~(1u << t.out_row);
+          ctl.prog[t.out_row] = 0u;
+          o.rows |= 1u << t.out_row;
+          o.last_row = t.out_row;
+        }
+        ++o.next;
+        ++o.running;
+        ctl.stop[warp] = 0u;
+        ctl.task[warp] = t;
+        got = 1;
+      }
+    }
+    unlock(ctl);
+    return got;
+  }
+
+  // Closes this warp's item, if it is still open, and stops the other warps on
+  // it; whether this warp closed it (the same in every lane): it then writes the
+  // item's results or rescues.
+  __device__ static bool close(const ClassLaunch& c, int warp, int lane, Ctl& ctl) {
+    bool won = false;
+    if (lane == 0 && lock(ctl, c.error_flags)) {
+      const uint32_t slot = ctl.task[warp].slot;
+      if (ctl.open[slot].state == kOpen && !ctl.stop[warp] && !ctl.fail) {
+        ctl.open[slot].state = kClosed;
+        for (int w = 0; w < W; ++w)
+          if (w != warp && ctl.task[w].slot == slot) ctl.stop[w] = 1u;
+        won = true;
+      }
+      unlock(ctl);
+    }
+    return __shfl_sync(kFullMask, (int)won, 0) != 0;
+  }
+
+  // The end of this warp's pass; swept: to its last column.
+  __device__ static void release(const ClassLaunch& c, int warp, int lane, Ctl& ctl, bool swept) {
+    __syncwarp();
+    if (lane == 0 && lock(ctl, c.error_flags)) {
+      const Task t = ctl.task[warp];
+      Open& o = ctl.open[t.slot];
+      auto give_back = [&](uint32_t bits) {
+        o.rows &= ~bits;
+        o.wrote &= ~bits;
+        o.read &= ~bits;
+        ctl.free_rows |= bits;
+      };
+      --o.running;
+      if (swept) {
+        // a row is free once its writer has ended (it may still be summing the
+        // row) and its reader has read it all
+        if (t.pass > 0) o.read |= 1u << t.in_row;
+        if (!t.last) o.wrote |= 1u << t.out_row;
+        give_back(o.read & o.wrote);
+        o.done = o.done > t.pass + 1 ? o.done : t.pass + 1;
+      }
+      if (o.state == kClosed && o.running == 0) {
+        give_back(o.rows);
+        o.state = kFree;
+        --ctl.num_open;
+      }
+      ctl.task[warp].slot = W;  // none
+      unlock(ctl);
+    }
+    __syncwarp();
+  }
+
+  // The whole warp waits until *word >= want; false (in every lane) when its
+  // item was closed meanwhile or the wait expired (which stops the block).
+  __device__ static bool wait_word(Ctl& ctl, int warp, const uint32_t* word, uint32_t want,
+                                   uint32_t* err, uint32_t polls) {
     for (uint32_t k = 0;; ++k) {
       if (__all_sync(kFullMask, ld_acquire_cta(word) >= want)) return true;
-      if (stopped(ctl)) return false;
+      if (stopped(ctl, warp)) return false;
       if (k >= polls) {
         if ((threadIdx.x & (kWarp - 1)) == 0) {
           atomicOr(err, kErrWaitTimeout);
-          atomicExch(&ctl.stop, kStopFailed);
+          atomicExch(&ctl.fail, 1u);
         }
         __syncwarp();
         return false;
@@ -220,26 +434,14 @@ struct PipeForward {
     }
   }
 
-  // What the warp of the item's last pass keeps for the commit.
-  struct Sums {
-    V acc;          // column sum of the I of the last row (a pass-through row)
-    S frozen;       // slot y's sum at its own last column (two-haplotype items)
-    uint32_t passes;
-    bool ok;        // the item's descriptors were valid
-  };
-
-  // This warp's passes of work item `item`.
-  __device__ static Sums run(const BatchView& b, const ClassLaunch& c, uint32_t item, int warp,
-                             int lane, uint4* table, Ctl& ctl, Cell* rows) {
-    Sums out;
-    out.acc = P::zero();
-    out.frozen = 0;
-    out.passes = 0;
-    out.ok = false;
+  // Sweeps this warp's pass (ctl.task[warp]) and, as the warp that ends or
+  // rejects its item, writes the item's results or rescues.
+  __device__ static void run(const BatchView& b, const ClassLaunch& c, int warp, int lane,
+                             uint4* table, Ctl& ctl, Cell* rows) {
+    const uint32_t item = ctl.task[warp].item;
+    const uint32_t p = ctl.task[warp].pass;
     PairRef refs[2];
     F::load_refs(c, item, refs);
-    // an FP64 list position that no rescue filled (kLaunchRescueByItem lists)
-    if (P::kSlots == 1 && refs[0].read == kNoPair) return out;
     SlotInfo sl[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
@@ -252,16 +454,6 @@ struct PipeForward {
       sl[s].L = rd.len;
       sl[s].row_off = rd.row_off;
     }
-    const uint32_t Lmax = sl[0].L > sl[1].L ? sl[0].L : sl[1].L;
-    if (sl[0].H == 0 || sl[1].H == 0 || sl[0].L == 0 || sl[1].L == 0 ||
-        (F::kSameHap && sl[0].hap != sl[1].hap) || sl[1].H > sl[0].H ||
-        (uint64_t)sl[0].H + kPad + 8 > c.scratch_cols) {
-      if (warp == 0 && lane == 0) atomicOr(c.error_flags, kErrBadLength);
-      return out;
-    }
-    out.ok = true;
-    const uint32_t passes = pipe_passes(Lmax, R);
-    out.passes = passes;
     const uint32_t H = sl[0].H;
     const int nsteps = (int)H + kLag * (kWarp - 1);  // slot x has the longer haplotype
     // slot y's last accumulated step + 1
@@ -273,12 +465,13 @@ struct PipeForward {
     const uint32_t polls = c.wait_polls ? c.wait_polls : kWaitPolls;
     const bool publish = (c.flags & kLaunchNoPublish) == 0;
 
-    for (uint32_t p = (uint32_t)warp; p < passes; p += W) {
-      if (stopped(ctl)) break;
-      const bool last = p + 1 == passes;
-      const bool store = !last && lane == kWarp - 1;
-      const int out_row = (int)(p % kRows);
-      const int in_row = (int)((p + kRows - 1) % kRows);
+    V acc = P::zero();  // column sum of the I of the last row
+    S frozen = 0;       // slot y's, at its own last column (two-haplotype items)
+    bool alive = true;
+    {
+      const bool store = !ctl.task[warp].last && lane == kWarp - 1;
+      const int out_row = (int)ctl.task[warp].out_row;
+      const int in_row = (int)ctl.task[warp].in_row;
       Cell* const out_cells = rows + (size_t)out_row * c.scratch_cols + kPad;  // column 0
       // lane 31's step s holds column s - 31 kLag + 1 after the step
       constexpr int kLastCol = kLag * (kWarp - 1) - 1;
@@ -290,7 +483,7 @@ struct PipeForward {
         const uint32_t first = (uint32_t)k * kWarp + 1u;
         if (first <= H) {
           const uint32_t upto = first + kWarp - 1 < H ? first + kWarp - 1 : H;
-          if (!wait_word(ctl, &ctl.prog[in_row], enc(p - 1, upto), c.error_flags, polls))
+          if (!wait_word(ctl, warp, &ctl.prog[in_row], enc(p - 1, upto), c.error_flags, polls))
             return false;
         }
         const uint32_t idx = first + (uint32_t)lane;
@@ -316,7 +509,6 @@ struct PipeForward {
 #pragma unroll
       for (int k = 0; k < R; ++k) M[k] = I[k] = D[k] = P::zero();
       const bool from_ring = p > 0;
-      bool alive = true;
       if (from_ring) {
         alive = fetch_chunk(0);
       } else {
@@ -335,8 +527,6 @@ struct PipeForward {
       uint32_t cy_next = F::kSameHap ? 0u : (uint32_t)sl[1].hap[-kLag * lane];
       const uint8_t* hx = sl[0].hap - kLag * lane + 1;  // code of the step after s: hx[s]
       const uint8_t* hy = sl[1].hap - kLag * lane + 1;
-      V acc = P::zero();
-      S frozen = 0;
       // two-value form: this lane's hand-over for the lane below, and the M
       // term of its first row carried to the next column
       V h_t = P::zero(), h_i = P::zero();
@@ -391,6 +581,10 @@ struct PipeForward {
 
       const int nchunks = (nsteps + kWarp - 1) / kWarp;
       for (int k = 0; k < nchunks; ++k) {
+        if (stopped(ctl, warp)) {
+          alive = false;
+          break;
+        }
         if (from_ring) {
           cp_async_wait_all();  // this chunk's cells
           __syncwarp();
@@ -398,9 +592,6 @@ struct PipeForward {
             alive = false;
             break;
           }
-        } else if (stopped(ctl)) {
-          alive = false;
-          break;
         }
         const Cell* rc = ring + (k & 1) * kWarp;
         cell_next = rc[0];
@@ -433,54 +624,48 @@ struct PipeForward {
         cp_async_wait_all();  // the prefetch past the last step lands before the ring is reused
         __syncwarp();
       }
-      if (!alive) break;
-      if (last) {
-        out.acc = acc;
-        out.frozen = frozen;
+    }
+    if (alive) {
+      if (ctl.task[warp].last) {
+        if (close(c, warp, lane, ctl) && lane == kWarp - 1)
+          results(b, c, item, ctl.task[warp].passes, acc, frozen);
       } else if constexpr (P::kSlots == 2) {
         __syncwarp();  // lane 31's row stores are visible to the whole warp
         const uint32_t Hs[2] = {sl[0].H, sl[1].H};
-        if (rejects(b, c, out_cells, Hs, L, (p + 1) * (kWarp * R) - 1, lane, item)) {
-          if (lane == 0) atomicCAS(&ctl.stop, 0u, kStopRejected);
-          break;
+        const Cell* out_cells = rows + (size_t)ctl.task[warp].out_row * c.scratch_cols + kPad;
+        if (rejects(b, c, out_cells, Hs, L, (p + 1) * (kWarp * R) - 1, lane, item) &&
+            close(c, warp, lane, ctl) && lane == 0) {
+          F::load_refs(c, item, refs);
+          const uint32_t pos = c.rescue_base + 2u * item;  // kLaunchRescueByItem positions
+          F::finish(b, c, refs[0], 0.0, (double)kMinAcceptedF, pos);
+          if (refs[1].read != kNoPair)
+            F::finish(b, c, refs[1], 0.0, (double)kMinAcceptedF, pos + 1);
         }
       }
     }
-    return out;
+    release(c, warp, lane, ctl, alive);
   }
 
-  // After the block barrier that ends the item: the results, or the FP64
-  // rescue of a rejected item.
-  __device__ static void commit(const BatchView& b, const ClassLaunch& c, uint32_t item,
-                                int warp, int lane, const Ctl& ctl, const Sums& sm) {
-    if (!sm.ok) return;
-    const uint32_t stop = ctl.stop;
-    if (stop == kStopFailed) return;  // the error flag is set
+  // The results of an item from the sums of its last pass (one lane).
+  __device__ static void results(const BatchView& b, const ClassLaunch& c, uint32_t item,
+                                 uint32_t passes, V acc, S frozen) {
     PairRef fr[2];
     F::load_refs(c, item, fr);
     const bool valid_y = P::kSlots == 2 && fr[1].read != kNoPair;
     const uint32_t pos = c.rescue_base + 2u * item;  // kLaunchRescueByItem positions
-    if (stop == kStopRejected) {
-      if (warp == 0 && lane == 0) {
-        F::finish(b, c, fr[0], 0.0, (double)kMinAcceptedF, pos);
-        if (valid_y) F::finish(b, c, fr[1], 0.0, (double)kMinAcceptedF, pos + 1);
-      }
-      return;
-    }
-    if (warp != (int)((sm.passes - 1) % W) || lane != kWarp - 1) return;
     // both slots of a same-haplotype item ran exactly their own columns
-    const S fy = (P::kSlots == 2 && F::kSameHap) ? P::sy(sm.acc) : sm.frozen;
+    const S fy = (P::kSlots == 2 && F::kSameHap) ? P::sy(acc) : frozen;
     const uint32_t Lx = b.reads[fr[0].read].len;
     const uint32_t Ly = valid_y ? b.reads[fr[1].read].len : 0u;
-    const uint32_t rows = sm.passes * kWarp * R;
+    const uint32_t rows = passes * kWarp * R;
     double res[2] = {0.0, 0.0};
     double amin[2] = {(double)kMinAcceptedF, (double)kMinAcceptedF};
     if (F::kScaled) {
-      res[0] = F::scaled_result(b, c.gaps, fr[0].read, Lx, rows, S(0), P::sx(sm.acc), &amin[0]);
+      res[0] = F::scaled_result(b, c.gaps, fr[0].read, Lx, rows, S(0), P::sx(acc), &amin[0]);
       if (valid_y) res[1] = F::scaled_result(b, c.gaps, fr[1].read, Ly, rows, S(0), fy, &amin[1]);
     } else {
       // the pass-through row holds M_L + I_L in its I (non-uniform form)
-      res[0] = P::sx(sm.acc);
+      res[0] = P::sx(acc);
       res[1] = fy;
     }
     F::finish(b, c, fr[0], res[0], amin[0], pos);
@@ -488,8 +673,8 @@ struct PipeForward {
   }
 };
 
-// One work item per block at a time; c.scratch holds kRows boundary rows of
-// c.scratch_cols cells for every block of the grid.
+// c.scratch holds kRows boundary rows of c.scratch_cols cells for every block of
+// the grid.
 template <class P, int R, int GAPS, bool SAME, int MINB, int W>
 __global__ void __launch_bounds__(W * kWarp, MINB)
     forward_pipe_kernel(BatchView b, ClassLaunch c) {
@@ -502,21 +687,18 @@ __global__ void __launch_bounds__(W * kWarp, MINB)
   typename F::Cell* rows = reinterpret_cast<typename F::Cell*>(c.scratch) +
                            (size_t)blockIdx.x * F::kRows * c.scratch_cols;
   const uint32_t n = c.work_count ? *c.work_count : c.static_count;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      ctl.item = atomicAdd(c.counter, 1u);
-      ctl.stop = 0;
-#pragma unroll
-      for (int k = 0; k < F::kRows; ++k) ctl.prog[k] = 0;
+  const uint32_t max_open = (n + gridDim.x - 1) / gridDim.x;
+  if (threadIdx.x == 0) {
+    ctl.lock = ctl.fail = ctl.exhausted = ctl.num_open = 0u;
+    ctl.free_rows = (1u << F::kRows) - 1u;
+    for (int w = 0; w < W; ++w) {
+      ctl.stop[w] = 0u;
+      ctl.task[w].slot = W;
+      ctl.open[w].state = F::kFree;
     }
-    __syncthreads();
-    const uint32_t item = ctl.item;
-    if (item >= n) break;
-    const typename F::Sums sm = F::run(b, c, item, warp, lane, table, ctl, rows);
-    __syncthreads();
-    F::commit(b, c, item, warp, lane, ctl, sm);
-    __syncthreads();  // ctl is reset for the next item
   }
+  __syncthreads();
+  while (F::acquire(b, c, n, max_open, warp, lane, ctl)) F::run(b, c, warp, lane, table, ctl, rows);
 }
 
 }  // namespace rodv
