@@ -369,11 +369,14 @@ rodv_status Engine::load_kernels() {
 // rows of the largest grid any of its variants launches (the autotuner runs
 // every variant on its batches).
 size_t Engine::multi_scratch_bytes(bool uniform, size_t cols) const {
-  size_t rows = 0;
-  for_each_kernel([&](const KernelInfo& k) {
-    if (k.multi && k.uniform == uniform)
-      rows = std::max(rows, (size_t)persistent_blocks(k) * k.boundary_rows);
-  });
+  size_t rows = multi_rows_[uniform].load();
+  if (!rows) {
+    for_each_kernel([&](const KernelInfo& k) {
+      if (k.multi && k.uniform == uniform)
+        rows = std::max(rows, (size_t)persistent_blocks(k) * k.boundary_rows);
+    });
+    multi_rows_[uniform].store(rows);
+  }
   return align_up(rows * cols * (uniform ? 16 : 24));
 }
 
@@ -1033,8 +1036,19 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
 // ---------------------------------------------------------------------------
 // Launches
 // ---------------------------------------------------------------------------
+namespace {
+// Grid of a multi-pass launch of `items` items, at most `blocks` resident: up to
+// three items a block, every block gets as many (540 pairs of reads of 850 x
+// 4,300 bases: 1.68 ms on 444 blocks, 1.38 on 270 of two items each).
+int even_blocks(int blocks, int items) {
+  const int rounds = (items + blocks - 1) / blocks;
+  return rounds > 1 && rounds <= 3 ? (items + rounds - 1) / rounds : blocks;
+}
+}  // namespace
+
 rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int c, bool same,
-                                      int variant, int blocks_cap, cudaStream_t stream) {
+                                      int variant, int blocks_cap, cudaStream_t stream,
+                                      size_t scratch_skip) {
   ArenaView a = arena_view(plan, dbase, tab_);
   const uint32_t n = same ? plan.same_items[c] : plan.diff_items[c];
   if (!n) return RODV_OK;
@@ -1051,6 +1065,7 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   cl.rescue_list = reinterpret_cast<PairRef*>(dbase + plan.off_lists[c]);
   cl.rescue_count = a.counts + kCtrRescue + c;
   cl.scratch = class_scratch(plan, a, c);
+  if (cl.scratch) cl.scratch += scratch_skip / sizeof(float);
   cl.scratch_cols = plan.scratch_cols;
   cl.error_flags = a.counts + kCtrError;
   cl.stack = reinterpret_cast<const uint32_t*>(dbase + plan.off_stack[c]);
@@ -1063,6 +1078,7 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   const int per_block = k.items_per_block;
   const int need = (int)((n + per_block - 1) / per_block);
   int blocks = std::max(1, std::min(persistent_blocks(k), need));
+  if (class_multi(c)) blocks = even_blocks(blocks, need);
   if (blocks_cap > 0) blocks = std::min(blocks, blocks_cap);
   void* args[] = {&a.view, &cl};
   RODV_CUDA(cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream));
@@ -1120,7 +1136,7 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
   cl.error_flags = a.counts + kCtrError;
   apply_wait_fault(cl, c);
   const int need = (int)((plan.pairs[c] + k.items_per_block - 1) / k.items_per_block);
-  const int blocks = std::max(1, std::min(persistent_blocks(k), need));
+  const int blocks = even_blocks(std::max(1, std::min(persistent_blocks(k), need)), need);
   void* args[] = {&a.view, &cl};
   RODV_CUDA(cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream));
   return RODV_OK;
@@ -1181,15 +1197,30 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
     // branch of their own: a handful of items behind the class's chains added
     // their whole sweep to a small batch (7 regions of per-row-gap reads: 131 us
     // on the device, 103 so).
-    // The multi-pass classes' two kinds share boundary rows and stay in
-    // sequence.
-    auto branch = [](int c, bool same) {
-      return same || class_multi(c) ? c : c + kNumClasses;
+    // So are the multi-pass classes' where the class's boundary rows hold both
+    // launches' (diff_skip: where the second one's start; else the two share
+    // rows and stay in sequence).
+    size_t diff_skip[kNumClasses] = {};
+    for (int c = kSinglePassClasses; c < kNumClasses; ++c) {
+      size_t bytes[2];
+      for (int same = 0; same < 2; ++same) {
+        const KernelInfo k = forward_kernel_info(Precision::kF32x2, class_rows(c),
+                                                 plan.gap_form(c), true, same, plan.variant[c]);
+        const uint32_t n = same ? plan.same_items[c] : plan.diff_items[c];
+        bytes[same] = (size_t)std::min<uint32_t>(n, persistent_blocks(k)) * k.boundary_rows *
+                      plan.scratch_cols * (class_uniform(c) ? 16 : 24);
+      }
+      if (bytes[0] && bytes[1] && bytes[0] + bytes[1] <= plan.scratch_bytes[class_uniform(c)])
+        diff_skip[c] = bytes[1];
+    }
+    auto branch = [&](int c, bool same) {
+      return same || (class_multi(c) && !diff_skip[c]) ? c : c + kNumClasses;
     };
     int branches = 0;
     for (int c = 0; c < kNumClasses; ++c)
-      branches += class_multi(c) ? plan.same_items[c] + plan.diff_items[c] > 0
-                                 : (plan.same_items[c] > 0) + (plan.diff_items[c] > 0);
+      branches += class_multi(c) && !diff_skip[c]
+                      ? plan.same_items[c] + plan.diff_items[c] > 0
+                      : (plan.same_items[c] > 0) + (plan.diff_items[c] > 0);
     RODV_CUDA(fork(branches));
     // the longest reads first: the short items of the small classes fill the
     // tail (300 regions of 1-300 reads x 1-32 haplotypes: 7.5 ms shortest
@@ -1199,7 +1230,8 @@ rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stat
         if (!(same ? plan.same_items[c] : plan.diff_items[c])) continue;
         const cudaStream_t ls = lane(branch(c, same != 0));
         if (!ls) return cuda_fail(cudaErrorUnknown, "class stream fork");
-        rodv_status s = launch_fp32_class(plan, dbase, c, same != 0, plan.variant[c], 0, ls);
+        rodv_status s = launch_fp32_class(plan, dbase, c, same != 0, plan.variant[c], 0, ls,
+                                          same ? 0 : diff_skip[c]);
         if (s != RODV_OK) return s;
         ++launches;
       }
@@ -1441,7 +1473,10 @@ rodv_status Engine::run_host_chunked(const rodv_batch& b, double* out, rodv_stat
     // the range's classes as parallel branches (their tails overlap; 130 ms
     // per call of the uneven batch against 132-134 without)
     result = launch_all(p, d, &acc, l.stream, l.ev, 3, /*fan_out=*/true);
-    if (result != RODV_OK) break;
+    if (result != RODV_OK) {
+      cudaDeviceSynchronize();  // branches already launched
+      break;
+    }
     e = cudaMemcpyAsync(h, d + p.off_counts, ob, cudaMemcpyDeviceToHost, l.stream);
     if (e == cudaSuccess) e = cudaEventRecord(l.done, l.stream);
     if (e != cudaSuccess) {
@@ -1489,7 +1524,11 @@ rodv_status Engine::run_host_single(const rodv_batch& b, double* out, rodv_stats
   // of items per class, each launch far from filling the GPU (7 regions of
   // per-row-gap reads in 8 classes: 0.58 -> 0.26 ms)
   s = launch_all(plan, d, st, stream_, ev_, 3, /*fan_out=*/true);
-  if (s != RODV_OK) return s;
+  if (s != RODV_OK) {
+    // branches already launched still use the arena the next call writes
+    cudaDeviceSynchronize();
+    return s;
+  }
   uint8_t* hs = static_cast<uint8_t*>(out_staging_.ptr);
   // counters and results in one copy; the counters came with the upload (a
   // reset and a copy of their own cost a call of one pair 5 us of 80)

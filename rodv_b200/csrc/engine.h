@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -199,7 +200,8 @@ class Engine {
                          cudaStream_t stream, cudaEvent_t* ev, int parts,
                          bool fan_out = false, bool reset = false);
   rodv_status launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int cls, bool same,
-                                int variant, int blocks_cap, cudaStream_t stream);
+                                int variant, int blocks_cap, cudaStream_t stream,
+                                size_t scratch_skip = 0);
   rodv_status launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int cls, int variant,
                                 cudaStream_t stream);
   rodv_status launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform,
@@ -217,6 +219,8 @@ class Engine {
   bool save_tuning(const std::string& path) const;
 
   rodv_options opt_;
+  // boundary rows of the multi-pass kernels (per-row, uniform; 0: not counted yet)
+  mutable std::atomic<size_t> multi_rows_[2] = {};
   mutable std::mutex occ_mu_;
   mutable std::unordered_map<const void*, int> occ_cache_;  // kernel -> resident blocks
   int device_ = 0;
