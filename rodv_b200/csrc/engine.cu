@@ -131,6 +131,9 @@ void for_each_kernel(const Fn& fn) {
         const int nv = forward_kernel_variants(pr, p == 0, class_rows(c), class_multi(c));
         for (int v = 0; v < nv; ++v)
           fn(forward_kernel_info(pr, class_rows(c), gaps, class_multi(c), p == 0, v));
+        if (class_multi(c) && pipe_has_few(pr, class_uniform(c)))
+          for (int v = 0; v < nv; ++v)
+            fn(forward_kernel_info(pr, class_rows(c), gaps, true, p == 0, v | kPipeFew));
       }
 }
 
@@ -1054,9 +1057,9 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   if (!n) return RODV_OK;
   // the multi-pass two-haplotype kernel shares the class's variant (strip
   // height), which the packer paired its items by
-  const KernelInfo k = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c),
-                                           class_multi(c), same,
-                                           (same || class_multi(c)) ? variant : 0);
+  KernelInfo k = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c),
+                                     class_multi(c), same,
+                                     (same || class_multi(c)) ? variant : 0);
   ClassLaunch cl{};
   cl.work = dbase + (same ? plan.off_same[c] : plan.off_diff[c]);
   cl.work_count = nullptr;
@@ -1078,7 +1081,20 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   const int per_block = k.items_per_block;
   const int need = (int)((n + per_block - 1) / per_block);
   int blocks = std::max(1, std::min(persistent_blocks(k), need));
-  if (class_multi(c)) blocks = even_blocks(blocks, need);
+  if (class_multi(c)) {
+    blocks = even_blocks(blocks, need);
+    // A grid that fits at 8 warps per SM takes the kernel built for those: its
+    // items' sweeps are shorter (pairs of reads of about 1,500 x 4,350 bases, 18
+    // items 1.08 -> 1.04 ms, 540 in 270 blocks 2.70 -> 2.59).  Above that, the
+    // resident warps count for more (2,160 such items 7.78 ms at 12 warps per SM,
+    // 8.64 at 8).
+    if (pipe_has_few(Precision::kF32x2, class_uniform(c))) {
+      const KernelInfo few = forward_kernel_info(Precision::kF32x2, class_rows(c),
+                                                 plan.gap_form(c), true, same,
+                                                 variant | kPipeFew);
+      if (blocks <= persistent_blocks(few)) k = few;
+    }
+  }
   if (blocks_cap > 0) blocks = std::min(blocks, blocks_cap);
   void* args[] = {&a.view, &cl};
   RODV_CUDA(cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream));

@@ -33,11 +33,11 @@ KernelInfo make_info(int variant) {
 }
 
 // Multi-pass kernels: the passes of one item on the W warps of a block.
-template <class P, int R, int GAPS, bool SAME, int W>
+template <class P, int R, int GAPS, bool SAME, int W, int WARPS = 12>
 KernelInfo make_pipe_info(int variant) {
-  // 168 registers (12 warps per SM) in the scaled form; per-row kernels keep
-  // five coefficients a row
-  constexpr int kMinBlocks = GAPS == kGapsPerRow ? 1 : 12 / W;
+  // 168 registers (12 warps per SM) in the scaled form, 8 warps for launches
+  // of few blocks; per-row kernels keep five coefficients a row
+  constexpr int kMinBlocks = GAPS == kGapsPerRow ? 1 : WARPS / W;
   using F = PipeForward<P, R, GAPS, SAME, kMinBlocks, W>;
   KernelInfo k;
   k.fn = reinterpret_cast<const void*>(&forward_pipe_kernel<P, R, GAPS, SAME, kMinBlocks, W>);
@@ -81,6 +81,15 @@ KernelInfo pipe_gap_info(Precision prec, bool same, int variant) {
   if (prec == Precision::kF64)
     return w4 ? make_pipe_info<F64, R, GAPS, false, 4>(variant)
               : make_pipe_info<F64, R, GAPS, false, 2>(variant);
+  if constexpr (GAPS != kGapsPerRow) {
+    if (variant & kPipeFew) {
+      if (same)
+        return w4 ? make_pipe_info<F32x2, R, GAPS, true, 4, 8>(variant)
+                  : make_pipe_info<F32x2, R, GAPS, true, 2, 8>(variant);
+      return w4 ? make_pipe_info<F32x2, R, GAPS, false, 4, 8>(variant)
+                : make_pipe_info<F32x2, R, GAPS, false, 2, 8>(variant);
+    }
+  }
   if (same)
     return w4 ? make_pipe_info<F32x2, R, GAPS, true, 4>(variant)
               : make_pipe_info<F32x2, R, GAPS, true, 2>(variant);

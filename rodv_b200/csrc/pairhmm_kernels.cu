@@ -18,7 +18,7 @@ KernelInfo pipe_info_for(Precision prec, GapForm gaps, bool same, int variant);
 KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, GapForm gaps, bool multi,
                                bool same, int variant) {
   if (multi) {
-    const int v = variant >= 0 && variant < kPipeVariants ? variant : 0;
+    const int v = variant >= 0 && variant < kPipeVariants + kPipeFew ? variant : 0;
     return pipe_variant_rows(v) == 4 ? pipe_info_for<4>(prec, gaps, same, v)
                                      : pipe_info_for<8>(prec, gaps, same, v);
   }

@@ -153,7 +153,11 @@ struct PipeForward {
   // steps 6.46 and 11.3, sixteen 6.34 and 11.5); at 128 registers and 16 warps,
   // with spills, 6.80 and 11.2 (four steps 6.78 and 12.1), and a lone item takes
   // 0.92 and 0.78 ms instead of 0.81 and 0.72.
-  static constexpr int kUnroll = 8;
+  // The kernels for few blocks (FP32, 8 warps per SM) take four: a lone item of
+  // two reads of 850 (1,500) x 4,300 bases 0.458 (0.875) ms, with eight 0.477
+  // (0.908), at 12 warps 0.489 (0.932), four steps at 12 warps 0.483 (0.921).
+  static constexpr bool kFew = P::kSlots == 2 && kTwo && MINB * W <= 8;
+  static constexpr int kUnroll = kFew ? 4 : 8;
   static constexpr int kSmemPerWarp = F::kSmemPerWarp;  // emission table + cell ring
   // polls of a progress word (about 100 ns each) before a wait gives up
   static constexpr uint32_t kWaitPolls = 1u << 24;
