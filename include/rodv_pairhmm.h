@@ -373,6 +373,9 @@ rodv_status rodv_fault_inject_alloc(int32_t kind, int64_t nth);
  * returns, and the call fails with RODV_ERR_DEVICE_CHECK.  Tests the expiry
  * path with no hang and no fault; the device stays usable. */
 rodv_status rodv_fault_inject_wait(int32_t enable);
+/* The nth next forward-kernel launch is not made and reports an error (0
+ * disarms it): the call fails with RODV_ERR_CUDA. */
+rodv_status rodv_fault_inject_launch(int64_t nth);
 void rodv_debug_live_allocations(uint64_t* device, uint64_t* pinned_host);
 /* The chain items the packer makes of one region's reads, on the host only
  * (no device call; for tests of the placement rules).  Reads 0..num_reads-1

@@ -231,6 +231,11 @@ rodv_status rodv_fault_inject_wait(int32_t enable) {
   return RODV_OK;
 }
 
+rodv_status rodv_fault_inject_launch(int64_t nth) {
+  rodv::set_launch_fault(nth);
+  return RODV_OK;
+}
+
 void rodv_debug_live_allocations(uint64_t* device, uint64_t* pinned_host) {
   rodv::live_allocations(device, pinned_host);
 }

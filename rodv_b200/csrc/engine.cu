@@ -193,6 +193,22 @@ void apply_wait_fault(ClassLaunch& cl, int cls) {
 }
 }  // namespace
 void set_wait_fault(bool on) { g_wait_fault.store(on); }
+
+// Testing hook (rodv_fault_inject_launch): the n-th next forward kernel is not
+// launched, and the launch returns an error.
+namespace {
+std::atomic<int64_t> g_launch_countdown{0};
+}  // namespace
+void set_launch_fault(int64_t nth) { g_launch_countdown.store(nth > 0 ? nth : 0); }
+static cudaError_t launch_kernel(const KernelInfo& k, int blocks, void** args, cudaStream_t stream) {
+  int64_t v = g_launch_countdown.load();
+  while (v > 0)
+    if (g_launch_countdown.compare_exchange_weak(v, v - 1)) {
+      if (v == 1) return cudaErrorLaunchOutOfResources;
+      break;
+    }
+  return cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream);
+}
 void live_allocations(uint64_t* device, uint64_t* pinned) {
   if (device) *device = (uint64_t)g_live[0].load();
   if (pinned) *pinned = (uint64_t)g_live[1].load();
@@ -1097,7 +1113,7 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   }
   if (blocks_cap > 0) blocks = std::min(blocks, blocks_cap);
   void* args[] = {&a.view, &cl};
-  RODV_CUDA(cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream));
+  RODV_CUDA(launch_kernel(k, blocks, args, stream));
   return RODV_OK;
 }
 
@@ -1125,7 +1141,7 @@ rodv_status Engine::launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool u
   const uint64_t need = (pairs + k.items_per_block - 1) / k.items_per_block;
   const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(persistent_blocks(k), need));
   void* args[] = {&a.view, &r};
-  RODV_CUDA(cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream));
+  RODV_CUDA(launch_kernel(k, blocks, args, stream));
   return RODV_OK;
 }
 
@@ -1154,13 +1170,29 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
   const int need = (int)((plan.pairs[c] + k.items_per_block - 1) / k.items_per_block);
   const int blocks = even_blocks(std::max(1, std::min(persistent_blocks(k), need)), need);
   void* args[] = {&a.view, &cl};
-  RODV_CUDA(cudaLaunchKernel(k.fn, dim3(blocks), dim3(k.threads), args, k.smem_bytes, stream));
+  RODV_CUDA(launch_kernel(k, blocks, args, stream));
   return RODV_OK;
 }
 
 rodv_status Engine::launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stats* st,
                                cudaStream_t stream, cudaEvent_t* ev, int parts, bool fan_out,
                                bool reset) {
+  const rodv_status s = launch_parts(plan, dbase, st, stream, ev, parts, fan_out, reset);
+  if (s == RODV_OK) return s;
+  // What was launched before the failure runs on, on branches that were not
+  // joined, and writes the arena that the caller uploads its next batch into.
+  // (A captured launch runs nothing.)
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    for (cudaStream_t side : side_) cudaStreamSynchronize(side);
+    cudaStreamSynchronize(stream);
+  }
+  return s;
+}
+
+rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_stats* st,
+                                 cudaStream_t stream, cudaEvent_t* ev, int parts, bool fan_out,
+                                 bool reset) {
   ArenaView a = arena_view(plan, dbase, tab_);
   uint32_t launches = 0;
   // fan-out: the first branch of a part stays on `stream`; the first launch of
@@ -1489,14 +1521,12 @@ rodv_status Engine::run_host_chunked(const rodv_batch& b, double* out, rodv_stat
     // the range's classes as parallel branches (their tails overlap; 130 ms
     // per call of the uneven batch against 132-134 without)
     result = launch_all(p, d, &acc, l.stream, l.ev, 3, /*fan_out=*/true);
-    if (result != RODV_OK) {
-      cudaDeviceSynchronize();  // branches already launched
-      break;
-    }
+    if (result != RODV_OK) break;
     e = cudaMemcpyAsync(h, d + p.off_counts, ob, cudaMemcpyDeviceToHost, l.stream);
     if (e == cudaSuccess) e = cudaEventRecord(l.done, l.stream);
     if (e != cudaSuccess) {
       result = cuda_fail(e, "chunk download");
+      cudaStreamSynchronize(l.stream);  // the range's kernels
       break;
     }
     l.out_off = out_off;
@@ -1540,11 +1570,7 @@ rodv_status Engine::run_host_single(const rodv_batch& b, double* out, rodv_stats
   // of items per class, each launch far from filling the GPU (7 regions of
   // per-row-gap reads in 8 classes: 0.58 -> 0.26 ms)
   s = launch_all(plan, d, st, stream_, ev_, 3, /*fan_out=*/true);
-  if (s != RODV_OK) {
-    // branches already launched still use the arena the next call writes
-    cudaDeviceSynchronize();
-    return s;
-  }
+  if (s != RODV_OK) return s;
   uint8_t* hs = static_cast<uint8_t*>(out_staging_.ptr);
   // counters and results in one copy; the counters came with the upload (a
   // reset and a copy of their own cost a call of one pair 5 us of 80)
@@ -1728,8 +1754,7 @@ rodv_status Engine::plain(rodv_device_batch* db, double* out, rodv_stats* st) {
           rl.count[class_rows(c) - 1] = reinterpret_cast<const uint32_t*>(w + 72);
           const bool rescue = f64 && !class_multi(c);
           void* args[] = {&a.view, rescue ? (void*)&rl : (void*)&cl};
-          RODV_CUDA(
-              cudaLaunchKernel(k.fn, dim3(1), dim3(k.threads), args, k.smem_bytes, stream_));
+          RODV_CUDA(launch_kernel(k, 1, args, stream_));
           ++launches;
           if (f64) break;
           RODV_CUDA(cudaMemcpyAsync(hc + 2, wc + 2, 8, cudaMemcpyDeviceToHost, stream_));

@@ -55,6 +55,7 @@ enum CounterBlock : int {
 // kind 0 = device (cudaMalloc), 1 = pinned host (cudaMallocHost).
 void set_alloc_fault(int kind, int64_t nth);
 void set_wait_fault(bool on);
+void set_launch_fault(int64_t nth);
 void live_allocations(uint64_t* device, uint64_t* pinned);
 
 struct DeviceMem {
@@ -195,10 +196,14 @@ class Engine {
   // side stream (forked from and joined back into `stream`), so that class
   // kernels fill each other's tails.  The side streams are the engine's: the
   // captured resident path, the host-buffer ranges and the service's batches
-  // use them from the one thread that launches for the engine at a time.
+  // use them from the one thread that launches for the engine at a time.  On
+  // failure nothing of the launch is left running.
   rodv_status launch_all(const PackedPlan& plan, uint8_t* dbase, rodv_stats* st,
                          cudaStream_t stream, cudaEvent_t* ev, int parts,
                          bool fan_out = false, bool reset = false);
+  rodv_status launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_stats* st,
+                           cudaStream_t stream, cudaEvent_t* ev, int parts, bool fan_out,
+                           bool reset);
   rodv_status launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int cls, bool same,
                                 int variant, int blocks_cap, cudaStream_t stream,
                                 size_t scratch_skip = 0);
