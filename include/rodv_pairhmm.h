@@ -371,7 +371,8 @@ rodv_status rodv_fault_inject_alloc(int32_t kind, int64_t nth);
  * another's progress, each wait bounded) run with progress publication off
  * and a short wait limit: every wait runs out, the kernel records it and
  * returns, and the call fails with RODV_ERR_DEVICE_CHECK.  Tests the expiry
- * path with no hang and no fault; the device stays usable. */
+ * path with no hang and no fault; the device stays usable.  enable = 2: the
+ * short limit alone, with which every launch still has to succeed. */
 rodv_status rodv_fault_inject_wait(int32_t enable);
 /* The nth next forward-kernel launch is not made and reports an error (0
  * disarms it): the call fails with RODV_ERR_CUDA. */

@@ -227,7 +227,7 @@ rodv_status rodv_fault_inject_alloc(int32_t kind, int64_t nth) {
 }
 
 rodv_status rodv_fault_inject_wait(int32_t enable) {
-  rodv::set_wait_fault(enable != 0);
+  rodv::set_wait_fault(enable == 2 ? 2 : enable != 0);
   return RODV_OK;
 }
 

@@ -181,18 +181,18 @@ bool injected_failure(int kind) {
 void set_alloc_fault(int kind, int64_t nth) { g_fail_countdown[kind].store(nth > 0 ? nth : 0); }
 
 // Testing hook (rodv_fault_inject_wait): multi-pass launches made while it is
-// set publish no progress and give up a wait after kTestWaitPolls polls.
+// set give up a wait after kTestWaitPolls polls, and (1) publish no progress.
 namespace {
-std::atomic<bool> g_wait_fault{false};
+std::atomic<int> g_wait_fault{0};
 constexpr uint32_t kTestWaitPolls = 1u << 12;
 void apply_wait_fault(ClassLaunch& cl, int cls) {
-  if (class_multi(cls) && g_wait_fault.load()) {
-    cl.flags |= kLaunchNoPublish;
-    cl.wait_polls = kTestWaitPolls;
-  }
+  const int fault = g_wait_fault.load();
+  if (!class_multi(cls) || !fault) return;
+  cl.wait_polls = kTestWaitPolls;
+  if (fault == 1) cl.flags |= kLaunchNoPublish;
 }
 }  // namespace
-void set_wait_fault(bool on) { g_wait_fault.store(on); }
+void set_wait_fault(int mode) { g_wait_fault.store(mode); }
 
 // Testing hook (rodv_fault_inject_launch): the n-th next forward kernel is not
 // launched, and the launch returns an error.

@@ -180,9 +180,11 @@ struct PipeForward {
     bool last;
   };
   struct Ctl {
-    uint32_t lock;
+    uint32_t ticket, serving;  // the lock: next ticket, the ticket that holds it
+    uint32_t broken;     // a warp gave up its ticket: the lock serves nobody any more
     uint32_t fail;       // a wait expired: every warp stops
     uint32_t started;    // the block's first item is taken
+    uint32_t scanning;   // a warp is taking the queue's next item
     uint32_t exhausted;  // the queue is empty
     uint32_t num_open;
     uint32_t free_rows;  // bits
@@ -204,11 +206,17 @@ struct PipeForward {
   }
 
   // The block's lock, taken by one lane; false if it was not to be had (which
-  // stops the block).
-  __device__ static bool lock(Ctl& ctl, uint32_t* err) {
-    for (uint32_t k = 0; atomicCAS(&ctl.lock, 0u, 1u) != 0u; ++k) {
-      if (k >= kLockPolls) {
-        atomicOr(err, kErrWaitTimeout);
+  // stops the block).  Tickets are served in order: with a test-and-set word,
+  // warps that look again and again (acquire) can keep one that ends its pass
+  // from ever finding the lock free, since their sleeps end in step.
+  __device__ static bool lock(Ctl& ctl, const ClassLaunch& c) {
+    const uint32_t polls = c.wait_polls ? c.wait_polls : kLockPolls;
+    const uint32_t mine = atomicAdd(&ctl.ticket, 1u);
+    for (uint32_t k = 0; *reinterpret_cast<volatile uint32_t*>(&ctl.serving) != mine; ++k) {
+      if (*reinterpret_cast<volatile uint32_t*>(&ctl.broken)) return false;
+      if (k >= polls) {
+        atomicOr(c.error_flags, kErrWaitTimeout);
+        atomicExch(&ctl.broken, 1u);
         atomicExch(&ctl.fail, 1u);
         return false;
       }
@@ -219,24 +227,22 @@ struct PipeForward {
   }
   __device__ static void unlock(Ctl& ctl) {
     __threadfence_block();
-    atomicExch(&ctl.lock, 0u);
+    atomicAdd(&ctl.serving, 1u);
   }
 
-  // Opens the queue's next valid item in a free slot; its slot, or -1 if the
-  // queue is empty.  Under the lock.
-  __device__ static int open_item(const BatchView& b, const ClassLaunch& c, uint32_t n, Ctl& ctl) {
-    int slot = -1;
-    for (int k = 0; k < W; ++k)
-      if (ctl.open[k].state == kFree) slot = k;
-    while (slot >= 0 && !ctl.exhausted) {
+  // Opens the queue's next valid item, or notes that the queue is empty, for the
+  // lane whose try_acquire returned kScan (and set ctl.scanning, so that no
+  // other opens one meanwhile).  The queue is read outside the lock: an FP64
+  // list of 1e8 positions that no rescue filled keeps a block looking for half
+  // a second.  False if the lock was not to be had.
+  __device__ static bool open_item(const BatchView& b, const ClassLaunch& c, uint32_t n, Ctl& ctl) {
+    uint32_t found = kNoPair, passes = 0;
+    for (;;) {
       // the block's first item is its own: another block that opens two at once
       // must not leave it without
       const uint32_t item = ctl.started ? gridDim.x + atomicAdd(c.counter, 1u) : blockIdx.x;
       ctl.started = 1u;
-      if (item >= n) {
-        ctl.exhausted = 1u;
-        break;
-      }
+      if (item >= n) break;
       PairRef refs[2];
       F::load_refs(c, item, refs);
       // an FP64 list position that no rescue filled (kLaunchRescueByItem lists)
@@ -251,24 +257,43 @@ struct PipeForward {
         atomicOr(c.error_flags, kErrBadLength);
         continue;
       }
-      ctl.open[slot] = Open{kOpen, item, pipe_passes(lx > ly ? lx : ly, R), 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-      ++ctl.num_open;
-      return slot;
+      found = item;
+      passes = pipe_passes(lx > ly ? lx : ly, R);
+      break;
     }
-    return -1;
+    if (!lock(ctl, c)) return false;
+    ctl.scanning = 0u;
+    if (found == kNoPair) {
+      ctl.exhausted = 1u;
+    } else {
+      int slot = 0;  // num_open < W when the scan began: one is free
+      while (slot < W - 1 && ctl.open[slot].state != kFree) ++slot;
+      ctl.open[slot] = Open{kOpen, found, passes, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      ++ctl.num_open;
+    }
+    unlock(ctl);
+    return true;
   }
 
   // The next pass for this warp, in ctl.task[warp]; false (in every lane) when
   // there is none.  max_open: the block's even share of the queue.
   __device__ static bool acquire(const BatchView& b, const ClassLaunch& c, uint32_t n,
                                  uint32_t max_open, int warp, int lane, Ctl& ctl) {
-    int got = 0;  // 1: a pass, 0: none left, -1: none now
+    int got = kNone;
     for (uint32_t tries = 0;; ++tries) {
-      if (lane == 0) got = try_acquire(b, c, n, max_open, warp, ctl);
+      if (lane == 0) {
+        while ((got = try_acquire(c, max_open, warp, ctl)) == kScan)
+          if (!open_item(b, c, n, ctl)) {
+            got = kNone;
+            break;
+          }
+        // a scan ends by itself, however long the list
+        if (*reinterpret_cast<volatile uint32_t*>(&ctl.scanning)) tries = 0;
+      }
       got = __shfl_sync(kFullMask, got, 0);
       __syncwarp();  // ctl.task[warp] is visible to the whole warp
-      if (got >= 0) return got != 0;
-      if (tries >= kLockPolls) {
+      if (got != kLater) return got == kPass;
+      if (__shfl_sync(kFullMask, tries, 0) >= kLockPolls) {
         if (lane == 0) {
           atomicOr(c.error_flags, kErrWaitTimeout);
           atomicExch(&ctl.fail, 1u);
@@ -279,12 +304,13 @@ struct PipeForward {
     }
   }
 
-  // One try, by one lane: 1, 0 (no pass is left to start) or -1 (every row or
-  // slot is held by items that are being closed: their last passes end within a
-  // chunk).
-  __device__ static int try_acquire(const BatchView& b, const ClassLaunch& c, uint32_t n,
-                                    uint32_t max_open, int warp, Ctl& ctl) {
-    if (!lock(ctl, c.error_flags)) return 0;
+  // One try, by one lane.  kNone: no pass is left to start.  kLater: another
+  // warp is taking an item off the queue, or every row or slot is held by items
+  // that are being closed (their last passes end within kStopChunks chunks).
+  // kScan: a new item is wanted, and this lane is to take it (open_item).
+  enum : int { kNone, kPass, kLater, kScan };
+  __device__ static int try_acquire(const ClassLaunch& c, uint32_t max_open, int warp, Ctl& ctl) {
+    if (!lock(ctl, c)) return kNone;
     auto oldest = [&](uint32_t window) {
       int best = -1;
       for (int k = 0; k < W; ++k) {
@@ -295,13 +321,17 @@ struct PipeForward {
       }
       return best;
     };
-    int k = -1, got = 0;
+    int k = -1, got = kNone;
     if (!ctl.fail) {
+      const bool can_open = !ctl.exhausted && !ctl.scanning && ctl.num_open < W;
       k = oldest(kWindow);
-      if (k < 0 && ctl.num_open < max_open) k = open_item(b, c, n, ctl);
-      if (k < 0) k = oldest(~0u);
-      if (k < 0) k = open_item(b, c, n, ctl);
-      if (k < 0 && !ctl.exhausted) got = -1;
+      if (k < 0 && can_open && ctl.num_open < max_open) got = kScan;
+      if (k < 0 && got != kScan && !ctl.scanning) {
+        k = oldest(~0u);
+        if (k < 0 && can_open) got = kScan;
+      }
+      if (k < 0 && got != kScan && !ctl.exhausted) got = kLater;
+      if (got == kScan) ctl.scanning = 1u;
     }
     if (k >= 0) {
       Open& o = ctl.open[k];
@@ -314,7 +344,7 @@ struct PipeForward {
       t.in_row = o.last_row;
       t.out_row = 0;
       if (!t.last && ctl.free_rows == 0u) {
-        got = -1;
+        got = kLater;
       } else {
         if (!t.last) {
           t.out_row = (uint32_t)__ffs((int)ctl.free_rows) - 1u;
@@ -327,7 +357,7 @@ struct PipeForward {
         ++o.running;
         ctl.stop[warp] = 0u;
         ctl.task[warp] = t;
-        got = 1;
+        got = kPass;
       }
     }
     unlock(ctl);
@@ -339,7 +369,7 @@ struct PipeForward {
   // item's results or rescues.
   __device__ static bool close(const ClassLaunch& c, int warp, int lane, Ctl& ctl) {
     bool won = false;
-    if (lane == 0 && lock(ctl, c.error_flags)) {
+    if (lane == 0 && lock(ctl, c)) {
       const uint32_t slot = ctl.task[warp].slot;
       if (ctl.open[slot].state == kOpen && !ctl.stop[warp] && !ctl.fail) {
         ctl.open[slot].state = kClosed;
@@ -355,7 +385,7 @@ struct PipeForward {
   // The end of this warp's pass; swept: to its last column.
   __device__ static void release(const ClassLaunch& c, int warp, int lane, Ctl& ctl, bool swept) {
     __syncwarp();
-    if (lane == 0 && lock(ctl, c.error_flags)) {
+    if (lane == 0 && lock(ctl, c)) {
       const Task t = ctl.task[warp];
       Open& o = ctl.open[t.slot];
       auto give_back = [&](uint32_t bits) {
@@ -700,7 +730,8 @@ __global__ void __launch_bounds__(W * kWarp, MINB)
   const uint32_t n = c.work_count ? *c.work_count : c.static_count;
   const uint32_t max_open = (n + gridDim.x - 1) / gridDim.x;
   if (threadIdx.x == 0) {
-    ctl.lock = ctl.fail = ctl.started = ctl.exhausted = ctl.num_open = 0u;
+    ctl.ticket = ctl.serving = ctl.broken = ctl.fail = 0u;
+    ctl.started = ctl.scanning = ctl.exhausted = ctl.num_open = 0u;
     ctl.free_rows = (1u << F::kRows) - 1u;
     for (int w = 0; w < W; ++w) {
       ctl.stop[w] = 0u;
