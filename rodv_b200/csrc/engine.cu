@@ -214,20 +214,18 @@ void live_allocations(uint64_t* device, uint64_t* pinned) {
   if (pinned) *pinned = (uint64_t)g_live[1].load();
 }
 
-DeviceMem::~DeviceMem() {
-  if (ptr) {
-    cudaFree(ptr);
-    --g_live[0];
-  }
-}
-cudaError_t DeviceMem::ensure(size_t n) {
-  if (n <= bytes && ptr) return cudaSuccess;
+DeviceMem::~DeviceMem() { reset(); }
+void DeviceMem::reset() {
   if (ptr) {
     cudaFree(ptr);
     --g_live[0];
   }
   ptr = nullptr;
   bytes = 0;
+}
+cudaError_t DeviceMem::ensure(size_t n) {
+  if (n <= bytes && ptr) return cudaSuccess;
+  reset();
   if (injected_failure(0)) return cudaErrorMemoryAllocation;
   cudaError_t e = cudaMalloc(&ptr, std::max<size_t>(n, 1));
   if (e == cudaSuccess) {
@@ -238,20 +236,18 @@ cudaError_t DeviceMem::ensure(size_t n) {
   }
   return e;
 }
-PinnedMem::~PinnedMem() {
-  if (ptr) {
-    cudaFreeHost(ptr);
-    --g_live[1];
-  }
-}
-cudaError_t PinnedMem::ensure(size_t n) {
-  if (n <= bytes && ptr) return cudaSuccess;
+PinnedMem::~PinnedMem() { reset(); }
+void PinnedMem::reset() {
   if (ptr) {
     cudaFreeHost(ptr);
     --g_live[1];
   }
   ptr = nullptr;
   bytes = 0;
+}
+cudaError_t PinnedMem::ensure(size_t n) {
+  if (n <= bytes && ptr) return cudaSuccess;
+  reset();
   if (injected_failure(1)) return cudaErrorMemoryAllocation;
   cudaError_t e = cudaMallocHost(&ptr, std::max<size_t>(n, 1));
   if (e == cudaSuccess) {
@@ -383,20 +379,56 @@ rodv_status Engine::load_kernels() {
   return RODV_OK;
 }
 
-// Bytes of boundary rows of `cols` cells that the kernels of a multi-pass class
-// need (cells of 16 bytes in the uniform form, 24 in the per-row one): the
-// rows of the largest grid any of its variants launches (the autotuner runs
-// every variant on its batches).
-size_t Engine::multi_scratch_bytes(bool uniform, size_t cols) const {
+namespace {
+// Bytes of a boundary row's cell in the uniform and in the per-row form.
+size_t boundary_cell(bool uniform) { return uniform ? 16 : 24; }
+}  // namespace
+
+// Boundary rows of the largest grid of any variant of a multi-pass class's
+// kernels.  (The kernels for few blocks launch no larger ones.)
+size_t Engine::multi_rows(bool uniform) const {
   size_t rows = multi_rows_[uniform].load();
   if (!rows) {
     for_each_kernel([&](const KernelInfo& k) {
-      if (k.multi && k.uniform == uniform)
+      if (k.multi && k.uniform == uniform && !(k.variant & kPipeFew))
         rows = std::max(rows, (size_t)persistent_blocks(k) * k.boundary_rows);
     });
     multi_rows_[uniform].store(rows);
   }
-  return align_up(rows * cols * (uniform ? 16 : 24));
+  return rows;
+}
+// Bytes of boundary rows of `cols` cells that a multi-pass class's launches use
+// at most, whatever the batch.
+size_t Engine::multi_scratch_bytes(bool uniform, size_t cols) const {
+  return align_up(multi_rows(uniform) * cols * boundary_cell(uniform));
+}
+
+// Boundary rows of a plan's multi-pass class: of its own launches' grids (every
+// variant's: of the autotuner's).  The same- and two-haplotype launches have
+// rows of their own (and run side by side) if both fit where the largest grid's
+// would.  (Rows for the largest grids of both classes, whatever the batch, were
+// 0.8 GB for one pair at 5,000-base haplotypes and 11 GB at 65,536.)
+size_t Engine::plan_rows(const PackedPlan& plan, int c, bool every_variant) const {
+  const bool uniform = class_uniform(c);
+  const size_t most = multi_rows(uniform);
+  if (!plan.pairs[c]) return 0;
+  // rows of the grid for n items
+  auto rows_of = [&](Precision pr, bool same, int variant, uint32_t n) {
+    const KernelInfo k =
+        forward_kernel_info(pr, class_rows(c), plan.gap_form(c), true, same, variant);
+    return (size_t)std::min<uint32_t>(n, persistent_blocks(k)) * k.boundary_rows;
+  };
+  size_t rows = 2 * kMaxPipeWarps;  // one block of any variant (plain form)
+  for (int v = 0; v < kPipeVariants; ++v) {
+    if (every_variant || v == plan.variant64[c])
+      rows = std::max(rows, rows_of(Precision::kF64, false, v, plan.pairs[c]));
+    if (every_variant || v == plan.variant[c]) {
+      const size_t same = rows_of(Precision::kF32x2, true, v, plan.same_items[c]);
+      const size_t diff = rows_of(Precision::kF32x2, false, v, plan.diff_items[c]);
+      rows = std::max({rows, same, diff, same + diff <= most ? same + diff : 0});
+    }
+  }
+  return rows;
 }
 
 // Resident blocks of a kernel on the whole device, queried once per kernel
@@ -877,7 +909,8 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
     // one region per multi-pass class: the two classes' kernels run as
     // parallel graph branches and must not share boundary rows
     for (int u = 0; u < 2; ++u) {
-      plan.scratch_bytes[u] = multi_scratch_bytes(u != 0, plan.scratch_cols);
+      plan.scratch_bytes[u] = align_up(plan_rows(plan, kSinglePassClasses + u, !stack) *
+                                       plan.scratch_cols * boundary_cell(u != 0));
       o = align_up(o + plan.scratch_bytes[u]);
     }
   }
@@ -1063,6 +1096,14 @@ int even_blocks(int blocks, int items) {
   const int rounds = (items + blocks - 1) / blocks;
   return rounds > 1 && rounds <= 3 ? (items + rounds - 1) / rounds : blocks;
 }
+
+// Blocks of a multi-pass launch that the plan's boundary rows hold, from `skip`
+// bytes on.
+int scratch_blocks(const PackedPlan& plan, int c, const KernelInfo& k, size_t skip) {
+  const bool u = class_uniform(c);
+  const size_t block = (size_t)k.boundary_rows * plan.scratch_cols * boundary_cell(u);
+  return (int)std::min<size_t>((plan.scratch_bytes[u] - skip) / block, INT32_MAX);
+}
 }  // namespace
 
 rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int c, bool same,
@@ -1112,6 +1153,8 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
     }
   }
   if (blocks_cap > 0) blocks = std::min(blocks, blocks_cap);
+  if (class_multi(c)) blocks = std::min(blocks, scratch_blocks(plan, c, k, scratch_skip));
+  if (blocks < 1) return fail(RODV_ERR_INTERNAL, "no boundary rows for a multi-pass launch");
   void* args[] = {&a.view, &cl};
   RODV_CUDA(launch_kernel(k, blocks, args, stream));
   return RODV_OK;
@@ -1168,7 +1211,10 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
   cl.error_flags = a.counts + kCtrError;
   apply_wait_fault(cl, c);
   const int need = (int)((plan.pairs[c] + k.items_per_block - 1) / k.items_per_block);
-  const int blocks = even_blocks(std::max(1, std::min(persistent_blocks(k), need)), need);
+  const int blocks =
+      std::min(even_blocks(std::max(1, std::min(persistent_blocks(k), need)), need),
+               scratch_blocks(plan, c, k, 0));
+  if (blocks < 1) return fail(RODV_ERR_INTERNAL, "no boundary rows for a multi-pass launch");
   void* args[] = {&a.view, &cl};
   RODV_CUDA(launch_kernel(k, blocks, args, stream));
   return RODV_OK;
@@ -1256,7 +1302,7 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
                                                  plan.gap_form(c), true, same, plan.variant[c]);
         const uint32_t n = same ? plan.same_items[c] : plan.diff_items[c];
         bytes[same] = (size_t)std::min<uint32_t>(n, persistent_blocks(k)) * k.boundary_rows *
-                      plan.scratch_cols * (class_uniform(c) ? 16 : 24);
+                      plan.scratch_cols * boundary_cell(class_uniform(c));
       }
       if (bytes[0] && bytes[1] && bytes[0] + bytes[1] <= plan.scratch_bytes[class_uniform(c)])
         diff_skip[c] = bytes[1];
@@ -1460,7 +1506,18 @@ rodv_status Engine::run_host(const rodv_batch& b, double* out, rodv_stats* st, b
   in_order = in_order && h_end == b.num_haps && r_end == b.num_reads;
   if (bounds.size() < 3 || (cum[G] < kMaxWholeCells && !in_order && !cut_pays(b, bounds)))
     return run_host_single(b, out, st, fp64, prec);
-  return run_host_chunked(b, out, st, fp64, bounds, prec);
+  const rodv_status s = run_host_chunked(b, out, st, fp64, bounds, prec);
+  if (s != RODV_ERR_OUT_OF_MEMORY || cum[G] >= kMaxWholeCells) return s;
+  // Three ranges in flight do not fit (boundary rows of long haplotypes, a GPU
+  // that others use too): in one piece, with the ranges' memory given back.
+  cudaGetLastError();
+  for (HostLane& l : lanes_) {
+    l.arena.reset();
+    l.staging.reset();
+    l.out.reset();
+  }
+  if (st) *st = rodv_stats{};
+  return run_host_single(b, out, st, fp64, prec);
 }
 
 rodv_status Engine::finish_lane(HostLane& l, double* out, rodv_stats* st, uint8_t* prec) {
@@ -1561,7 +1618,10 @@ rodv_status Engine::run_host_chunked(const rodv_batch& b, double* out, rodv_stat
               (double)l.plan.cells, t_pack0, ms_since(t0));
     const PackedPlan& p = l.plan;
     cudaError_t e = cudaSuccess;
-    if (l.arena.bytes < p.total_bytes) e = l.arena.ensure(p.total_bytes + p.total_bytes / 4);
+    // headroom for the next ranges' items; boundary rows do not grow with them
+    const size_t scratch = p.scratch_bytes[0] + p.scratch_bytes[1];
+    if (l.arena.bytes < p.total_bytes)
+      e = l.arena.ensure(p.total_bytes + (p.total_bytes - scratch) / 4);
     const size_t ob = p.result_bytes();
     if (e == cudaSuccess && l.out.bytes < ob) e = l.out.ensure(ob + ob / 4);
     uint8_t* d = static_cast<uint8_t*>(l.arena.ptr);

@@ -62,6 +62,7 @@ struct DeviceMem {
   void* ptr = nullptr;
   size_t bytes = 0;
   ~DeviceMem();
+  void reset();
   cudaError_t ensure(size_t n);
 };
 
@@ -69,6 +70,7 @@ struct PinnedMem {
   void* ptr = nullptr;
   size_t bytes = 0;
   ~PinnedMem();
+  void reset();
   cudaError_t ensure(size_t n);
 };
 
@@ -218,7 +220,9 @@ class Engine {
                                const std::vector<uint32_t>& bounds, uint8_t* prec);
   rodv_status finish_lane(HostLane& lane, double* out, rodv_stats* st, uint8_t* prec);
   int persistent_blocks(const KernelInfo& k) const;
+  size_t multi_rows(bool uniform) const;
   size_t multi_scratch_bytes(bool uniform, size_t cols) const;
+  size_t plan_rows(const PackedPlan& plan, int c, bool every_variant) const;
   std::string device_key() const;
   bool load_tuning(const std::string& path);
   bool save_tuning(const std::string& path) const;
