@@ -230,19 +230,15 @@ struct PipeForward {
     atomicAdd(&ctl.serving, 1u);
   }
 
-  // Opens the queue's next valid item, or notes that the queue is empty, for the
-  // lane whose try_acquire returned kScan (and set ctl.scanning, so that no
-  // other opens one meanwhile).  The queue is read outside the lock: an FP64
-  // list of 1e8 positions that no rescue filled keeps a block looking for half
-  // a second.  False if the lock was not to be had.
-  __device__ static bool open_item(const BatchView& b, const ClassLaunch& c, uint32_t n, Ctl& ctl) {
-    uint32_t found = kNoPair, passes = 0;
+  // The queue's next valid item and its passes; kNoPair when the queue is empty.
+  __device__ static uint32_t next_item(const BatchView& b, const ClassLaunch& c, uint32_t n,
+                                       Ctl& ctl, uint32_t& passes) {
     for (;;) {
       // the block's first item is its own: another block that opens two at once
       // must not leave it without
       const uint32_t item = ctl.started ? gridDim.x + atomicAdd(c.counter, 1u) : blockIdx.x;
       ctl.started = 1u;
-      if (item >= n) break;
+      if (item >= n) return kNoPair;
       PairRef refs[2];
       F::load_refs(c, item, refs);
       // an FP64 list position that no rescue filled (kLaunchRescueByItem lists)
@@ -257,20 +253,35 @@ struct PipeForward {
         atomicOr(c.error_flags, kErrBadLength);
         continue;
       }
-      found = item;
       passes = pipe_passes(lx > ly ? lx : ly, R);
-      break;
+      return item;
     }
+  }
+
+  // Opens `item` (next_item) in a free slot, of which there is one; its slot, or -1
+  // if the queue was empty.  Under the lock.
+  __device__ static int open_item(Ctl& ctl, uint32_t item, uint32_t passes) {
+    if (item == kNoPair) {
+      ctl.exhausted = 1u;
+      return -1;
+    }
+    int slot = 0;
+    while (slot < W - 1 && ctl.open[slot].state != kFree) ++slot;
+    ctl.open[slot] = Open{kOpen, item, passes, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+    ++ctl.num_open;
+    return slot;
+  }
+
+  // Takes the queue's next item for the lane whose try_acquire returned kScan (and
+  // set ctl.scanning, so that no other takes one meanwhile), outside the lock: an
+  // FP64 list of 1e8 positions that no rescue filled keeps a block looking for
+  // half a second.  False if the lock was not to be had.
+  __device__ static bool scan(const BatchView& b, const ClassLaunch& c, uint32_t n, Ctl& ctl) {
+    uint32_t passes = 0;
+    const uint32_t item = next_item(b, c, n, ctl, passes);
     if (!lock(ctl, c)) return false;
     ctl.scanning = 0u;
-    if (found == kNoPair) {
-      ctl.exhausted = 1u;
-    } else {
-      int slot = 0;  // num_open < W when the scan began: one is free
-      while (slot < W - 1 && ctl.open[slot].state != kFree) ++slot;
-      ctl.open[slot] = Open{kOpen, found, passes, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-      ++ctl.num_open;
-    }
+    open_item(ctl, item, passes);
     unlock(ctl);
     return true;
   }
@@ -282,8 +293,8 @@ struct PipeForward {
     int got = kNone;
     for (uint32_t tries = 0;; ++tries) {
       if (lane == 0) {
-        while ((got = try_acquire(c, max_open, warp, ctl)) == kScan)
-          if (!open_item(b, c, n, ctl)) {
+        while ((got = try_acquire(b, c, n, max_open, warp, ctl)) == kScan)
+          if (!scan(b, c, n, ctl)) {
             got = kNone;
             break;
           }
@@ -307,9 +318,11 @@ struct PipeForward {
   // One try, by one lane.  kNone: no pass is left to start.  kLater: another
   // warp is taking an item off the queue, or every row or slot is held by items
   // that are being closed (their last passes end within kStopChunks chunks).
-  // kScan: a new item is wanted, and this lane is to take it (open_item).
+  // kScan: a new item is wanted, and this lane is to take it (scan).  FP32 lists
+  // have no empty positions: their next item is taken under the lock.
   enum : int { kNone, kPass, kLater, kScan };
-  __device__ static int try_acquire(const ClassLaunch& c, uint32_t max_open, int warp, Ctl& ctl) {
+  __device__ static int try_acquire(const BatchView& b, const ClassLaunch& c, uint32_t n,
+                                    uint32_t max_open, int warp, Ctl& ctl) {
     if (!lock(ctl, c)) return kNone;
     auto oldest = [&](uint32_t window) {
       int best = -1;
@@ -325,13 +338,18 @@ struct PipeForward {
     if (!ctl.fail) {
       const bool can_open = !ctl.exhausted && !ctl.scanning && ctl.num_open < W;
       k = oldest(kWindow);
-      if (k < 0 && can_open && ctl.num_open < max_open) got = kScan;
-      if (k < 0 && got != kScan && !ctl.scanning) {
-        k = oldest(~0u);
-        if (k < 0 && can_open) got = kScan;
+      if (P::kSlots == 2) {
+        uint32_t passes = 0;
+        if (k < 0 && can_open && ctl.num_open < max_open)
+          k = open_item(ctl, next_item(b, c, n, ctl, passes), passes);
+        if (k < 0) k = oldest(~0u);
+        if (k < 0 && can_open && !ctl.exhausted)
+          k = open_item(ctl, next_item(b, c, n, ctl, passes), passes);
+      } else if (k < 0 && can_open) {  // (kWindow takes every pass that can start)
+        got = kScan;
+        ctl.scanning = 1u;
       }
-      if (k < 0 && got != kScan && !ctl.exhausted) got = kLater;
-      if (got == kScan) ctl.scanning = 1u;
+      if (k < 0 && got == kNone && !ctl.exhausted) got = kLater;
     }
     if (k >= 0) {
       Open& o = ctl.open[k];
