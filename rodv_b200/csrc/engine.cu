@@ -37,6 +37,7 @@
 
 #include "engine.h"
 #include "chain_plan.h"
+#include "multi_grid.h"
 #include "pack_rows.h"
 #include "tables.h"
 #include "trace.h"
@@ -1089,14 +1090,6 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
 // Launches
 // ---------------------------------------------------------------------------
 namespace {
-// Grid of a multi-pass launch of `items` items, at most `blocks` resident: up to
-// three items a block, every block gets as many (540 pairs of reads of 850 x
-// 4,300 bases: 1.68 ms on 444 blocks, 1.38 on 270 of two items each).
-int even_blocks(int blocks, int items) {
-  const int rounds = (items + blocks - 1) / blocks;
-  return rounds > 1 && rounds <= 3 ? (items + rounds - 1) / rounds : blocks;
-}
-
 // Blocks of a multi-pass launch that the plan's boundary rows hold, from `skip`
 // bytes on.
 int scratch_blocks(const PackedPlan& plan, int c, const KernelInfo& k, size_t skip) {
@@ -1107,8 +1100,8 @@ int scratch_blocks(const PackedPlan& plan, int c, const KernelInfo& k, size_t sk
 }  // namespace
 
 rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int c, bool same,
-                                      int variant, int blocks_cap, cudaStream_t stream,
-                                      size_t scratch_skip) {
+                                      int variant, cudaStream_t stream, size_t scratch_skip,
+                                      bool few) {
   ArenaView a = arena_view(plan, dbase, tab_);
   const uint32_t n = same ? plan.same_items[c] : plan.diff_items[c];
   if (!n) return RODV_OK;
@@ -1139,21 +1132,12 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   const int need = (int)((n + per_block - 1) / per_block);
   int blocks = std::max(1, std::min(persistent_blocks(k), need));
   if (class_multi(c)) {
-    blocks = even_blocks(blocks, need);
-    // A grid that fits at 8 warps per SM takes the kernel built for those: its
-    // items' sweeps are shorter (pairs of reads of about 1,500 x 4,350 bases, 18
-    // items 1.08 -> 1.04 ms, 540 in 270 blocks 2.70 -> 2.59).  Above that, the
-    // resident warps count for more (2,160 such items 7.78 ms at 12 warps per SM,
-    // 8.64 at 8).
-    if (pipe_has_few(Precision::kF32x2, class_uniform(c))) {
-      const KernelInfo few = forward_kernel_info(Precision::kF32x2, class_rows(c),
-                                                 plan.gap_form(c), true, same,
-                                                 variant | kPipeFew);
-      if (blocks <= persistent_blocks(few)) k = few;
-    }
+    blocks = even_blocks(persistent_blocks(k), need);
+    if (few && pipe_has_few(Precision::kF32x2, class_uniform(c)))
+      k = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c), true, same,
+                              variant | kPipeFew);
+    blocks = std::min(blocks, scratch_blocks(plan, c, k, scratch_skip));
   }
-  if (blocks_cap > 0) blocks = std::min(blocks, blocks_cap);
-  if (class_multi(c)) blocks = std::min(blocks, scratch_blocks(plan, c, k, scratch_skip));
   if (blocks < 1) return fail(RODV_ERR_INTERNAL, "no boundary rows for a multi-pass launch");
   void* args[] = {&a.view, &cl};
   RODV_CUDA(launch_kernel(k, blocks, args, stream));
@@ -1212,8 +1196,7 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
   apply_wait_fault(cl, c);
   const int need = (int)((plan.pairs[c] + k.items_per_block - 1) / k.items_per_block);
   const int blocks =
-      std::min(even_blocks(std::max(1, std::min(persistent_blocks(k), need)), need),
-               scratch_blocks(plan, c, k, 0));
+      std::min(even_blocks(persistent_blocks(k), need), scratch_blocks(plan, c, k, 0));
   if (blocks < 1) return fail(RODV_ERR_INTERNAL, "no boundary rows for a multi-pass launch");
   void* args[] = {&a.view, &cl};
   RODV_CUDA(launch_kernel(k, blocks, args, stream));
@@ -1295,18 +1278,23 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
     // launches' (diff_skip: where the second one's start; else the two share
     // rows and stay in sequence).
     size_t diff_skip[kNumClasses] = {};
+    long multi_warps = 0;  // of the multi-pass launches that run at a time
     for (int c = kSinglePassClasses; c < kNumClasses; ++c) {
       size_t bytes[2];
+      long warps[2] = {0, 0};
       for (int same = 0; same < 2; ++same) {
         const KernelInfo k = forward_kernel_info(Precision::kF32x2, class_rows(c),
                                                  plan.gap_form(c), true, same, plan.variant[c]);
         const uint32_t n = same ? plan.same_items[c] : plan.diff_items[c];
         bytes[same] = (size_t)std::min<uint32_t>(n, persistent_blocks(k)) * k.boundary_rows *
                       plan.scratch_cols * boundary_cell(class_uniform(c));
+        if (n) warps[same] = (long)even_blocks(persistent_blocks(k), (int)n) * k.warps_per_block;
       }
       if (bytes[0] && bytes[1] && bytes[0] + bytes[1] <= plan.scratch_bytes[class_uniform(c)])
         diff_skip[c] = bytes[1];
+      multi_warps += diff_skip[c] ? warps[0] + warps[1] : std::max(warps[0], warps[1]);
     }
+    const bool few = takes_few(multi_warps, num_sms_);
     auto branch = [&](int c, bool same) {
       return same || (class_multi(c) && !diff_skip[c]) ? c : c + kNumClasses;
     };
@@ -1324,8 +1312,8 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
         if (!(same ? plan.same_items[c] : plan.diff_items[c])) continue;
         const cudaStream_t ls = lane(branch(c, same != 0));
         if (!ls) return cuda_fail(cudaErrorUnknown, "class stream fork");
-        rodv_status s = launch_fp32_class(plan, dbase, c, same != 0, plan.variant[c], 0, ls,
-                                          same ? 0 : diff_skip[c]);
+        rodv_status s = launch_fp32_class(plan, dbase, c, same != 0, plan.variant[c], ls,
+                                          same ? 0 : diff_skip[c], few);
         if (s != RODV_OK) return s;
         ++launches;
       }
@@ -2087,7 +2075,7 @@ rodv_status Engine::autotune(const char* cache_path, int force, int32_t* variant
             db->plan, d,
             [&]() {
               return f64 ? launch_fp64_class(db->plan, d, c, v, stream_)
-                         : launch_fp32_class(db->plan, d, c, true, v, 0, stream_);
+                         : launch_fp32_class(db->plan, d, c, true, v, stream_);
             },
             &ms);
         if (s != RODV_OK) {

@@ -207,8 +207,8 @@ class Engine {
                            cudaStream_t stream, cudaEvent_t* ev, int parts, bool fan_out,
                            bool reset);
   rodv_status launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int cls, bool same,
-                                int variant, int blocks_cap, cudaStream_t stream,
-                                size_t scratch_skip = 0);
+                                int variant, cudaStream_t stream, size_t scratch_skip = 0,
+                                bool few = false);
   rodv_status launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int cls, int variant,
                                 cudaStream_t stream);
   rodv_status launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform,

@@ -35,8 +35,9 @@ inline int pipe_variant_rows(int variant) { return (variant & 2) ? 4 : 8; }
 inline int pipe_variant_warps(int variant) { return (variant & 1) ? 4 : 2; }
 constexpr int kMaxPipeWarps = 4;
 // A variant with this bit set is the same FP32 uniform-gap kernel built for
-// launches of few blocks: up to 8 warps per SM instead of 12.  The engine sets
-// it by a launch's grid (pipe_has_few); it is no variant of the autotuner's.
+// launches of few blocks: up to 8 warps per SM (takes_few), with as many registers
+// as it asks for.  The engine sets it by the launches' grids; it is no variant of
+// the autotuner's.
 constexpr int kPipeFew = 4;
 inline bool pipe_has_few(Precision prec, bool uniform) {
   return prec == Precision::kF32x2 && uniform;
