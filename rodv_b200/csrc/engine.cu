@@ -1101,7 +1101,7 @@ int scratch_blocks(const PackedPlan& plan, int c, const KernelInfo& k, size_t sk
 
 rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int c, bool same,
                                       int variant, cudaStream_t stream, size_t scratch_skip,
-                                      bool few) {
+                                      MultiKernel multi, int* grid) {
   ArenaView a = arena_view(plan, dbase, tab_);
   const uint32_t n = same ? plan.same_items[c] : plan.diff_items[c];
   if (!n) return RODV_OK;
@@ -1132,13 +1132,14 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   const int need = (int)((n + per_block - 1) / per_block);
   int blocks = std::max(1, std::min(persistent_blocks(k), need));
   if (class_multi(c)) {
-    blocks = even_blocks(persistent_blocks(k), need);
-    if (few && pipe_has_few(Precision::kF32x2, class_uniform(c)))
+    if (multi != MultiKernel::kFull) blocks = even_blocks(persistent_blocks(k), need);
+    if (multi == MultiKernel::kFew && pipe_has_few(Precision::kF32x2, class_uniform(c)))
       k = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c), true, same,
                               variant | kPipeFew);
     blocks = std::min(blocks, scratch_blocks(plan, c, k, scratch_skip));
   }
   if (blocks < 1) return fail(RODV_ERR_INTERNAL, "no boundary rows for a multi-pass launch");
+  if (grid) *grid = blocks;
   void* args[] = {&a.view, &cl};
   RODV_CUDA(launch_kernel(k, blocks, args, stream));
   return RODV_OK;
@@ -1174,7 +1175,8 @@ rodv_status Engine::launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool u
 
 // FP64 launch of multi-pass class c over its list.
 rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int c,
-                                      int variant, cudaStream_t stream) {
+                                      int variant, cudaStream_t stream, bool full_grid,
+                                      int* grid) {
   ArenaView a = arena_view(plan, dbase, tab_);
   const KernelInfo k = forward_kernel_info(Precision::kF64, class_rows(c), plan.gap_form(c),
                                            true, false, variant);
@@ -1195,9 +1197,11 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
   cl.error_flags = a.counts + kCtrError;
   apply_wait_fault(cl, c);
   const int need = (int)((plan.pairs[c] + k.items_per_block - 1) / k.items_per_block);
-  const int blocks =
-      std::min(even_blocks(persistent_blocks(k), need), scratch_blocks(plan, c, k, 0));
+  const int blocks = std::min(full_grid ? std::min(persistent_blocks(k), need)
+                                        : even_blocks(persistent_blocks(k), need),
+                              scratch_blocks(plan, c, k, 0));
   if (blocks < 1) return fail(RODV_ERR_INTERNAL, "no boundary rows for a multi-pass launch");
+  if (grid) *grid = blocks;
   void* args[] = {&a.view, &cl};
   RODV_CUDA(launch_kernel(k, blocks, args, stream));
   return RODV_OK;
@@ -1294,7 +1298,8 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
         diff_skip[c] = bytes[1];
       multi_warps += diff_skip[c] ? warps[0] + warps[1] : std::max(warps[0], warps[1]);
     }
-    const bool few = takes_few(multi_warps, num_sms_);
+    const MultiKernel multi =
+        takes_few(multi_warps, num_sms_) ? MultiKernel::kFew : MultiKernel::kEven;
     auto branch = [&](int c, bool same) {
       return same || (class_multi(c) && !diff_skip[c]) ? c : c + kNumClasses;
     };
@@ -1313,7 +1318,7 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
         const cudaStream_t ls = lane(branch(c, same != 0));
         if (!ls) return cuda_fail(cudaErrorUnknown, "class stream fork");
         rodv_status s = launch_fp32_class(plan, dbase, c, same != 0, plan.variant[c], ls,
-                                          same ? 0 : diff_skip[c], few);
+                                          same ? 0 : diff_skip[c], multi);
         if (s != RODV_OK) return s;
         ++launches;
       }
@@ -2033,12 +2038,21 @@ rodv_status Engine::autotune(const char* cache_path, int force, int32_t* variant
     const bool multi = class_multi(c), uni = class_uniform(c);
     TuneBatch tb;
     if (multi) {
-      // long pairs, several waves of the largest grid of one item per block:
-      // half the regions with reads of 1% differences (the FP32 sweep runs
+      // long pairs, three rounds and more of the largest grid of one item per
+      // block (every variant runs on its full grid, with the kernel built for
+      // it): half the regions with reads of 1% differences (the FP32 sweep runs
       // every pass), half with 8% (it stops after the first passes and the
       // pairs go to FP64), so the choice weighs both kinds of long read
-      make_tune_batch(tb, rng, num_sms_ * 2, 1, 2, 3000, 1500, uni, 100);
-      make_tune_batch(tb, rng, num_sms_ * 2, 1, 2, 3000, 1500, uni, 12);
+      size_t most = 1;
+      for (int f64 = 0; f64 < 2; ++f64)
+        for (int v = 0; v < kPipeVariants; ++v)
+          most = std::max<size_t>(
+              most, persistent_blocks(forward_kernel_info(
+                        f64 ? Precision::kF64 : Precision::kF32x2, R,
+                        uni ? kGapsConst : kGapsPerRow, true, !f64, v)));
+      const int haps = 8, regions = (int)(3 * most / (2 * haps)) + 1;  // items: regions x haps
+      make_tune_batch(tb, rng, regions, haps, 2, 3000, 1500, uni, 100);
+      make_tune_batch(tb, rng, regions, haps, 2, 3000, 1500, uni, 12);
     } else {
       // Enough items that every warp of the largest grid takes several (chain
       // items of 4 haplotypes: ~8), so the timing reflects per-item throughput
@@ -2067,15 +2081,18 @@ rodv_status Engine::autotune(const char* cache_path, int force, int32_t* variant
       const Precision pr = f64 ? Precision::kF64 : Precision::kF32x2;
       const int nvar = forward_kernel_variants(pr, !f64, R, multi);
       int* slot = f64 ? &variant64_[c] : &variant_[c];
-      float best_ms = 1e30f;
+      float best_ms = 1e30f, default_ms = 1e30f;
       int best_v = *slot;
+      const int dv = f64 ? default_variant64(c) : default_variant(c);
       for (int v = 0; v < nvar; ++v) {
         float ms = 0.f;
+        int grid = 0;
         s = time_launch(
             db->plan, d,
             [&]() {
-              return f64 ? launch_fp64_class(db->plan, d, c, v, stream_)
-                         : launch_fp32_class(db->plan, d, c, true, v, stream_);
+              return f64 ? launch_fp64_class(db->plan, d, c, v, stream_, true, &grid)
+                         : launch_fp32_class(db->plan, d, c, true, v, stream_, 0,
+                                             MultiKernel::kFull, &grid);
             },
             &ms);
         if (s != RODV_OK) {
@@ -2083,13 +2100,23 @@ rodv_status Engine::autotune(const char* cache_path, int force, int32_t* variant
           return s;
         }
         if (opt_.verbose)
-          fprintf(stderr, "rodv: tune %s class %d (R=%d%s%s) variant %d (%s): %.3f ms\n",
+          fprintf(stderr,
+                  "rodv: tune %s class %d (R=%d%s%s) variant %d (%s): %.3f ms, %u items on %d "
+                  "blocks\n",
                   f64 ? "FP64" : "FP32", c, R, uni ? ", uniform" : "",
-                  multi ? ", multi-pass" : "", v, variant_name(c, v, f64).c_str(), ms);
+                  multi ? ", multi-pass" : "", v, variant_name(c, v, f64).c_str(), ms,
+                  f64 ? db->plan.pairs[c] : db->plan.same_items[c], grid);
+        if (v == dv) default_ms = ms;
         if (ms < best_ms) {
           best_ms = ms;
           best_v = v;
         }
+      }
+      // Full grids of two and of four warps an item come within a few thousandths
+      // of each other; with four, the items of a small batch take half as long.
+      if (multi && best_ms > 0.98f * default_ms) {
+        best_v = dv;
+        best_ms = default_ms;
       }
       delete db;
       *slot = best_v;

@@ -206,11 +206,15 @@ class Engine {
   rodv_status launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_stats* st,
                            cudaStream_t stream, cudaEvent_t* ev, int parts, bool fan_out,
                            bool reset);
+  // multi (multi-pass classes): kFull as the autotuner times the kernel of full
+  // grids, kEven and kFew by the batch (multi_grid.h); grid: takes the blocks.
+  enum class MultiKernel { kFull, kEven, kFew };
   rodv_status launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, int cls, bool same,
-                                int variant, cudaStream_t stream, size_t scratch_skip = 0,
-                                bool few = false);
+                                int variant, cudaStream_t stream, size_t scratch_skip,
+                                MultiKernel multi, int* grid = nullptr);
   rodv_status launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int cls, int variant,
-                                cudaStream_t stream);
+                                cudaStream_t stream, bool full_grid = false,
+                                int* grid = nullptr);
   rodv_status launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform,
                             cudaStream_t stream);
   rodv_status check_errors(const PackedPlan& plan, uint8_t* dbase);
