@@ -732,7 +732,7 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
     Counts n = {};                               // same: of multi-pass classes only
     uint64_t chains[kSinglePassClasses][kCaps] = {};  // chain items by cap
     uint64_t cells = 0;
-    uint32_t multi_hap = 0;
+    uint32_t multi_hap = 0, multi_read[2] = {0, 0};
     bool bad_class = false;
   };
   const uint32_t nblocks = (G + kBlockRegions - 1) / kBlockRegions;
@@ -756,7 +756,11 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
           const int c = read_class[r];
           ++n[c];
           rs += b.read_lengths[r];
-          if (class_multi(c)) rp.left[c - kSinglePassClasses] = r;
+          if (class_multi(c)) {
+            const int u = c - kSinglePassClasses;
+            rp.left[u] = r;
+            bl.multi_read[u] = std::max(bl.multi_read[u], b.read_lengths[r]);
+          }
         }
         bl.cells += hsum[g] * rs;
         for (int c = 0; c < kNumClasses; ++c) {
@@ -805,6 +809,8 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
                   "packer placed a chain item outside the single-pass classes");
     plan.cells += bl.cells;
     plan.multi_max_hap = std::max(plan.multi_max_hap, bl.multi_hap);
+    for (int u = 0; u < 2; ++u)
+      plan.multi_max_read[u] = std::max(plan.multi_max_read[u], bl.multi_read[u]);
   }
   // Haplotypes per chain item, per class: the longest chains (up to
   // kChainHaps) that still leave every resident warp of the class's launch
@@ -1132,7 +1138,7 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   const int need = (int)((n + per_block - 1) / per_block);
   int blocks = std::max(1, std::min(persistent_blocks(k), need));
   if (class_multi(c)) {
-    if (multi != MultiKernel::kFull) blocks = even_blocks(persistent_blocks(k), need);
+    if (multi != MultiKernel::kFull) blocks = even_blocks(persistent_blocks(k), need, kEvenRoundsF32);
     if (multi == MultiKernel::kFew && pipe_has_few(Precision::kF32x2, class_uniform(c)))
       k = forward_kernel_info(Precision::kF32x2, class_rows(c), plan.gap_form(c), true, same,
                               variant | kPipeFew);
@@ -1197,8 +1203,12 @@ rodv_status Engine::launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, in
   cl.error_flags = a.counts + kCtrError;
   apply_wait_fault(cl, c);
   const int need = (int)((plan.pairs[c] + k.items_per_block - 1) / k.items_per_block);
-  const int blocks = std::min(full_grid ? std::min(persistent_blocks(k), need)
-                                        : even_blocks(persistent_blocks(k), need),
+  const int rounds =
+      full_grid ? 1
+                : even_rounds_f64((int)pipe_passes(plan.multi_max_read[class_uniform(c)],
+                                                   k.rows_per_lane),
+                                  k.warps_per_block);
+  const int blocks = std::min(even_blocks(persistent_blocks(k), need, rounds),
                               scratch_blocks(plan, c, k, 0));
   if (blocks < 1) return fail(RODV_ERR_INTERNAL, "no boundary rows for a multi-pass launch");
   if (grid) *grid = blocks;
@@ -1292,7 +1302,9 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
         const uint32_t n = same ? plan.same_items[c] : plan.diff_items[c];
         bytes[same] = (size_t)std::min<uint32_t>(n, persistent_blocks(k)) * k.boundary_rows *
                       plan.scratch_cols * boundary_cell(class_uniform(c));
-        if (n) warps[same] = (long)even_blocks(persistent_blocks(k), (int)n) * k.warps_per_block;
+        if (n)
+          warps[same] = (long)even_blocks(persistent_blocks(k), (int)n, kEvenRoundsF32) *
+                        k.warps_per_block;
       }
       if (bytes[0] && bytes[1] && bytes[0] + bytes[1] <= plan.scratch_bytes[class_uniform(c)])
         diff_skip[c] = bytes[1];

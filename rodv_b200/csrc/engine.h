@@ -82,6 +82,7 @@ struct PackedPlan {
   uint32_t num_haps = 0, num_reads = 0;
   uint32_t max_hap_len = 0;
   uint32_t multi_max_hap = 0;
+  uint32_t multi_max_read[2] = {0, 0};     // of the per-row and the uniform multi-pass class
   bool fp64 = false;                       // every pair computed in FP64
   bool raw = false;                        // raw likelihoods and their precision
   // Every uniform-gap read of the batch has the same gap qualities: the
