@@ -158,6 +158,12 @@ struct PipeForward {
   // (0.908), at 12 warps 0.489 (0.932), four steps at 12 warps 0.483 (0.921).
   static constexpr bool kFew = P::kSlots == 2 && kTwo && MINB * W <= 8;
   static constexpr int kUnroll = kFew ? 4 : 8;
+  // Where lane 0 alone reads its row above from the ring, in the step itself:
+  // in FP64 the three-value form's cells (24 bytes) cost the other lanes more
+  // than the load's latency costs lane 0.  20 pairs of 1,000-2,000 bases
+  // 1.33 -> 1.24 ms, 100 pairs 1.41 -> 1.31, 1,500 pairs 6.45 -> 6.30 (four steps
+  // an iteration, all lanes reading: 1.31, 1.38, 6.6).
+  static constexpr bool kLoneRead = !kTwo && P::kSlots == 1;
   static constexpr int kSmemPerWarp = F::kSmemPerWarp;  // emission table + cell ring
   // polls of a progress word (about 100 ns each) before a wait gives up
   static constexpr uint32_t kWaitPolls = 1u << 24;
@@ -258,6 +264,13 @@ struct PipeForward {
     }
   }
 
+  // The same out of line, for the kernel whose sweep is a hundredth slower with it
+  // in line (kLoneRead; the others' are with the call).
+  __device__ __noinline__ static uint32_t next_item_call(const BatchView& b, const ClassLaunch& c,
+                                                         uint32_t n, Ctl& ctl, uint32_t& passes) {
+    return next_item(b, c, n, ctl, passes);
+  }
+
   // Opens `item` (next_item) in a free slot, of which there is one; its slot, or -1
   // if the queue was empty.  Under the lock.
   __device__ static int open_item(Ctl& ctl, uint32_t item, uint32_t passes) {
@@ -278,7 +291,8 @@ struct PipeForward {
   // half a second.  False if the lock was not to be had.
   __device__ static bool scan(const BatchView& b, const ClassLaunch& c, uint32_t n, Ctl& ctl) {
     uint32_t passes = 0;
-    const uint32_t item = next_item(b, c, n, ctl, passes);
+    const uint32_t item = kLoneRead ? next_item_call(b, c, n, ctl, passes)
+                                    : next_item(b, c, n, ctl, passes);
     if (!lock(ctl, c)) return false;
     ctl.scanning = 0u;
     open_item(ctl, item, passes);
@@ -346,8 +360,17 @@ struct PipeForward {
         if (k < 0 && can_open && !ctl.exhausted)
           k = open_item(ctl, next_item(b, c, n, ctl, passes), passes);
       } else if (k < 0 && can_open) {  // (kWindow takes every pass that can start)
-        got = kScan;
-        ctl.scanning = 1u;
+        // kLoneRead, up to two items a block: the further one waits until half the
+        // block's warps are free for it.  Begun by one warp, it ends a whole pass
+        // later than in a block whose item ends next (400 pairs of 1,000-2,000
+        // bases on 296 blocks: 2.37 -> 2.22 ms; 1,500 pairs 6.37 -> 6.52).
+        uint32_t running = 0;
+        for (int w = 0; w < W && kLoneRead && max_open <= 2u; ++w)
+          running += ctl.open[w].state != kFree ? ctl.open[w].running : 0u;
+        if (running <= W / 2) {
+          got = kScan;
+          ctl.scanning = 1u;
+        }
       }
       if (k < 0 && got == kNone && !ctl.exhausted) got = kLater;
     }
@@ -598,13 +621,13 @@ struct PipeForward {
       // in every pass (only the last pass's is used): a test in each step
       // cost more than the add.
       Cell cell_next;  // lane 0's row above in the next step, loaded a step ahead
-      auto step = [&](int s, const Cell* next) {
+      auto step = [&](int s, const Cell* now, const Cell* next) {
         const uint32_t cx = cx_next, cy = cy_next;
         cx_next = hx[s];
         if (!F::kSameHap) cy_next = hy[s];
         V e[R], t_last;
-        const Cell cl = cell_next;
-        cell_next = *next;
+        Cell cl = cell_next;
+        if (!kLoneRead) cell_next = *next;
         if constexpr (kTwo) {
           V in_t = P::shfl_up(h_t), in_i = P::shfl_up(h_i);
           if (kLag == 2) {
@@ -626,6 +649,7 @@ struct PipeForward {
           V up_i = P::shfl_up(I[R - 1]);
           V up_d = P::shfl_up(D[R - 1]);
           if (lane == 0) {
+            if (kLoneRead) cl = *now;
             up_m = cl.m; up_i = cl.i; up_d = cl.d;
           }
           F::load_emission(table, lane, cx, cy, e);
@@ -662,12 +686,13 @@ struct PipeForward {
 #pragma unroll 1
           for (int i = 0; i < kWarp; i += kUnroll) {
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) step(s0 + i + u, rc + ((i + u + 1) & (kWarp - 1)));
+            for (int u = 0; u < kUnroll; ++u)
+              step(s0 + i + u, rc + i + u, rc + ((i + u + 1) & (kWarp - 1)));
           }
         } else {
 #pragma unroll 1
           for (int i = 0; i < cnt; ++i) {
-            step(s0 + i, rc + ((i + 1) & (kWarp - 1)));
+            step(s0 + i, rc + i, rc + ((i + 1) & (kWarp - 1)));
             if (freeze && s0 + i == nfreeze - 1) frozen = P::sy(acc);
           }
         }
