@@ -1151,27 +1151,27 @@ rodv_status Engine::launch_fp32_class(const PackedPlan& plan, uint8_t* dbase, in
   return RODV_OK;
 }
 
-// FP64 launch of every single-pass class of one gap form over their lists
-// (rescued pairs, or every pair when FP64 is forced); the lists' lengths are
-// read by the kernel.
-rodv_status Engine::launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform,
-                                  cudaStream_t stream) {
+// FP64 launch of the single-pass classes of one gap form with lo to hi rows per
+// lane over their lists (rescued pairs, or every pair when FP64 is forced); the
+// lists' lengths are read by the kernel.
+rodv_status Engine::launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform, int lo,
+                                  int hi, cudaStream_t stream) {
   ArenaView a = arena_view(plan, dbase, tab_);
   RescueLaunch r{};
   uint64_t pairs = 0;
-  for (int R = 1; R <= kMaxRowsPerLane; ++R) {
+  for (int R = lo; R <= hi; ++R) {
     const int c = single_pass_class(R, uniform);
     if (!plan.pairs[c]) continue;
     pairs += plan.pairs[c];
     r.list[R - 1] = reinterpret_cast<const PairRef*>(dbase + plan.off_lists[c]);
     r.count[R - 1] = a.counts + kCtrRescue + c;
   }
-  const int first = single_pass_class(1, uniform);
+  const int first = single_pass_class(lo, uniform);
   r.c.counter = a.counts + kCtrF64 + first;
   r.c.error_flags = a.counts + kCtrError;
   r.c.gaps = plan.gaps;
-  const KernelInfo k = forward_kernel_info(Precision::kF64, kMaxRowsPerLane,
-                                           plan.gap_form(first), false, false, 0);
+  const KernelInfo k =
+      forward_kernel_info(Precision::kF64, hi, plan.gap_form(first), false, false, 0);
   const uint64_t need = (pairs + k.items_per_block - 1) / k.items_per_block;
   const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(persistent_blocks(k), need));
   void* args[] = {&a.view, &r};
@@ -1338,14 +1338,37 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
     RODV_CUDA(join());
   }
   if (ev) RODV_CUDA(cudaEventRecord(ev[1], stream));
-  bool f64_form[2] = {};  // single-pass classes of the form have FP64 work
-  for (int c = 0; c < kSinglePassClasses; ++c)
-    f64_form[class_uniform(c)] = f64_form[class_uniform(c)] || plan.pairs[c] > 0;
+  // FP64 launches of the single-pass classes: one of each gap form, on the side
+  // stream of its first class.  Where FP64 is forced on eight pairs and more for
+  // every resident warp of the per-row kernel of all classes, the per-row
+  // classes have a launch for each of their kernels (kRescueRows), whose
+  // occupancy counts then: 60,000 pairs of 36-101 bases 0.88 ms in one launch of
+  // the kernel of all classes, 0.76 so, of 50-250 bases 1.46 and 1.38; 4,000
+  // pairs of 50-250 bases as fast in one launch, and the call 5% slower so.
+  struct F64Launch {
+    bool uniform;
+    int lo, hi;
+  } f64_single[1 + kNumRescueKernels];
+  int nf64 = 0, top[2] = {0, 0};  // top: most rows of the form's classes with FP64 work
+  uint64_t row_pairs = 0;
+  for (int c = 0; c < kSinglePassClasses; ++c) {
+    if (!plan.pairs[c]) continue;
+    top[class_uniform(c)] = class_rows(c);
+    if (!class_uniform(c)) row_pairs += plan.pairs[c];
+  }
+  if (top[1]) f64_single[nf64++] = {true, 1, kMaxRowsPerLane};
+  const bool split = plan.fp64 && row_pairs >= (uint64_t)num_sms_ * 8 * 8;
+  if (top[0] && !split) f64_single[nf64++] = {false, 1, top[0]};
+  for (int g = kNumRescueKernels - 1; g >= 0 && split; --g) {
+    const int lo = g ? kRescueRows[g - 1] + 1 : 1;
+    uint64_t n = 0;
+    for (int R = lo; R <= kRescueRows[g]; ++R) n += plan.pairs[single_pass_class(R, false)];
+    if (n) f64_single[nf64++] = {false, lo, kRescueRows[g]};
+  }
   if (parts & 2)
-    RODV_CUDA(fork(f64_form[0] + f64_form[1] + (plan.pairs[kSinglePassClasses] > 0) +
+    RODV_CUDA(fork(nf64 + (plan.pairs[kSinglePassClasses] > 0) +
                    (plan.pairs[kSinglePassClasses + 1] > 0)));
-  // the multi-pass classes, then the single-pass ones of each gap form (on
-  // the side stream of the form's first class)
+  // the multi-pass classes, then the single-pass ones
   for (int c = kNumClasses - 1; c >= kSinglePassClasses && (parts & 2); --c) {
     if (!plan.pairs[c]) continue;
     const cudaStream_t ls = lane(c);
@@ -1354,11 +1377,11 @@ rodv_status Engine::launch_parts(const PackedPlan& plan, uint8_t* dbase, rodv_st
     if (s != RODV_OK) return s;
     ++launches;
   }
-  for (int u = 1; u >= 0 && (parts & 2); --u) {
-    if (!f64_form[u]) continue;
-    const cudaStream_t ls = lane(single_pass_class(1, u != 0));
+  for (int q = 0; q < nf64 && (parts & 2); ++q) {
+    const F64Launch& f = f64_single[q];
+    const cudaStream_t ls = lane(single_pass_class(f.lo, f.uniform));
     if (!ls) return cuda_fail(cudaErrorUnknown, "class stream fork");
-    const rodv_status s = launch_rescue(plan, dbase, u != 0, ls);
+    const rodv_status s = launch_rescue(plan, dbase, f.uniform, f.lo, f.hi, ls);
     if (s != RODV_OK) return s;
     ++launches;
   }

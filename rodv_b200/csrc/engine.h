@@ -216,7 +216,7 @@ class Engine {
   rodv_status launch_fp64_class(const PackedPlan& plan, uint8_t* dbase, int cls, int variant,
                                 cudaStream_t stream, bool full_grid = false,
                                 int* grid = nullptr);
-  rodv_status launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform,
+  rodv_status launch_rescue(const PackedPlan& plan, uint8_t* dbase, bool uniform, int lo, int hi,
                             cudaStream_t stream);
   rodv_status check_errors(const PackedPlan& plan, uint8_t* dbase);
   rodv_status run_host_single(const rodv_batch& b, double* out, rodv_stats* st, bool fp64,

@@ -57,20 +57,30 @@ KernelInfo make_pipe_info(int variant) {
   return k;
 }
 
-// The FP64 kernel of every single-pass class of one gap form.
-template <int GAPS>
-KernelInfo rescue_info_for() {
-  using F = Forward<F64, kMaxRowsPerLane, GAPS, false, false, 1>;
+// The FP64 kernel of the single-pass classes of up to HI rows per lane.
+template <int GAPS, int HI>
+KernelInfo make_rescue_info() {
+  using F = Forward<F64, HI, GAPS, false, false, 1>;
   KernelInfo k;
-  k.fn = reinterpret_cast<const void*>(&rescue_kernel<GAPS>);
+  k.fn = reinterpret_cast<const void*>(&rescue_kernel<GAPS, HI>);
   k.threads = F::kWarpsPerBlock * kWarp;
   k.warps_per_block = F::kWarpsPerBlock;
   k.smem_bytes = F::kWarpsPerBlock * F::kSmemPerWarp;
-  k.rows_per_lane = kMaxRowsPerLane;
+  k.rows_per_lane = HI;
   k.uniform = GAPS != kGapsPerRow;
   k.same_hap = true;
   k.items_per_block = F::kWarpsPerBlock;
   return k;
+}
+// The one with the fewest rows that has the class of `rows` rows per lane.
+template <int GAPS>
+KernelInfo rescue_info_for(int rows) {
+  if constexpr (GAPS == kGapsPerRow) {
+    if (rows <= kRescueRows[0]) return make_rescue_info<GAPS, kRescueRows[0]>();
+    if (rows <= kRescueRows[1]) return make_rescue_info<GAPS, kRescueRows[1]>();
+    if (rows <= kRescueRows[2]) return make_rescue_info<GAPS, kRescueRows[2]>();
+  }
+  return make_rescue_info<GAPS, kMaxRowsPerLane>();
 }
 
 // The multi-pass variants of strip height R (pipe_variant_rows) for one

@@ -65,14 +65,20 @@ constexpr int kMaxGroupedRows = 4;  // classes with R <= 4 have the grouped vari
 // same: FP32 items whose reads share the haplotypes -- ChainItem for
 // single-pass classes, SameItem for multi-pass ones; !same: DiffItem
 // (multi-pass leftovers; in a single-pass class, the pairs of each region's
-// odd read).  FP64 kernels take PairRef lists; the single-pass classes of one
-// gap form share one, whatever rows_per_lane.  variant <
+// odd read).  FP64 kernels take PairRef lists; that of a single-pass class also
+// takes the lists of the classes of the gap form with fewer rows (uniform gaps:
+// with any).  variant <
 // forward_kernel_variants(...) selects the variant: of same-haplotype FP32
 // single-pass kernels, and of every multi-pass kernel (FP32 same and
 // two-haplotype items share the class's variant, so they agree on the pass
 // count; FP64 ones have their own).
 KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, GapForm gaps, bool multi,
                                bool same = true, int variant = 0);
+// Rows per lane of the longest class that each per-row FP64 kernel of the
+// single-pass classes has; their 5, 4, 3 and 2 blocks per SM are what the
+// registers of that class leave.
+constexpr int kNumRescueKernels = 4;
+constexpr int kRescueRows[kNumRescueKernels] = {2, 4, 6, kMaxRowsPerLane};
 inline int forward_kernel_variants(Precision prec, bool same, int rows_per_lane = 8,
                                    bool multi = true) {
   if (multi) return kPipeVariants;

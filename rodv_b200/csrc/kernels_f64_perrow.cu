@@ -2,5 +2,5 @@
 #include "kernel_table.cuh"
 
 namespace rodv {
-template KernelInfo rescue_info_for<kGapsPerRow>();
+template KernelInfo rescue_info_for<kGapsPerRow>(int);
 }  // namespace rodv

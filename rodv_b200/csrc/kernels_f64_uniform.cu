@@ -2,5 +2,5 @@
 #include "kernel_table.cuh"
 
 namespace rodv {
-template KernelInfo rescue_info_for<kGapsUniform>();
+template KernelInfo rescue_info_for<kGapsUniform>(int);
 }  // namespace rodv

@@ -1268,8 +1268,10 @@ __global__ void __launch_bounds__(
 // after an FP32 pass that rescues a handful of pairs, and with the classes'
 // tails one after the other when every pair is FP64 (use_double on 50 uneven
 // regions: 1.65 -> 1.44 ms; 16 launches of a 100-region batch become 9).  The
-// rows-per-lane code of all classes shares one register budget: 118 with four
-// blocks per SM; uncapped it takes 166 and three blocks.
+// rows-per-lane code of all classes shares one register budget: in the scaled
+// form 118 with four blocks per SM (uncapped it takes 166 and three blocks).
+// Per-row gaps take 221 registers with R = 8 and 88 up to R = 2, so that form has
+// kernels of the classes up to HI (kernels.h, kRescueRows).
 template <int R, int GAPS>
 __device__ __forceinline__ void rescue_one(const BatchView& b, const RescueLaunch& r,
                                            uint32_t item, int lane, uint4* table) {
@@ -1280,20 +1282,37 @@ __device__ __forceinline__ void rescue_one(const BatchView& b, const RescueLaunc
     F::run_item(b, r.c, r.list[R - 1], item, lane, 0, table);
 }
 
-template <int GAPS>
-__global__ void __launch_bounds__(4 * kWarp, GAPS == kGapsPerRow ? 2 : 4)
+// rescue_one of the class of R rows, 1 <= R <= HI.
+template <int HI, int GAPS>
+__device__ __forceinline__ void rescue_rows(int R, const BatchView& b, const RescueLaunch& r,
+                                            uint32_t item, int lane, uint4* table) {
+  if constexpr (HI > 1) {
+    if (R != HI) {
+      rescue_rows<HI - 1, GAPS>(R, b, r, item, lane, table);
+      return;
+    }
+  }
+  rescue_one<HI, GAPS>(b, r, item, lane, table);
+}
+
+constexpr int rescue_min_blocks(int gaps, int hi) {
+  return gaps != kGapsPerRow ? 4 : hi > 6 ? 2 : hi > 4 ? 3 : hi > 2 ? 4 : 5;
+}
+
+template <int GAPS, int HI>
+__global__ void __launch_bounds__(4 * kWarp, rescue_min_blocks(GAPS, HI))
     rescue_kernel(BatchView b, RescueLaunch r) {
-  using F = Forward<F64, kMaxRowsPerLane, GAPS, false, false, 1>;
+  using F = Forward<F64, HI, GAPS, false, false, 1>;
   static_assert(F::kWarpsPerBlock == 4, "launch bounds");
   extern __shared__ uint4 smem[];
-  __shared__ uint32_t ends[kMaxRowsPerLane];  // items of the classes of 8, 7, ... rows per lane
+  __shared__ uint32_t ends[HI];  // items of the classes of HI, HI - 1, ... rows per lane
   const int lane = threadIdx.x & (kWarp - 1);
   const int warp = threadIdx.x / kWarp;
   uint4* table = smem + warp * (F::kSmemPerWarp / 16);
   if (threadIdx.x == 0) {
     uint32_t n = 0;
-    for (int k = 0; k < kMaxRowsPerLane; ++k) {
-      const uint32_t* count = r.count[kMaxRowsPerLane - 1 - k];
+    for (int k = 0; k < HI; ++k) {
+      const uint32_t* count = r.count[HI - 1 - k];
       if (count) n += *count;
       ends[k] = n;
     }
@@ -1303,20 +1322,11 @@ __global__ void __launch_bounds__(4 * kWarp, GAPS == kGapsPerRow ? 2 : 4)
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(r.c.counter, 1u);
     item = __shfl_sync(kFullMask, item, 0);
-    if (item >= ends[kMaxRowsPerLane - 1]) break;
+    if (item >= ends[HI - 1]) break;
     int k = 0;
     while (item >= ends[k]) ++k;
     if (k) item -= ends[k - 1];
-    switch (kMaxRowsPerLane - k) {
-      case 8: rescue_one<8, GAPS>(b, r, item, lane, table); break;
-      case 7: rescue_one<7, GAPS>(b, r, item, lane, table); break;
-      case 6: rescue_one<6, GAPS>(b, r, item, lane, table); break;
-      case 5: rescue_one<5, GAPS>(b, r, item, lane, table); break;
-      case 4: rescue_one<4, GAPS>(b, r, item, lane, table); break;
-      case 3: rescue_one<3, GAPS>(b, r, item, lane, table); break;
-      case 2: rescue_one<2, GAPS>(b, r, item, lane, table); break;
-      default: rescue_one<1, GAPS>(b, r, item, lane, table); break;
-    }
+    rescue_rows<HI, GAPS>(HI - k, b, r, item, lane, table);
     __syncwarp();
   }
 }

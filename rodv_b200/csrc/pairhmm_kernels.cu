@@ -11,7 +11,7 @@ namespace rodv {
 template <int R, bool MU>
 KernelInfo info_for(GapForm gaps, bool same, int variant);
 template <int GAPS>
-KernelInfo rescue_info_for();
+KernelInfo rescue_info_for(int rows);
 template <int R>
 KernelInfo pipe_info_for(Precision prec, GapForm gaps, bool same, int variant);
 
@@ -22,11 +22,11 @@ KernelInfo forward_kernel_info(Precision prec, int rows_per_lane, GapForm gaps, 
     return pipe_variant_rows(v) == 4 ? pipe_info_for<4>(prec, gaps, same, v)
                                      : pipe_info_for<8>(prec, gaps, same, v);
   }
-  if (prec == Precision::kF64) {  // one kernel for every single-pass class
+  if (prec == Precision::kF64) {  // kernels of several single-pass classes
     switch (gaps) {
-      case kGapsPerRow: return rescue_info_for<kGapsPerRow>();
-      case kGapsUniform: return rescue_info_for<kGapsUniform>();
-      default: return rescue_info_for<kGapsConst>();
+      case kGapsPerRow: return rescue_info_for<kGapsPerRow>(rows_per_lane);
+      case kGapsUniform: return rescue_info_for<kGapsUniform>(rows_per_lane);
+      default: return rescue_info_for<kGapsConst>(rows_per_lane);
     }
   }
   switch (rows_per_lane) {
