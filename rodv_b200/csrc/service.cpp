@@ -1,6 +1,10 @@
 // service.cpp -- streaming PairHMM service: continuous batching of submitted
 // regions over three device batch slots (see service.h).
 #include "service.h"
+
+#if defined(__linux__)
+#include <sys/prctl.h>
+#endif
 #include "trace.h"
 #include "worker_pool.h"
 
@@ -232,7 +236,11 @@ rodv_status Service::submit(const rodv_batch& b, uint64_t* ticket) {
 
 void Service::worker() {
   cudaSetDevice(engine_.device_);
+#if defined(__linux__)
+  prctl(PR_SET_TIMERSLACK, 1000ul);  // this thread's sleeps end within a microsecond or so
+#endif
   std::deque<int> busy;  // slots with a batch in flight, oldest first
+  Clock::time_point last_launch = Clock::now();
   for (;;) {
     // Collect every batch that is done, in whatever order they finish (a
     // small batch launched after a large one often finishes first, and its
@@ -276,11 +284,21 @@ void Service::worker() {
         }
       } else {
         // Batches in flight, and no launch due or nothing queued: look again
-        // in a few microseconds.  (Asleep here, the worker cost every submit
-        // meanwhile a wake-up call.)
-        lk.unlock();
-        const Clock::time_point until = Clock::now() + std::chrono::microseconds(4);
-        while (Clock::now() < until) std::this_thread::yield();
+        // after a thirty-second of the time since the last launch, so that a
+        // batch's end is seen within 3% of its length and a long batch keeps no
+        // core busy.  In the first milliseconds the worker sleeps without
+        // waiting for a notification, which would cost every submit meanwhile a
+        // wake-up call; later, arrivals wake it as soon as a launch is due.
+        const auto since = std::chrono::duration_cast<std::chrono::microseconds>(
+            Clock::now() - last_launch);
+        const auto nap = std::min(std::max(since / 32, std::chrono::microseconds(5)),
+                                  std::chrono::microseconds(500));
+        if (since < std::chrono::milliseconds(2)) {
+          lk.unlock();
+          std::this_thread::sleep_for(nap);
+        } else {
+          cv_work_.wait_for(lk, nap, [&] { return can_launch && !pending_.empty(); });
+        }
         continue;
       }
     }
@@ -289,6 +307,7 @@ void Service::worker() {
     s.batch_id = next_batch_++;
     const Clock::time_point t0 = Clock::now();
     const rodv_status st = launch(s);
+    last_launch = Clock::now();
     release_ring(s);  // packed into the slot's staging: the ring ranges are free
     {
       std::lock_guard<std::mutex> lk(mu_);
