@@ -12,8 +12,10 @@
 //      against one haplotype) and leftover two-haplotype items; pairs whose
 //      scaled FP32 result is below 1e-28 are appended to the class's FP64
 //      list on the device;
-//   4. per work class, one persistent FP64 launch that drains that list (its
-//      length is read by the kernel, never by the host);
+//   4. persistent FP64 launches that drain those lists (their lengths are read
+//      by the kernels, never by the host): one for the single-pass classes of
+//      each gap form (several where FP64 is forced on a large batch of per-row
+//      gaps), one for each multi-pass class;
 //   5. one D2H copy of the log10 results.
 // The reference instead groups pairs into SIMD-width groups by padded area
 // (greedy_grouping, :46-105) and sends leftovers to a per-pair kernel; here
@@ -107,7 +109,7 @@ float* class_scratch(const PackedPlan& p, const ArenaView& a, int c) {
 // measured best for each rows-per-lane value on B200.
 int default_variant(int cls) {
   const int R = class_rows(cls);
-  if (class_multi(cls)) return 1;            // strip height 8, 4 warps per item
+  if (class_multi(cls)) return 1;            // strip height 8, 4 warps per block
   // two 16-lane groups, 4 (per-row R = 4: 3) blocks/SM: uniform R = 3 2.61 ms
   // on its tuning batch against 2.99 with one chain per warp, R = 4 3.44 and
   // 3.31; per-row R = 4 4.91 and 5.33
@@ -670,9 +672,6 @@ rodv_status Engine::pack(const rodv_batch& b, PackedPlan& plan, PinnedMem& stagi
   const ChainStacking stacking = !stack ? ChainStacking::kNone
                                  : pairs >= (uint64_t)num_sms_ * 16 * 8 ? ChainStacking::kAll
                                                                         : ChainStacking::kUniform;
-  auto region_chains = [&](const std::vector<uint32_t>& sr, RegionChains& rc) {
-    plan_region_chains(b.read_lengths, read_class.data(), geoms, stacking, sr, rc);
-  };
   for (int c = 0; c < kNumClasses; ++c) {
     plan.variant[c] = variant_[c];
     plan.variant64[c] = variant64_[c];
@@ -1932,7 +1931,7 @@ rodv_status Engine::plain(rodv_device_batch* db, double* out, rodv_stats* st) {
 //     registers) and, for reads up to 128 bases, one or two chain items per
 //     warp (16-lane groups with twice the rows per lane);
 //   multi-pass classes: the strip height (4 or 8 rows per lane per pass) and
-//     the warps that sweep one item's passes concurrently (2 or 4), for the
+//     the warps of a block, which sweep its items' passes (2 or 4), for the
 //     FP32 kernel and, on a batch forced to FP64, for the FP64 kernel.
 // Synthetic batches: reads of 32R-5 bases against four 400-base haplotypes
 // per region (single-pass), or 1,500-base reads against 3,000-base
@@ -1983,7 +1982,7 @@ namespace {
 std::string variant_name(int cls, int v, bool fp64) {
   char buf[96];
   if (class_multi(cls))
-    snprintf(buf, sizeof(buf), "strip height %d, %d warps per item", pipe_variant_rows(v),
+    snprintf(buf, sizeof(buf), "strip height %d, %d warps per block", pipe_variant_rows(v),
              pipe_variant_warps(v));
   else if (fp64)
     snprintf(buf, sizeof(buf), "one variant");

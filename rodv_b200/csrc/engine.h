@@ -242,8 +242,8 @@ class Engine {
   std::string device_name_;
   cudaStream_t stream_ = nullptr;
   cudaEvent_t ev_[4] = {};
-  // launch_all fan-out: one per class, then one per single-pass class's
-  // two-haplotype items
+  // launch_all fan-out: one per class, then one per class's two-haplotype items
+  // (a multi-pass class's where both launches have boundary rows of their own)
   static constexpr int kBranches = 2 * kNumClasses;
   cudaStream_t side_[kBranches] = {};
   cudaEvent_t fork_ev_ = nullptr, join_ev_[kBranches] = {};

@@ -32,7 +32,7 @@ KernelInfo make_info(int variant) {
   return k;
 }
 
-// Multi-pass kernels: the passes of one item on the W warps of a block.
+// Multi-pass kernels: a pool of passes on the W warps of a block.
 template <class P, int R, int GAPS, bool SAME, int W, int WARPS = 12>
 KernelInfo make_pipe_info(int variant) {
   // 168 registers (12 warps per SM) in the scaled form, 8 warps for launches
@@ -84,7 +84,7 @@ KernelInfo rescue_info_for(int rows) {
 }
 
 // The multi-pass variants of strip height R (pipe_variant_rows) for one
-// precision, gap form and item kind: W = 2 or 4 warps per item.
+// precision, gap form and item kind: W = 2 or 4 warps per block.
 template <int R, int GAPS>
 KernelInfo pipe_gap_info(Precision prec, bool same, int variant) {
   const bool w4 = pipe_variant_warps(variant) == 4;
@@ -120,9 +120,9 @@ KernelInfo pipe_info_for(Precision prec, GapForm gaps, bool same, int variant) {
 // the chain kernels of reads up to 128 bases (R <= 4) also in a lane-grouped
 // form: two 16-lane groups per warp, each sweeping its own chain item with
 // 2R rows per lane, so that each lane's per-step overhead (shuffles, code and
-// table loads, row-0 selects) covers twice the rows (faster at R <= 2 on B200,
-// slower at R >= 3, where the longer per-step dependency chain shows; the
-// autotuner picks).  Every other kernel has one variant.
+// table loads, row-0 selects) covers twice the rows (faster on B200 at R <= 3
+// and, with per-row gaps, R = 4; slower at uniform R = 4, where the longer
+// per-step dependency chain shows; the autotuner picks).  Every other kernel has one variant.
 template <class P, int R, int GAPS, bool MU, bool SAME>
 KernelInfo variant_info(int variant) {
   if constexpr (!(std::is_same<P, F32x2>::value && SAME)) {

@@ -52,8 +52,9 @@ constexpr int kTuneVariants = 8;
 constexpr int kOccupancyTargets = 4;
 constexpr int kVariantMinBlocks[kTuneVariants] = {4, 5, 6, 8, 4, 5, 6, 8};
 // Per-row kernels of seven and eight rows per lane keep five coefficients a
-// row: at 128 registers (four blocks per SM) R = 7 spills 240 and R = 8 860
-// bytes a thread, so their targets start at three blocks (168 registers).
+// row: at 128 registers (four blocks per SM) R = 7 spills 164 bytes a thread
+// (stores), R = 8 440 and eight rows in 16-lane groups 824, so their targets
+// start at three blocks (168 registers: none, 16 and 88 bytes).
 constexpr int kPerRowMinBlocks[kTuneVariants] = {3, 4, 5, 6, 3, 4, 5, 6};
 constexpr int variant_min_blocks(int variant, int rows, bool per_row) {
   return per_row && rows >= 7 ? kPerRowMinBlocks[variant] : kVariantMinBlocks[variant];

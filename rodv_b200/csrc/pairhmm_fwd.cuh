@@ -354,8 +354,7 @@ struct Forward {
   // row below the read's last row L takes ii = mi instead of 1, so it holds
   // mi*I^_L + M~_L = (M_L + I_L)/gapm, and the rows below it copy that value
   // down.  The likelihood term of a DP with row 0 = init is (M_L + I_L)/c, so
-  // the result is (sum of that row)/mi when lane 31's last register is a
-  // pass-through row, and sum(M~_L)/mi + sum(I^_L) when it is row L itself.
+  // the result is (sum of that row)/mi (every sweep ends in a pass-through row).
   // (Scaling row L by 1/mi instead would make the next row's (mm/c)*M~
   // overflow for likely pairs on short haplotypes.)
   // sum_lane (scaled form, chain sweeps): this lane's last row is a pair's
@@ -500,43 +499,34 @@ struct Forward {
   // column on entry (the left neighbours) and this column on exit; dg is the
   // row above the lane's first row at the previous column, up the same row
   // at this column.  t_last: the last row's M before the emission multiply
-  // (M[R-1] = t_last * e[R-1]), for the running sum of the last row.
+  // (M[R-1] = t_last * e[R-1]), for the running sum of the last row.  Per-row
+  // gaps; the scaled form's sweeps all use cells_scaled.
   __device__ __forceinline__ static void cells(const V (&e)[R], V up_m, V up_i, V up_d, V& dg_m,
                                                V& dg_i, V& dg_d, V (&M)[R], V (&I)[R], V (&D)[R],
                                                const Priors& p, V& t_last) {
+    static_assert(!kScaled, "uniform gaps use cells_scaled");
     V dm = dg_m, di = dg_i, dd = dg_d, um = up_m, ui = up_i;
 #pragma unroll
     for (int k = 0; k < R; ++k) {
       const V oM = M[k], oI = I[k], oD = D[k];
-      V t = P::add(di, dd);
-      if constexpr (kScaled) {
-        t = P::fma(p.mmU, dm, t);
-      } else {
-        t = P::mul(p.gapm[k], t);
-        t = P::fma(p.mm[k], dm, t);
-      }
+      const V t = P::fma(p.mm[k], dm, P::mul(p.gapm[k], P::add(di, dd)));
       M[k] = emit(t, e[k]);
       if (k == R - 1) t_last = t;
-      if constexpr (kScaled) {
-        I[k] = P::fma(p.ii[k], ui, um);
-        D[k] = P::fma(p.ddU, oD, oM);
-      } else {
-        I[k] = P::fma(p.ii[k], ui, P::mul(p.mi[k], um));
-        D[k] = P::fma(p.ii[k], oD, P::mul(p.md[k], oM));
-      }
+      I[k] = P::fma(p.ii[k], ui, P::mul(p.mi[k], um));
+      D[k] = P::fma(p.ii[k], oD, P::mul(p.md[k], oM));
       dm = oM; di = oI; dd = oD;
       um = M[k]; ui = I[k];
     }
     dg_m = up_m; dg_i = up_i; dg_d = up_d;
   }
 
-  // cells() of the scaled form with the row above the lane's first row
+  // One column of the scaled form with the row above the lane's first row
   // folded by the lane above (run_chain): t0 is the first row's M term
   // (mm/c)*M~_d + I^_d + D^_d and i0 its I^, both computed by the lane above
-  // with the same operations cells() would apply here, so the results are
-  // bitwise the same while the lanes exchange two values a step instead of
-  // three.  D takes each row's ii: the read's dd on its rows (uniform gaps:
-  // ii == dd, the value cells() uses), and 1 on pass-through rows below row
+  // with the operations of the rows below, so the results are bitwise those of
+  // a hand-over of M~, I^ and D^ while the lanes exchange two values a step
+  // instead of three.  D takes each row's ii: the read's dd on its rows (uniform
+  // gaps: ii == dd), and 1 on pass-through rows below row
   // L, where M is 0 and D stays 0 -- except on a chain sweep's sum row, whose
   // emission 1 makes its M the pass-through value one column back and its D
   // the exact running sum of the earlier ones (run_chain).  kConst: every row
@@ -597,20 +587,18 @@ struct Forward {
     }
   }
 
-  // The scaled form's likelihood from the last register's column sums of
-  // M~ (acc_m) and I^ (acc_i); rows: the rows the sweep held for the read.
+  // The scaled form's likelihood from the column sum of I^ of a pass-through row.
   // accept_min: the FP32 acceptance bound for it.  The scaled sweep keeps M
   // about c = mi*gapm times smaller than the reference's FP32 sweep, so its
   // bound is 1e-28/c: an accepted result keeps the reference's headroom above
   // the FP32 denormal range (below the bound, the pair goes to FP64).
   __device__ __forceinline__ static double scaled_result(const BatchView& b,
                                                          const GapConsts& gaps, uint32_t read,
-                                                         uint32_t len, uint32_t rows, S acc_m,
-                                                         S acc_i, double* accept_min) {
+                                                         S sum, double* accept_min) {
     double mi, gapm;
     read_gaps(b, gaps, read, &mi, &gapm);
     *accept_min = (double)kMinAcceptedF / (mi * gapm);
-    return len < rows ? (double)acc_i / mi : (double)acc_m / mi + (double)acc_i;
+    return (double)sum / mi;
   }
 
   // Early end of an FP32 multi-pass sweep.  Every alignment emits read row r
@@ -623,12 +611,11 @@ struct Forward {
   // pair is rejected at the end of the sweep whatever the remaining passes
   // compute, so when both slots are decided the sweep stops and queues them
   // for FP64 now: the same pairs reach FP64 and every result is unchanged.
-  // `row`: 0-based read row of the boundary; H: the slots' haplotype lengths.
+  // H: the slots' haplotype lengths.
   __device__ static bool sweep_rejected(const BatchView& b, const ClassLaunch& c,
                                         const BoundaryCell* buf, const uint32_t (&H)[2],
-                                        const uint32_t (&L)[2], uint32_t row, int lane,
-                                        uint32_t item) {
-    const bool rejected = row_bound_rejects(b, c, buf, H, L, row, lane, item);
+                                        int lane, uint32_t item) {
+    const bool rejected = row_bound_rejects(c, buf, H, lane, item);
     if (rejected && lane == 0) {
       PairRef refs[2];
       load_refs(c, item, refs);
@@ -640,10 +627,8 @@ struct Forward {
 
   // The decision of sweep_rejected, taken by the whole warp (the same value
   // in every lane); nothing is written.
-  __device__ static bool row_bound_rejects(const BatchView& b, const ClassLaunch& c,
-                                           const BoundaryCell* buf, const uint32_t (&H)[2],
-                                           const uint32_t (&L)[2], uint32_t row, int lane,
-                                           uint32_t item) {
+  __device__ static bool row_bound_rejects(const ClassLaunch& c, const BoundaryCell* buf,
+                                           const uint32_t (&H)[2], int lane, uint32_t item) {
     V sm = P::zero(), si = P::zero();
     for (uint32_t col = 1 + (uint32_t)lane; col <= H[0]; col += kWarp) {
       const BoundaryCell cell = buf[col];
@@ -667,25 +652,17 @@ struct Forward {
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       if (s == 1 && refs[1].read == kNoPair) continue;
-      double bound, amin = (double)kMinAcceptedF;
-      if (kScaled) {
-        // M~ = mi * M and I^ = I; a pass-through row holds mi * (M_L + I_L) in I^
-        double mi, gapm;
-        read_gaps(b, c.gaps, refs[s].read, &mi, &gapm);
-        bound = row < L[s] ? sum_m[s] / mi + sum_i[s] : sum_i[s] / mi;
-        amin /= mi * gapm;
-      } else {
-        bound = sum_m[s] + sum_i[s];
-      }
-      rejected = rejected && bound >= 0.0 && bound < amin * 1e-6;
+      const double bound = sum_m[s] + sum_i[s];
+      rejected = rejected && bound >= 0.0 && bound < (double)kMinAcceptedF * 1e-6;
     }
     return rejected;
   }
 
   // One pair per slot (SameItem, DiffItem or, for F64, PairRef), swept in one
-  // or (MULTI) several passes of 32R rows.
+  // or (MULTI) several passes of 32R rows.  Per-row gaps.
   __device__ static void run_item(const BatchView& b, const ClassLaunch& c, const void* work,
                                   uint32_t item, int lane, int gwarp, uint4* table) {
+    static_assert(!kScaled, "uniform gaps: run_single and the pipelined sweeps");
     PairRef refs[2];
     load_refs(work, item, refs);
     SlotInfo sl[2];
@@ -808,8 +785,7 @@ struct Forward {
       }
       if constexpr (MULTI && P::kSlots == 2) {
         const uint32_t H[2] = {sl[0].H, sl[1].H};
-        if (!last && sweep_rejected(b, c, buf, H, L, (pass + 1) * (kWarp * R) - 1, lane, item))
-          return;
+        if (!last && sweep_rejected(b, c, buf, H, lane, item)) return;
       }
     }
 
@@ -823,19 +799,8 @@ struct Forward {
     PairRef fr[2];
     load_refs(work, item, fr);
     const bool valid_y = P::kSlots == 2 && fr[1].read != kNoPair;
-    double res[2] = {0.0, 0.0};
-    double amin[2] = {(double)kMinAcceptedF, (double)kMinAcceptedF};
-    if (kScaled) {
-      const uint32_t rows = passes * kWarp * R;
-      res[0] = scaled_result(b, c.gaps, fr[0].read, L[0], rows, P::sx(acc_m), P::sx(acc_i), &amin[0]);
-      if (valid_y)
-        res[1] = scaled_result(b, c.gaps, fr[1].read, L[1], rows, frozen_m, frozen_i, &amin[1]);
-    } else {
-      res[0] = P::sx(acc_m) + P::sx(acc_i);
-      res[1] = frozen_m + frozen_i;
-    }
-    finish(b, c, fr[0], res[0], amin[0]);
-    if (valid_y) finish(b, c, fr[1], res[1], amin[1]);
+    finish(b, c, fr[0], P::sx(acc_m) + P::sx(acc_i));
+    if (valid_y) finish(b, c, fr[1], frozen_m + frozen_i);
   }
 
   // One pair per slot (DiffItem or, for F64, PairRef) in one sweep, scaled
@@ -924,10 +889,9 @@ struct Forward {
 #pragma unroll
     for (int q = 0; q < P::kSlots; ++q) {
       if (refs[q].read == kNoPair) continue;
-      const uint32_t len = b.reads[refs[q].read].len;
-      double amin = (double)kMinAcceptedF;
-      const double res = scaled_result(b, c.gaps, refs[q].read, len, len + 1, S(0),
-                                       q == 0 ? sum_x : sum_y, &amin);
+      double amin;
+      const double res =
+          scaled_result(b, c.gaps, refs[q].read, q == 0 ? sum_x : sum_y, &amin);
       finish(b, c, refs[q], res, amin);
     }
   }
@@ -1181,8 +1145,7 @@ struct Forward {
           const S sum = s == 0 ? a.x : a.y;
           double res, amin = (double)kMinAcceptedF;
           if (kScaled) {  // the pass-through row holds (M_L + I_L)/gapm: the sum / mi
-            const uint32_t len = b.reads[read[s]].len;
-            res = scaled_result(b, c.gaps, read[s], len, len + 1, S(0), sum, &amin);
+            res = scaled_result(b, c.gaps, read[s], sum, &amin);
           } else {        // the pass-through row holds M_L + I_L (its M is 0)
             res = sum;
           }
