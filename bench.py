@@ -445,17 +445,9 @@ def run_engine(args, world, rank, local):
                 if c["config"] in ("C1", "C3", "C4", "C5"):
                     line["config"][c["config"] + "_gcups"] = c["gcups"]
         if accuracy:
-            line["accuracy"] = {k: v for a in accuracy for k, v in flat_accuracy(a).items()}
-            worst = []
-            for key in ("vs_fp64_oracle", "vs_reference"):
-                vals = [a[key]["max"] for a in accuracy if a[key]["max"] is not None]
-                line["config"]["max_abs_dlog10_" + key] = max(vals) if vals else None
-                worst += vals
-            mism = sum(a[k]["non_finite_mismatches"] for a in accuracy
-                       for k in ("vs_fp64_oracle", "vs_reference"))
-            line["accuracy"]["tolerance_log10"] = ACCURACY_TOL
-            line["accuracy"]["within_tolerance"] = bool(worst and max(worst) <= ACCURACY_TOL
-                                                        and mism == 0)
+            line["accuracy"], worst = accuracy_fields(accuracy)
+            for key, v in worst.items():
+                line["config"]["max_abs_dlog10_" + key] = v
         if stream:
             line["streaming"] = stream
         print(json.dumps(line), flush=True)
@@ -701,7 +693,7 @@ def accuracy_per_config(eng):
         for key, scale in (("vs_fp64_oracle", s_oracle), ("vs_reference", s_ref)):
             if key == "vs_reference" and not oracle.ref_available():
                 row[key] = {"pairs": 0, "cells": 0, "max": None, "mean": None,
-                            "non_finite_mismatches": 0}
+                            "non_finite_mismatches": None}
                 continue
             b = workloads.make_workload(wl, seed=workloads.SEEDS[wl] + 99, scale=scale)
             got = eng.batch(b)
@@ -723,6 +715,28 @@ def flat_config(c):
     name = c["config"].replace(" ", "")
     return {f"{name}_{k}": v for k, v in c.items()
             if k != "config" and isinstance(v, (int, float, str))}
+
+
+def accuracy_fields(accuracy):
+    """The line's accuracy keys, and the largest |delta log10| of each comparison
+    (None: it did not run).  within_tolerance is of the comparisons that
+    within_tolerance_vs names, those that ran for every configuration, and None
+    if there is none."""
+    out = {k: v for a in accuracy for k, v in flat_accuracy(a).items()}
+    worst, ran, mism = {}, [], 0
+    for key in ("vs_fp64_oracle", "vs_reference"):
+        vals = [a[key]["max"] for a in accuracy if a[key]["max"] is not None]
+        worst[key] = max(vals) if vals else None
+        misses = [a[key]["non_finite_mismatches"] for a in accuracy]
+        mism += sum(m for m in misses if m is not None)
+        if misses and None not in misses:
+            ran.append(key)
+    out["tolerance_log10"] = ACCURACY_TOL
+    out["within_tolerance_vs"] = " ".join(ran)
+    out["within_tolerance"] = (mism == 0 and all(worst[k] is not None for k in ran) and
+                               all(v <= ACCURACY_TOL for v in worst.values() if v is not None)
+                               if ran else None)
+    return out, worst
 
 
 def flat_accuracy(a):
