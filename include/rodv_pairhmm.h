@@ -113,8 +113,9 @@ typedef struct rodv_stats {
   uint32_t kernel_launches;     /* forward/pack kernels launched by this call */
   uint32_t pad_;
   double total_ms;              /* wall time of the call */
-  double device_ms;             /* device time of the forward kernels (CUDA events) */
-  double fp32_ms;               /* device time of the FP32 pass */
+  double device_ms;             /* device time of the forward kernels (CUDA events); of a batch
+                                   cut in ranges, time in which any range's ran */
+  double fp32_ms;               /* device time of the FP32 pass, likewise */
   double h2d_ms;
   double d2h_ms;
   uint64_t h2d_bytes;

@@ -1547,7 +1547,8 @@ rodv_status Engine::run_host(const rodv_batch& b, double* out, rodv_stats* st, b
   return run_host_single(b, out, st, fp64, prec);
 }
 
-rodv_status Engine::finish_lane(HostLane& l, double* out, rodv_stats* st, uint8_t* prec) {
+rodv_status Engine::finish_lane(HostLane& l, double* out, rodv_stats* st, uint8_t* prec,
+                                double (&timed)[2]) {
   TraceRange trace("rodv: finish range");
   l.busy = false;
   RODV_CUDA(cudaEventSynchronize(l.done));
@@ -1573,11 +1574,16 @@ rodv_status Engine::finish_lane(HostLane& l, double* out, rodv_stats* st, uint8_
     if (prec) std::memcpy(prec + l.out_off + lo, hp + lo, hi - lo);
   });
   if (st) {
+    // the ranges' kernels overlap: time in which any range's (FP32) kernels ran
     float ms = 0.f;
-    cudaEventElapsedTime(&ms, l.ev[0], l.ev[2]);
-    st->device_ms += ms;
-    cudaEventElapsedTime(&ms, l.ev[0], l.ev[1]);
-    st->fp32_ms += ms;
+    double* const sums[2] = {&st->device_ms, &st->fp32_ms};
+    for (int q = 0; q < 2; ++q) {
+      cudaEventElapsedTime(&ms, ev_[3], l.ev[0]);
+      const double begin = std::max(timed[q], (double)ms);
+      cudaEventElapsedTime(&ms, ev_[3], l.ev[q == 0 ? 2 : 1]);
+      *sums[q] += std::max(0.0, ms - begin);
+      timed[q] = std::max(timed[q], (double)ms);
+    }
     cudaEventElapsedTime(&ms, l.ev[3], l.ev[0]);
     st->h2d_ms += ms;
     st->h2d_bytes += p.upload_bytes;
@@ -1595,15 +1601,16 @@ rodv_status Engine::run_host_chunked(const rodv_batch& b, double* out, rodv_stat
                                      uint8_t* prec) {
   const auto t0 = std::chrono::steady_clock::now();
   const bool timeline = opt_.verbose >= 2;
-  if (timeline) RODV_CUDA(cudaEventRecord(ev_[3], lanes_[0].stream));
+  RODV_CUDA(cudaEventRecord(ev_[3], lanes_[0].stream));
   rodv_stats acc{};
+  double timed[2] = {0.0, 0.0};  // end of the last range's kernels, of its FP32 pass
   const size_t nchunks = bounds.size() - 1;
   rodv_status result = RODV_OK;
   uint64_t out_off = 0;
   for (size_t k = 0; k < nchunks && result == RODV_OK; ++k) {
     HostLane& l = lanes_[k % kHostLanes];
     if (l.busy) {
-      result = finish_lane(l, out, &acc, prec);
+      result = finish_lane(l, out, &acc, prec, timed);
       if (result != RODV_OK) break;
     }
     // the range's regions over the batch's arrays, rebased to the range's
@@ -1681,7 +1688,7 @@ rodv_status Engine::run_host_chunked(const rodv_batch& b, double* out, rodv_stat
     HostLane& l = lanes_[k % kHostLanes];
     if (!l.busy) continue;
     if (result == RODV_OK) {
-      result = finish_lane(l, out, &acc, prec);
+      result = finish_lane(l, out, &acc, prec, timed);
     } else {
       cudaStreamSynchronize(l.stream);
       l.busy = false;

@@ -223,7 +223,10 @@ class Engine {
                               uint8_t* prec);
   rodv_status run_host_chunked(const rodv_batch& b, double* out, rodv_stats* st, bool fp64,
                                const std::vector<uint32_t>& bounds, uint8_t* prec);
-  rodv_status finish_lane(HostLane& lane, double* out, rodv_stats* st, uint8_t* prec);
+  // timed: up to when (after the call's start, ms) kernels and FP32 passes are
+  // counted in st already
+  rodv_status finish_lane(HostLane& lane, double* out, rodv_stats* st, uint8_t* prec,
+                          double (&timed)[2]);
   int persistent_blocks(const KernelInfo& k) const;
   size_t multi_rows(bool uniform) const;
   size_t multi_scratch_bytes(bool uniform, size_t cols) const;
