@@ -1778,7 +1778,8 @@ rodv_status Engine::run_device(rodv_device_batch* db, rodv_stats* st) {
   RODV_CUDA(cudaSetDevice(device_));
   uint8_t* d = static_cast<uint8_t*>(db->arena.ptr);
   const auto t0 = std::chrono::steady_clock::now();
-  if (!db->graph[0]) {
+  if (!db->graph[1]) {
+    db->drop_graphs();  // a capture that failed may have left the first one
     // Capture once, as two graphs (FP32 part: counter reset and the FP32 class
     // launches; FP64 part: the rescue launches) so that an event between them
     // times the FP32 pass; later runs are two graph launches.  Within each

@@ -280,8 +280,12 @@ struct rodv_device_batch {
   // launches) captured once as two CUDA graphs and replayed by every run.
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // FP32 part, FP64 part
   uint32_t graph_launches = 0;
-  ~rodv_device_batch() {
-    for (cudaGraphExec_t g : graph)
+  void drop_graphs() {
+    for (cudaGraphExec_t& g : graph) {
       if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+    graph_launches = 0;
   }
+  ~rodv_device_batch() { drop_graphs(); }
 };

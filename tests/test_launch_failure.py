@@ -71,3 +71,25 @@ def test_service_batch(batches, nth):
                 assert np.array_equal(sv.wait(t), ref)
     finally:
         sv.close()
+
+
+@pytest.mark.parametrize("nth", [1, 3, -1])
+def test_device_batch(batches, nth):
+    """A launch that fails while the step is captured, of the FP32 part or (-1: the
+    last) of the FP64 part: the next run captures again."""
+    eng = Engine(0)
+    try:
+        for b, want in batches:
+            db = eng.upload(b)
+            launches = db.run()["kernel_launches"]
+            db.free()
+            db = eng.upload(b)
+            with _Fault(nth if nth > 0 else launches), pytest.raises(RodvError) as ei:
+                db.run()
+            assert ei.value.status == RODV_ERR_CUDA
+            for _ in range(2):
+                assert db.run()["kernel_launches"] == launches
+                assert np.array_equal(db.download(), want)
+            db.free()
+    finally:
+        eng.close()
