@@ -1587,7 +1587,7 @@ rodv_status Engine::finish_lane(HostLane& l, double* out, rodv_stats* st, uint8_
     cudaEventElapsedTime(&ms, l.ev[3], l.ev[0]);
     st->h2d_ms += ms;
     st->h2d_bytes += p.upload_bytes;
-    st->d2h_bytes += p.num_pairs * 8 + kCountWords * 4;
+    st->d2h_bytes += p.result_bytes();
     st->pairs += p.num_pairs;
     st->cells += p.cells;
     for (int c = 0; c < kNumClasses; ++c)
@@ -1746,7 +1746,7 @@ rodv_status Engine::run_host_single(const rodv_batch& b, double* out, rodv_stats
     cudaEventElapsedTime(&ms, ev_[3], ev_[0]);
     st->h2d_ms = ms;
     st->h2d_bytes = plan.upload_bytes;
-    st->d2h_bytes = plan.num_pairs * 8 + kCountWords * 4;
+    st->d2h_bytes = plan.result_bytes();
     st->total_ms = ms_since(t0);
   }
   return RODV_OK;

@@ -1,5 +1,6 @@
-"""Device times of a host call cut in ranges: the ranges' kernels overlap, and time is
-counted once."""
+"""Statistics of a host call.  Device times of one cut in ranges: the ranges' kernels
+overlap, and time is counted once.  Downloaded bytes: each range's counters (a
+block of 512 bytes) and results come back in one copy."""
 import numpy as np
 import pytest
 
@@ -26,3 +27,9 @@ def test_overlapping_ranges_are_timed_once(engine):
         st = engine.batch(b, stats=True)[1]
         assert 0 < st["fp32_ms"] <= st["device_ms"] <= st["total_ms"]
         assert st["device_ms"] >= 0.9 * whole
+
+
+def test_downloaded_bytes(engine):
+    rng = np.random.default_rng(13)
+    one = Batch.from_regions([workloads.random_region(rng, 20, 5)])
+    assert engine.batch(one, stats=True)[1]["d2h_bytes"] == 512 + 8 * one.num_pairs
